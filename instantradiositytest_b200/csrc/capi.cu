@@ -821,13 +821,18 @@ static uint64_t plane_bytes(int fmt, int k, size_t P) {
     return b[fmt][k] * P;
 }
 
+// Offset of the plane after plane k in the staging: the kernels read planes
+// as vectors of up to 16 bytes, so each starts on a 256-byte boundary
+// whatever the frame's pixel count.
+static uint64_t plane_stride(int fmt, int k, size_t P) { return (plane_bytes(fmt, k, P) + 255) & ~255ull; }
+
 static irt_status pipe_setup(irt_session* s) {
     irt_context* ctx = s->ctx;
     irt_session::HostPipe& hp = s->pipe;
     const size_t P = s->P;
     const int fmt = s->desc.gbuffer_format;
     uint64_t gb = 0;
-    for (int k = 0; k < 5; k++) gb += plane_bytes(fmt, k, P);
+    for (int k = 0; k < 5; k++) gb += plane_stride(fmt, k, P);
     const uint64_t pool = (uint64_t)s->desc.settings.vpl_count * sizeof(irt_vpl);
     const uint64_t need = 2 * gb + 4 * pool + 2 * P * s->rad_bytes;
     uint64_t cur = ctx->in_use.load();
@@ -909,7 +914,7 @@ irt_status irt_render_frame_host(irt_session* s, const irt_scene* sc, const irt_
     for (int k = 0; k < 5; k++) {
         dst[k] = base + off;
         CK(cudaMemcpyAsync(base + off, src[k], plane_bytes(fmt, k, P), cudaMemcpyHostToDevice, hp.copy), "G-buffer in");
-        off += plane_bytes(fmt, k, P);
+        off += plane_stride(fmt, k, P);
     }
     const uint64_t pool = (uint64_t)s->desc.settings.vpl_count * sizeof(irt_vpl);
     irt_vpl* cur = hp.vpls + (size_t)vslot * s->desc.settings.vpl_count;

@@ -32,12 +32,15 @@ double seconds_since(Clock::time_point t0) {
     return std::chrono::duration<double>(Clock::now() - t0).count();
 }
 
-uint64_t gbuffer_bytes_per_pixel(int32_t fmt) {
-    switch (fmt) {
-    case IRT_GBUFFER_F32: return 4 + 16 + 16 + 8 + 8;
-    case IRT_GBUFFER_F16: return 4 + 8 + 8 + 4 + 4;
-    default: return 4 + 4 + 4 + 4 + 4;
-    }
+// The five G-buffer planes (depth, normal, color, params, motion) in one
+// allocation: plane k's offset and, at [5], the whole size.  The kernels read
+// planes as vectors of up to 16 bytes, so each starts on a 256-byte boundary
+// whatever the frame's pixel count.
+void plane_offsets(int32_t fmt, uint64_t pixels, uint64_t off[6]) {
+    static const uint64_t bytes[3][5] = {{4, 16, 16, 8, 8}, {4, 8, 8, 4, 4}, {4, 4, 4, 4, 4}};
+    const uint64_t* b = bytes[fmt == IRT_GBUFFER_F32 ? 0 : (fmt == IRT_GBUFFER_F16 ? 1 : 2)];
+    off[0] = 0;
+    for (int k = 0; k < 5; k++) off[k + 1] = off[k] + ((b[k] * pixels + 255) & ~255ull);
 }
 
 struct Inflight {
@@ -112,7 +115,9 @@ extern "C" uint64_t irt_server_request_bytes(const irt_server* s, const irt_requ
     scene += n * (208 + 2 * 48 + 176 + 33ull * 33 * 33 * 4) + 128 * w.meshes.size() + 2 * 48 * w.lights.size();
     for (const irt_mesh& m : w.meshes)  // corner cells of the field meshes (8 texels per cell)
         if (m.geometry_lo[3] <= .5f) scene += (uint64_t)(m.field[3] - 1) * (m.field[3] - 1) * (m.field[3] - 1) * texel * 8;
-    const uint64_t inputs = P * gbuffer_bytes_per_pixel(s->d.gbuffer_format) + 3ull * sd.settings.vpl_count * 48;
+    uint64_t off[6];
+    plane_offsets(s->d.gbuffer_format, P, off);
+    const uint64_t inputs = off[5] + 3ull * sd.settings.vpl_count * 48;
     return irt_session_bytes(&sd) + scene + inputs;
 }
 
@@ -189,8 +194,9 @@ static irt_status admit(irt_server* s, const irt_request& r, cudaStream_t st, Ac
                                      w.spec.sdf_format, &a->scene);
     if (!rc) rc = irt_session_create(s->ctx, &sd, &a->session);
     const size_t P = (size_t)a->W * a->H;
-    const uint64_t gb = P * gbuffer_bytes_per_pixel(s->d.gbuffer_format);
-    if (!rc && cudaMalloc(&a->gbuf, gb) != cudaSuccess) rc = IRT_E_CUDA;
+    uint64_t off[6];
+    plane_offsets(s->d.gbuffer_format, P, off);
+    if (!rc && cudaMalloc(&a->gbuf, off[5]) != cudaSuccess) rc = IRT_E_CUDA;
     if (!rc && cudaMalloc(&a->vpls, 3ull * a->vpl_count * sizeof(irt_vpl)) != cudaSuccess) rc = IRT_E_CUDA;
     if (!rc && cudaMemsetAsync(a->vpls + 2ull * a->vpl_count, 0, a->vpl_count * sizeof(irt_vpl), st) != cudaSuccess)
         rc = IRT_E_CUDA;
@@ -208,21 +214,13 @@ static irt_status admit(irt_server* s, const irt_request& r, cudaStream_t st, Ac
         release(a);
         return rc;
     }
-    // Plane layout: depth f32, then normal, color, params, motion.
-    char* base = static_cast<char*>(a->gbuf);
-    uint64_t nb, cb, pb, mb;
-    switch (s->d.gbuffer_format) {
-    case IRT_GBUFFER_F32: nb = 16, cb = 16, pb = 8, mb = 8; break;
-    case IRT_GBUFFER_F16: nb = 8, cb = 8, pb = 4, mb = 4; break;
-    default: nb = 4, cb = 4, pb = 4, mb = 4; break;
-    }
+    const char* base = static_cast<const char*>(a->gbuf);
     a->g.format = s->d.gbuffer_format;
-    a->g.depth = reinterpret_cast<const float*>(base);
-    a->g.normal = base + P * 4;
-    a->g.color = base + P * (4 + nb);
-    a->g.params = base + P * (4 + nb + cb);
-    a->g.motion = base + P * (4 + nb + cb + pb);
-    (void)mb;
+    a->g.depth = reinterpret_cast<const float*>(base + off[0]);
+    a->g.normal = base + off[1];
+    a->g.color = base + off[2];
+    a->g.params = base + off[3];
+    a->g.motion = base + off[4];
     a->objects.resize(w.objs.size());
     a->nodes.resize(2 * w.objs.size() - 1);
     a->lights.resize(std::max<size_t>(w.lights.size(), 1));
