@@ -162,8 +162,8 @@ LightingLaunch lighting_launch(irt_session* s, const irt_scene* sc, const irt_fr
     L.noisy_out = s->noisy;
     L.radiance_f16 = s->desc.radiance_format == IRT_RADIANCE_F16;
     L.keep_candidates = 0;
-    L.rays = s->rays;
-    L.ray_counters = s->ray_counters;
+    L.prep = s->prep;
+    L.prep_vpl = s->prep_vpl;
     L.vis = s->vis;
     L.pending = s->pending;
     L.guide = s->guide[0];
@@ -289,7 +289,7 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
                 if (scenes[v] != sc) continue;
                 if (queues.size() == G.q_begin) G.f = frames[v];
                 irt_session* s = b->sess[v];
-                queues.push_back(MarchQueue{s->rays, s->ray_counters, s->vis, (uint32_t)(2 * s->P)});
+                queues.push_back(MarchQueue{session_ray_setup(s, sc, cur[v], prev[v]), b->d_frames + v, s->W, s->H});
                 if (!G.error) G.error = s->error;
             }
             G.q_end = (uint32_t)queues.size();
@@ -410,14 +410,6 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
            "batch guides");
         CK(irt_launch_svgf_batched(batch_launch(b, w, t.sviews[7], sv, -1), 4, st), "batch previous guides");
         mark(2);
-        CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, -1), kStageArchive, st), "batch archive");
-        mark(3);
-        CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, shape_of[kTReuse]), kStageReuse, st),
-           "batch reuse");
-        mark(4);
-        CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, shape_of[kTSpatial]), kStageSpatial, st),
-           "batch spatial");
-        mark(5);
         MarchBatch M{};
         M.n_groups = t.wave_groups[w + 1] - t.wave_groups[w];
         M.groups = t.groups + t.wave_groups[w];
@@ -426,6 +418,14 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
         M.num_sms = b->num_sms;
         M.blocks_per_sm = kMarchBps[march_choice];
         M.fast = 1;
+        CK(irt_launch_ray_pools_batched(M, st), "batch ray pools");
+        mark(3);
+        CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, shape_of[kTReuse]), kStageReuse, st),
+           "batch reuse");
+        mark(4);
+        CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, shape_of[kTSpatial]), kStageSpatial, st),
+           "batch spatial");
+        mark(5);
         CK(irt_launch_march_batched(M, st), "batch march");
         mark(6);
         CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, -1), kStageCombine, st), "batch combine");

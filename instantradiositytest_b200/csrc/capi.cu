@@ -441,6 +441,15 @@ void irt_scene_destroy(irt_scene* sc) {
 }
 
 // ------------------------------------------------------------------ session
+// Every VPL's march endpoint (its position moved off the surface by one
+// distance query) is the same for all rays to it, so a frame tabulates them
+// once — unless the pools and the archive hold more VPLs than the frame has
+// pixels, and so rays to them: then each ray queries its own.
+static bool tabulates_ends(const irt_session_desc& d) {
+    return irt_ray_pool_entries(d.settings.vpl_count, d.settings.restir_max_history) <=
+           (uint64_t)d.settings.render_width * d.settings.render_height;
+}
+
 uint64_t irt_session_bytes(const irt_session_desc* d) {
     if (!d) return 0;
     uint64_t P = (uint64_t)d->settings.render_width * d->settings.render_height;
@@ -454,7 +463,10 @@ uint64_t irt_session_bytes(const irt_session_desc* d) {
     b += P * rad * 7;  // noisy, feedback x2, temporal, scratch x2, filtered
     b += P * (d->moments_format == IRT_MOMENTS_F16 ? 8 : 16) * 2;  // moments x2
     b += 16;           // error word
-    if (d->fused == 1) b += P * (2 * sizeof(RayRecord) + 2 * 4 + 2 * 16) + 16;  // ray queue, vis, pending
+    if (d->fused == 1) {
+        b += P * (2 * (sizeof(RayRecord) + 2 + 4 + 16) + 16 + 4) + 16;  // ray queue, vis, pending, ray names
+        if (tabulates_ends(*d)) b += 16 * irt_ray_pool_entries(d->settings.vpl_count, d->settings.restir_max_history);
+    }
     b += P * 16 * 2;                                                             // position guides
     b += P * 32;                                                                 // SVGF features
     return b;
@@ -527,6 +539,12 @@ irt_status irt_session_create(irt_context* ctx, const irt_session_desc* desc, ir
     if (!st) st = dev_alloc(ctx, &s->error, 16, used);
     if (desc->fused == 1) {
         if (!st) st = dev_alloc(ctx, &s->rays, P * 2 * sizeof(RayRecord), used);
+        if (!st) st = dev_alloc(ctx, &s->ray_hints, P * 2 * 2, used);
+        if (!st) st = dev_alloc(ctx, &s->prep, P * 16, used);
+        if (!st) st = dev_alloc(ctx, &s->prep_vpl, P * 4, used);
+        if (!st && tabulates_ends(*desc))
+            st = dev_alloc(ctx, &s->ray_ends,
+                           16 * irt_ray_pool_entries(desc->settings.vpl_count, desc->settings.restir_max_history), used);
         if (!st) st = dev_alloc(ctx, &s->ray_counters, 16, used);
         if (!st) st = dev_alloc(ctx, &s->vis, P * 2 * 4, used);
         if (!st) st = dev_alloc(ctx, &s->pending, P * 2 * 16, used);
@@ -553,7 +571,7 @@ void irt_session_destroy(irt_session* s) {
     void* ptrs[] = {s->dres[0], s->dres[1], s->dres[2], s->ires[0], s->ires[1], s->ires[2], s->archive,
                     s->prev_depth, s->prev_normal, s->direct, s->noisy, s->moments[0], s->moments[1],
                     s->feedback[0], s->feedback[1], s->temporal, s->scratch[0], s->scratch[1], s->filtered, s->error,
-                    s->rays, s->ray_counters, s->vis, s->pending, s->guide[0], s->guide[1], s->feat};
+                    s->rays, s->ray_hints, s->prep, s->prep_vpl, s->ray_ends, s->ray_counters, s->vis, s->pending, s->guide[0], s->guide[1], s->feat};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s->pipe.ready) {
@@ -647,10 +665,34 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
     s->prof_frame[s->prof_slot] = f->size[2];
     mark(s, 0, st);
     CK(compute_guides(s, f, g, st), "position guides");
-    // VPL archive ring slot frame % (H+1) (src/renderer.rs:1873-1884).
-    size_t pool = (size_t)set.vpl_count * sizeof(irt_vpl);
-    uint32_t slot = f->size[2] % (set.restir_max_history + 1u);
-    CK(cudaMemcpyAsync((char*)s->archive + slot * pool, cur, pool, cudaMemcpyDeviceToDevice, st), "archive copy");
+    // VPL archive ring slot frame % (H+1) (src/renderer.rs:1873-1884); with
+    // the ray queue, in one launch with the queue's reset and the endpoints.
+    MarchLaunch M{};
+    if (s->desc.fused == 1) {
+        M.frame = f;
+        M.objects = sc->objects;
+        M.meshes = sc->meshes;
+        M.nodes = sc->nodes;
+        M.atlas = sc->atlas;
+        M.sdf_f16 = sc->sdf_f16;
+        M.sdf_cells = sc->sdf_cells;
+        M.field_filter = scene_field_filter(sc);
+        M.error = s->error;
+        M.march_scene = sc->march_scene;
+        M.cells = sc->cells;
+        for (int a = 0; a < 3; a++) {
+            M.grid_org[a] = sc->grid_org[a];
+            M.grid_inv[a] = sc->grid_inv[a];
+        }
+        M.setup = session_ray_setup(s, sc, cur, prev);
+        M.num_sms = s->num_sms;
+        M.fast = s->desc.exact_march ? 0 : 1;
+        CK(irt_launch_ray_pools(M, st), "ray pools");
+    } else {
+        size_t pool = (size_t)set.vpl_count * sizeof(irt_vpl);
+        uint32_t slot = f->size[2] % (set.restir_max_history + 1u);
+        CK(cudaMemcpyAsync((char*)s->archive + slot * pool, cur, pool, cudaMemcpyDeviceToDevice, st), "archive copy");
+    }
     mark(s, 1, st);
     LightingLaunch L{};
     L.frame = f;
@@ -677,42 +719,20 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
     L.noisy_out = s->noisy;
     L.radiance_f16 = s->desc.radiance_format == IRT_RADIANCE_F16;
     L.keep_candidates = s->desc.keep_candidates;
-    L.rays = s->rays;
-    L.ray_counters = s->ray_counters;
+    L.prep = s->prep;
+    L.prep_vpl = s->prep_vpl;
     L.vis = s->vis;
     L.pending = s->pending;
     L.guide = s->guide[0];
     L.old_guide = s->guide[1];
     L.feat = s->desc.gbuffer_format == IRT_GBUFFER_F32 ? nullptr : s->feat;
     if (s->desc.fused == 1) {
-        // candidates+temporal -> spatial + resolve set-up (ray queue) ->
+        // candidates+temporal -> spatial + resolve set-up -> ray set-up and
         // persistent march -> resolve outputs.
-        CK(cudaMemsetAsync(s->ray_counters, 0, 16, st), "ray counters");
         CK(irt_launch_lighting(L, kStageReuse, st), "reuse kernel");
         mark(s, 2, st);
         CK(irt_launch_lighting(L, kStageSpatial, st), "spatial kernel");
         mark(s, 3, st);
-        MarchLaunch M{};
-        M.frame = f;
-        M.objects = sc->objects;
-        M.meshes = sc->meshes;
-        M.nodes = sc->nodes;
-        M.atlas = sc->atlas;
-        M.sdf_f16 = sc->sdf_f16;
-        M.sdf_cells = sc->sdf_cells;
-        M.field_filter = scene_field_filter(sc);
-        M.error = s->error;
-        M.march_scene = sc->march_scene;
-        M.cells = sc->cells;
-        for (int a = 0; a < 3; a++) {
-            M.grid_org[a] = sc->grid_org[a];
-            M.grid_inv[a] = sc->grid_inv[a];
-        }
-        M.rays = s->rays;
-        M.ray_counters = s->ray_counters;
-        M.vis = s->vis;
-        M.num_sms = s->num_sms;
-        M.fast = s->desc.exact_march ? 0 : 1;
         CK(irt_launch_march(M, st), "march kernel");
         if (s->pipe.ready) CK(cudaEventRecord(s->pipe.march_done, st), "pipeline event");
         mark(s, 4, st);

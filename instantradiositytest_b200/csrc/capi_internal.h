@@ -109,6 +109,10 @@ struct irt_session {
     cudaEvent_t ev[kProfRing][kProfEvents] = {};
     // ray-queue resolve buffers
     RayRecord* rays = nullptr;
+    uint16_t* ray_hints = nullptr;
+    float4* prep = nullptr;         // per pixel: surface normal, light of its direct ray
+    uint32_t* prep_vpl = nullptr;   // per pixel: VPL of its indirect ray
+    float4* ray_ends = nullptr;     // march endpoints of the pools' and the archive's VPLs, or null
     uint32_t* ray_counters = nullptr;
     float* vis = nullptr;
     float4* pending = nullptr;
@@ -141,6 +145,27 @@ struct irt_session {
     int prof_slot = 0;
     uint32_t prof_frame[kProfRing] = {};
 };
+
+// The ray set-up of a session's frame over its scene and the caller's pools.
+inline RaySetup session_ray_setup(const irt_session* s, const irt_scene* sc, const irt_vpl* cur,
+                                  const irt_vpl* prev) {
+    RaySetup r{};
+    r.guide = s->guide[0];
+    r.prep = s->prep;
+    r.prep_vpl = s->prep_vpl;
+    r.lights = sc->lights_prep;
+    r.cur = cur;
+    r.prev = prev;
+    r.arch = s->archive;
+    r.ends = s->ray_ends;
+    r.rays = s->rays;
+    r.hints = s->ray_hints;
+    r.counters = s->ray_counters;
+    r.vis = s->vis;
+    r.vpl_count = s->desc.settings.vpl_count;
+    r.slots = s->desc.settings.restir_max_history + 1u;
+    return r;
+}
 
 namespace {
 

@@ -258,9 +258,12 @@ __device__ __forceinline__ float march_top(const MarchState& m, uint32_t max_ste
 }
 __device__ __forceinline__ float march_begin(MarchState& m, V3 endpoint, float eps, uint32_t max_steps) {
     V3 delta = endpoint - m.origin;
-    m.limit = length(delta) - eps;
+    // The contraction of dot(delta, delta) is spelled out: left to the
+    // compiler, its order differed between the places this is inlined at.
+    const float len = sqrtf(fmaf(delta.z, delta.z, fmaf(delta.x, delta.x, delta.y * delta.y)));
+    m.limit = len - eps;
     if (m.limit <= 0.f) return 1.f;
-    m.dir = normalize(delta);
+    m.dir = delta / len;
     m.t = eps;
     m.result = 1.f;
     m.previous = 1e20f;

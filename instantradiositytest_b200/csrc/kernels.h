@@ -23,17 +23,44 @@ struct FieldFilter {
 // spatial_direct, spatial_indirect, resolve_direct, resolve_indirect).
 constexpr int kStageReuse = 100;    // fused 0..3
 constexpr int kStageShade = 101;    // fused 4..7 with the march inline (one thread per pixel)
-constexpr int kStageSpatial = 102;  // fused 4..5 + resolve set-up: emits visibility rays
+constexpr int kStageSpatial = 102;  // fused 4..5 + resolve set-up: names each pixel's visibility rays
 constexpr int kStageCombine = 103;  // resolve 6..7 from contributions x visibility
-constexpr int kStageArchive = 104;  // batched: VPL archive slot copy + ray-counter reset
 
-// A visibility ray of the resolve passes (sdf.wgsl:61-81 arguments), 64 bytes:
-//   a = (p.xyz, bits(pixel * 2 + kind))  kind 0 = direct, 1 = indirect
-//   b = (n.xyz, 1 if the endpoint is offset along end_normal else 0)
-//   c = (target.xyz, 0), d = (end_normal.xyz, 0)
+// A visibility ray of the resolve passes (sdf.wgsl:61-81) as its march
+// begins, 32 bytes: a = (origin.xyz, bits(pixel * 2 + kind)) with the surface
+// clearance applied, kind 0 = direct, 1 = indirect; b = (direction.xyz,
+// length).  The object nearest the surface point (the march's first hint) is
+// in a 16-bit array beside the records.
 struct RayRecord {
-    float4 a, b, c, d;
+    float4 a, b;
 };
+
+// What the ray set-up of a frame reads and writes (march.cu).
+struct RaySetup {
+    // From the spatial pass, per pixel: prep = (surface normal, bits(light id
+    // of its direct ray)), prep_vpl = VPL of its indirect ray; kNoRay = none.
+    // VPL v < vpl_count is entry v of the current pool, v < 2 * vpl_count
+    // entry v - vpl_count of the previous one, else of the archive.
+    const float4* guide;
+    float4* prep;
+    uint32_t* prep_vpl;
+    const irt_light* lights;
+    const irt_vpl* cur;
+    const irt_vpl* prev;
+    irt_vpl* arch;
+    // March endpoints of every VPL (the same order), or null: one query per ray.
+    float4* ends;
+    RayRecord* rays;     // capacity 2 * W * H
+    uint16_t* hints;     // capacity 2 * W * H
+    uint32_t* counters;  // [0] VPL rays (queue front), [1] rays fetched by the march, [2] light rays (back)
+    float* vis;          // visibility per pixel * 2 + kind
+    uint32_t vpl_count, slots;
+};
+constexpr uint32_t kNoRay = 0xffffffffu;
+// VPLs whose endpoints a session tabulates: the two pools and the archive.
+inline uint64_t irt_ray_pool_entries(uint32_t vpl_count, uint32_t max_history) {
+    return (uint64_t)vpl_count * (max_history + 3u);
+}
 
 struct LightingLaunch {
     const irt_frame* frame;
@@ -62,8 +89,8 @@ struct LightingLaunch {
     const float4* old_guide;  // ... of the previous frame's pixels
     const float4* feat;       // decoded normal/colour/params of this frame's pixels (f16, packed), or null
     // ray-queue resolve (kStageSpatial / march / kStageCombine)
-    RayRecord* rays;         // capacity 2 * W * H
-    uint32_t* ray_counters;  // [0] VPL rays (queue front), [1] rays fetched by the march, [2] light rays (back)
+    float4* prep;            // per pixel (RaySetup)
+    uint32_t* prep_vpl;
     float* vis;              // visibility per pixel * 2 + kind
     float4* pending;         // per pixel: direct contribution (w = 1: x vis), indirect (w = 1: x vis)
 };
@@ -84,12 +111,13 @@ struct MarchLaunch {
     // BVH leaf box, with those distances and the next one as a sentinel.
     const uint4* cells;
     float grid_org[3], grid_inv[3];
-    const RayRecord* rays;
-    uint32_t* ray_counters;
-    float* vis;
+    RaySetup setup;
     int num_sms;
     int fast;  // 1: approximate division / square root build (march_fast.cu)
 };
+// The frame's VPL archive slot, ray-counter reset and VPL endpoints (before
+// the lighting passes); the ray set-up and the march (after them).
+cudaError_t irt_launch_ray_pools(const MarchLaunch& M, cudaStream_t st);
 cudaError_t irt_launch_march(const MarchLaunch& M, cudaStream_t st);
 // Bytes of the compact march scene of `object_count` objects: 2N-1 nodes of
 // 32 bytes, then N object records of 176 bytes (mesh folded in).
@@ -197,10 +225,9 @@ cudaError_t irt_launch_svgf_spatial_batched(const BatchLaunch& B, int stage, cud
 // staged in shared memory once per CTA and the group's ray queues (one per
 // view) are consumed in order.
 struct MarchQueue {
-    const RayRecord* rays;
-    uint32_t* counters;  // [0] rays at the front, [1] rays fetched, [2] rays at the back
-    float* vis;
-    uint32_t cap;        // records (2 * W * H)
+    RaySetup setup;
+    const irt_frame* frame;  // the view's entry of the batch's device frame table
+    uint32_t width, height;
 };
 struct alignas(16) MarchGroup {
     irt_frame f;                // counts[3] and sdf[] of the group's views
@@ -227,6 +254,7 @@ struct MarchBatch {
     int blocks_per_sm;          // 0 = occupancy maximum
     int fast;
 };
+cudaError_t irt_launch_ray_pools_batched(const MarchBatch& M, cudaStream_t st);
 cudaError_t irt_launch_march_batched(const MarchBatch& M, cudaStream_t st);
 // Lights with the spot direction normalised and cos(angle / 2) in
 // direction_angle, the form the lighting kernels read.

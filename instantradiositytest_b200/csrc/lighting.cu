@@ -33,8 +33,8 @@ struct LightArgs {
     irt_reservoir* ires[3];
     float4* direct_out;  // resolve_direct output (f32x4), may be null in fused mode
     void* noisy_out;     // resolve_indirect output (radiance format)
-    RayRecord* rays;
-    uint32_t* ray_counters;
+    float4* prep;
+    uint32_t* prep_vpl;
     const float* vis;
     float4* pending;
     const float4* guide;      // world positions of this frame's pixels
@@ -134,6 +134,13 @@ struct Px {
     __device__ __forceinline__ bool vpl_sample_valid(const Res& r) const {
         return r.generation == f.size[3] && r.target > 0.f && r.id < f.counts[1] &&
                f.size[2] - r.source <= to_u32(f.rr[2]);
+    }
+    // The selected VPL's index in the frame's pools (RaySetup).
+    __device__ __forceinline__ uint32_t selected_index(const Res& r) const {
+        const uint32_t n = f.counts[1];
+        if (r.source == f.size[2]) return r.id;
+        if (r.source + 1u == f.size[2]) return n + r.id;
+        return (2u + r.source % (to_u32(f.rr[2]) + 1u)) * n + r.id;
     }
     // lighting.wgsl:25-29
     __device__ __forceinline__ DVpl selected_vpl(const Res& r) const {
@@ -355,108 +362,63 @@ __global__ void __launch_bounds__(256) shade_kernel(const __grid_constant__ irt_
 // ---------------------------------------------------------------- ray-queue resolve
 // spatial_direct + spatial_indirect, then the resolve passes up to their
 // visibility call: the pixel's contribution value * normalization is stored
-// and, where the reference would march, a ray is appended to the queue
-// (warp-aggregated: one atomic per ray class per warp).  Lanes of
-// out-of-image pixels stay in the warp until the append so every ballot sees
-// all 32 lanes.  VPL rays fill the queue from the front and light rays from
-// the back (ray_slot), so the march takes whole runs of one class and
-// neighbouring queue entries take the same phases (a VPL ray has one more
-// clearance query); each ray's result slot is in its record, so the order
-// changes no result.  The records' fields stay in registers (no indexed
-// local array).
-// Queue ends of the two ray classes: counter 0 fills from the front, 2 from the back.
-constexpr uint32_t kVplCounter = 0, kLightCounter = 2;
-
+// and, where the reference would march, the ray is named — the surface
+// normal, the light and the VPL (20 bytes a pixel); the set-up kernel of the
+// march (march.cu) turns them into ray records.
 template <class G, class R>
 __device__ __forceinline__ void spatial_prep_body(const irt_frame& f, const LightArgs<G>& a, uint32_t x, uint32_t y) {
-    const bool in = x < f.size[0] && y < f.size[1];
-    bool ray_d = false, ray_i = false;
-    V3 sp{0.f, 0.f, 0.f}, sn{0.f, 0.f, 0.f}, lpos{0.f, 0.f, 0.f}, vpos{0.f, 0.f, 0.f}, vnrm{0.f, 0.f, 0.f};
-    size_t id = 0;
-    if (in) {
-        Px<G> px(f, a, x, y);
-        id = px.id;
-        bool ok = px.valid();
-        Surface s;
-        if (ok) s = px.surface();
-        Res rd = px.template spatial<0>(res_load(a.dres[1], px.id), ok, s);
-        res_store(a.dres[2], px.id, rd);
-        Res ri = px.template spatial<1>(res_load(a.ires[1], px.id), ok, s);
-        res_store(a.ires[2], px.id, ri);
-        // resolve_direct (lighting.wgsl:106-122) up to visibility()
-        float4 pd = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t dbg = f.flags[2];
-        if (ok) {
-            if (rd.target > 0.f && dbg != 2u && dbg < 3u && index_ok(a.sc.error, rd.id, f.counts[0])) {
-                DLight l = load_light(a.sc.lights, rd.id);
-                V3 value = direct(s, l);
-                if (luminance(value) > 0.f) {
-                    float k = normalization(rd);
-                    pd = make_float4(value.x * k, value.y * k, value.z * k, 1.f);
-                    ray_d = true;
-                    lpos = xyz(l.ps);
-                }
-            }
-            if (dbg == 3u) pd = make_float4(s.color.x, s.color.y, s.color.z, 0.f);
-            if (dbg == 4u) pd = make_float4(s.n.x * .5f + .5f, s.n.y * .5f + .5f, s.n.z * .5f + .5f, 0.f);
-            if (dbg == 5u) {
-                float2 m = a.g.mv(px.id);
-                pd = make_float4(wclamp(.5f + m.x * 50.f, 0.f, 1.f), wclamp(.5f + m.y * 50.f, 0.f, 1.f), .5f, 0.f);
-            }
-        }
-        // resolve_indirect (lighting.wgsl:123-134) up to visibility()
-        float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ok && dbg != 1u && dbg < 3u && px.vpl_sample_valid(ri)) {
-            DVpl smp = px.selected_vpl(ri);
-            V3 value = indirect(s, smp);
+    if (x >= f.size[0] || y >= f.size[1]) return;
+    Px<G> px(f, a, x, y);
+    const size_t id = px.id;
+    bool ok = px.valid();
+    Surface s;
+    if (ok) s = px.surface();
+    Res rd = px.template spatial<0>(res_load(a.dres[1], px.id), ok, s);
+    res_store(a.dres[2], px.id, rd);
+    Res ri = px.template spatial<1>(res_load(a.ires[1], px.id), ok, s);
+    res_store(a.ires[2], px.id, ri);
+    uint32_t ray_d = kNoRay, ray_i = kNoRay;
+    // resolve_direct (lighting.wgsl:106-122) up to visibility()
+    float4 pd = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t dbg = f.flags[2];
+    if (ok) {
+        if (rd.target > 0.f && dbg != 2u && dbg < 3u && index_ok(a.sc.error, rd.id, f.counts[0])) {
+            DLight l = load_light(a.sc.lights, rd.id);
+            V3 value = direct(s, l);
             if (luminance(value) > 0.f) {
-                float k = normalization(ri);
-                pi = make_float4(value.x * k, value.y * k, value.z * k, 1.f);
-                ray_i = true;
-                vpos = xyz(smp.pos);
-                vnrm = xyz(smp.nrm);
+                float k = normalization(rd);
+                pd = make_float4(value.x * k, value.y * k, value.z * k, 1.f);
+                ray_d = rd.id;
             }
         }
-        if (ray_d || ray_i) {
-            sp = s.p;
-            sn = s.n;
+        if (dbg == 3u) pd = make_float4(s.color.x, s.color.y, s.color.z, 0.f);
+        if (dbg == 4u) pd = make_float4(s.n.x * .5f + .5f, s.n.y * .5f + .5f, s.n.z * .5f + .5f, 0.f);
+        if (dbg == 5u) {
+            float2 m = a.g.mv(px.id);
+            pd = make_float4(wclamp(.5f + m.x * 50.f, 0.f, 1.f), wclamp(.5f + m.y * 50.f, 0.f, 1.f), .5f, 0.f);
         }
-        a.pending[id * 2] = pd;
-        a.pending[id * 2 + 1] = pi;
     }
-    // Warp-aggregated append.
-    const unsigned full = 0xffffffffu;
-    // lane within the warp for any 2-D block shape (warps take consecutive linear thread ids)
-    const uint32_t lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31u;
-    const unsigned bd = __ballot_sync(full, ray_d), bi = __ballot_sync(full, ray_i);
-    const uint32_t nd = (uint32_t)__popc(bd), ni = (uint32_t)__popc(bi);
-    // VPL rays from the front of the queue, light rays from the back
-    // (ray_slot), so the march takes all VPL rays, then all light rays.
-    uint32_t base_i = 0, base_d = 0;
-    if (lane == 0) {
-        if (ni) base_i = atomicAdd(a.ray_counters + kVplCounter, ni);
-        if (nd) base_d = atomicAdd(a.ray_counters + kLightCounter, nd);
+    // resolve_indirect (lighting.wgsl:123-134) up to visibility()
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ok && dbg != 1u && dbg < 3u && px.vpl_sample_valid(ri)) {
+        DVpl smp = px.selected_vpl(ri);
+        V3 value = indirect(s, smp);
+        if (luminance(value) > 0.f) {
+            float k = normalization(ri);
+            pi = make_float4(value.x * k, value.y * k, value.z * k, 1.f);
+            ray_i = px.selected_index(ri);
+        }
     }
-    base_i = __shfl_sync(full, base_i, 0);
-    base_d = __shfl_sync(full, base_d, 0);
-    const uint32_t cap = 2u * f.size[0] * f.size[1];
-    const unsigned below = (1u << lane) - 1u;
-    if (ray_d) {
-        const uint32_t k = base_d + (uint32_t)__popc(bd & below);
-        float4* r = reinterpret_cast<float4*>(a.rays + (kLightCounter == 0 ? k : cap - 1u - k));
-        r[0] = make_float4(sp.x, sp.y, sp.z, __uint_as_float((uint32_t)(id * 2)));
-        r[1] = make_float4(sn.x, sn.y, sn.z, 0.f);
-        r[2] = make_float4(lpos.x, lpos.y, lpos.z, 0.f);
-        r[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+    a.pending[id * 2] = pd;
+    a.pending[id * 2 + 1] = pi;
+    float4 prep = make_float4(0.f, 0.f, 0.f, __uint_as_float(ray_d));
+    if (ok) {
+        prep.x = s.n.x;
+        prep.y = s.n.y;
+        prep.z = s.n.z;
     }
-    if (ray_i) {
-        const uint32_t k = base_i + (uint32_t)__popc(bi & below);
-        float4* r = reinterpret_cast<float4*>(a.rays + (kVplCounter == 0 ? k : cap - 1u - k));
-        r[0] = make_float4(sp.x, sp.y, sp.z, __uint_as_float((uint32_t)(id * 2 + 1)));
-        r[1] = make_float4(sn.x, sn.y, sn.z, 1.f);
-        r[2] = make_float4(vpos.x, vpos.y, vpos.z, 0.f);
-        r[3] = make_float4(vnrm.x, vnrm.y, vnrm.z, 0.f);
-    }
+    a.prep[id] = prep;
+    a.prep_vpl[id] = ray_i;
 }
 
 template <class G, class R>
@@ -599,25 +561,6 @@ __global__ void __launch_bounds__(256) combine_batched(const irt_frame* __restri
                     (size_t)(blockIdx.x - __ldg(tile_start + v)) * blockDim.x + threadIdx.x);
 }
 
-// VPL archive slot frame % (H+1) of every view, and the ray-queue counters
-// reset (src/renderer.rs:1873-1884).
-template <class G>
-__global__ void __launch_bounds__(256) archive_batched(const irt_frame* __restrict__ frames,
-                                                       const LightArgs<G>* __restrict__ args, uint32_t n) {
-    const uint32_t v = blockIdx.y;
-    if (v >= n) return;
-    const irt_frame& f = frames[v];
-    const LightArgs<G>& a = args[v];
-    const uint32_t count = f.counts[1];
-    const uint32_t slots = to_u32(f.rr[2]) + 1u;
-    const uint32_t slot = f.size[2] % slots;
-    const float4* src = reinterpret_cast<const float4*>(a.cur);
-    float4* dst = reinterpret_cast<float4*>(const_cast<irt_vpl*>(a.arch) + (size_t)slot * count);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count * 3u; i += gridDim.x * blockDim.x)
-        dst[i] = src[i];
-    if (blockIdx.x == 0 && threadIdx.x < 4) a.ray_counters[threadIdx.x] = 0u;
-}
-
 // ---------------------------------------------------------------- host launchers
 template <class G>
 static LightArgs<G> make_args(const LightingLaunch& L) {
@@ -647,8 +590,8 @@ static LightArgs<G> make_args(const LightingLaunch& L) {
     }
     a.direct_out = L.direct_out;
     a.noisy_out = L.noisy_out;
-    a.rays = L.rays;
-    a.ray_counters = L.ray_counters;
+    a.prep = L.prep;
+    a.prep_vpl = L.prep_vpl;
     a.vis = L.vis;
     a.pending = L.pending;
     a.guide = L.guide;
@@ -693,7 +636,6 @@ static cudaError_t launch_batched_typed(const BatchLaunch& B, int stage, cudaStr
     case kStageReuse: reuse_batched<G><<<B.tiles, block, 0, st>>>(frames, args, B.tile_start, B.n, B.keep); break;
     case kStageSpatial: spatial_prep_batched<G, R><<<B.tiles, block, 0, st>>>(frames, args, B.tile_start, B.n); break;
     case kStageCombine: combine_batched<G, R><<<B.tiles, 256, 0, st>>>(frames, args, B.tile_start, B.n); break;
-    case kStageArchive: archive_batched<G><<<dim3(8, B.n), 256, 0, st>>>(frames, args, B.n); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

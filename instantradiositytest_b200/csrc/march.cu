@@ -1,10 +1,15 @@
-// march.cu — persistent soft-shadow march over the ray queue.
+// march.cu — soft-shadow visibility of the frame's rays: ray set-up and a
+// persistent march over the ray queue.
 //
-// visibility() of sdf.wgsl:61-81 restated as a per-lane state machine over
-// its scene_distance queries: the clearance query at the surface point, the
-// endpoint clearance query for VPL rays, then up to sdf_max_steps march
-// steps.  A lane that finishes its ray refills from its warp's reserved
-// slice of the queue (one atomic per 32 entries, the records prefetched).
+// visibility() of sdf.wgsl:61-81 is a clearance query at the surface point,
+// for VPL rays one at the endpoint, then up to sdf_max_steps march steps, each
+// a scene_distance query.  The first two do not depend on the ray: a pixel's
+// two rays leave the same surface point, and all rays to a VPL share its
+// endpoint.  So they run once per pixel and once per VPL, in coherent kernels
+// of their own (ray_pools_kernel, ray_setup_kernel), with the same operations
+// on the same operands, and the persistent march holds march steps only.  It
+// restates them as a per-lane state machine; lanes that finish their rays
+// refill together from their warp's reserved slice of the queue.
 //
 // scene_distance (sdf.wgsl:42-60) returns the minimum object distance: the
 // walk skips a subtree only when its box bound exceeds the current best, and
@@ -44,7 +49,6 @@ namespace fast {
 namespace exact {
 #endif
 
-enum : uint32_t { kClear = 0, kEndpoint = 1, kMarch = 2 };
 // Resident warps: 64 registers a thread, no spills, 32 warps per SM.  In
 // CTAs of 128 threads (the batched march): 9 CTAs at 56 registers spill and
 // measured 3.82 ms, 7 CTAs 3.78 ms, 8 CTAs 3.56 ms per 1920x1200 frame.  The
@@ -95,7 +99,8 @@ struct Query {
     V3 p;
     float best;
     uint32_t closest, hint;
-    int32_t cur;          // next candidate: -1 hint, 0..7 cache entries, 8 after them, >= kAll all leaves
+    uint32_t oid;         // the object to evaluate next, or kNone
+    int32_t cur;          // the candidate after it: 0..7 cache entries, 8 after them, >= kAll all leaves
     const uint32_t* cw;   // the point's cache cell, or null outside the grid
 };
 constexpr int32_t kAfterEntries = (int32_t)kCellEntries;
@@ -115,7 +120,8 @@ __device__ __forceinline__ void query_begin(Query& qy, const Grid& g, V3 p, uint
         const uint32_t cell = ((uint32_t)fz * kGridRes + (uint32_t)fy) * kGridRes + (uint32_t)fx;
         qy.cw = reinterpret_cast<const uint32_t*>(g.cells + (size_t)cell * (kCellWords / 4));
     }
-    qy.cur = hint < n ? -1 : (inside ? 0 : kAll);
+    qy.cur = inside ? 0 : kAll;
+    qy.oid = hint < n ? hint : kNone;  // the hint first, unconditionally
 }
 
 // The walk's pruning test of leaf `oid`'s box against the best so far.
@@ -134,10 +140,6 @@ __device__ __forceinline__ uint32_t query_next(Query& qy, const MNode* nodes, co
                                                uint32_t* err) {
     for (;;) {
         const int32_t c = qy.cur;
-        if (c < 0) {  // the hint, unconditionally
-            qy.cur = qy.cw ? 0 : kAll;
-            return qy.hint;
-        }
         if (c < kAfterEntries) {
             const uint32_t oid = (__ldg(qy.cw + (c >> 1)) >> ((c & 1) * 16)) & 0xffffu;
             if (__uint_as_float(__ldg(qy.cw + 4 + c)) > wmax(qy.best, 0.f) || oid == 0xffffu) {
@@ -173,39 +175,138 @@ __device__ __forceinline__ void query_eval(Query& qy, const DevScene& sc, const 
     }
 }
 
-// A completed query's step of visibility() (sdf.wgsl:61-81): after the
-// clearance query the ray leaves the surface (and, for a VPL, queries the
-// endpoint's clearance), after the endpoint query the march begins, after a
-// march query the penumbra update.  Returns the visibility once the ray is
-// resolved, else -1 with the ray's next query begun.
-__device__ __forceinline__ float query_finish(Query& qy, MarchState& m, uint32_t& phase, const float4* rec,
-                                              const Grid& grid, const MObj* objs, uint32_t n_obj, float eps, float k,
-                                              uint32_t max_steps) {
-    const float voxel = (phase != kMarch && qy.closest < n_obj) ? objs[qy.closest].meta.y : eps;
-    float out = -1.f;
-    if (phase == kClear) {
-        m.closest = qy.closest;
-        m.origin = m.origin + m.dir * clearance_epsilon(eps, voxel);
-        const V3 endn = xyz(__ldg(rec + 3));
-        if (dot(endn, endn) > .5f) {
-            phase = kEndpoint;
-        } else {
-            phase = kMarch;
-            out = march_begin(m, xyz(__ldg(rec + 2)), eps, max_steps);
+// One distance query from p without a hint, walked to its end: the nearest
+// object, or kNone.
+__device__ __forceinline__ uint32_t query_closest(const DevScene& sc, const Grid& g, const MNode* nodes,
+                                                  const MObj* objs, uint32_t n, V3 p) {
+    Query qy;
+    query_begin(qy, g, p, kNone, n);
+    for (;;) {
+        const uint32_t oid = query_next(qy, nodes, objs, n, sc.error);
+        if (oid == kNone) break;
+        query_eval(qy, sc, objs, oid);
+    }
+    return qy.closest;
+}
+
+// The scene as a kernel's CTA reads it.
+struct SceneRefs {
+    const MNode* nodes;
+    const MObj* objs;
+    uint32_t n_obj;
+    float eps;
+    uint32_t max_steps;
+};
+__device__ __forceinline__ SceneRefs scene_refs(const irt_frame& f, const float4* smem) {
+    const uint32_t n = f.counts[3];
+    return SceneRefs{reinterpret_cast<const MNode*>(smem), reinterpret_cast<const MObj*>(smem + 2 * (2 * n - 1)), n,
+                     f.sdf[1], to_u32(f.sdf[0])};
+}
+
+// A point moved off the surface along its normal (sdf.wgsl:63, :66).
+__device__ __forceinline__ V3 cleared(V3 p, V3 n, uint32_t closest, const SceneRefs& R) {
+    const float voxel = closest < R.n_obj ? R.objs[closest].meta.y : R.eps;
+    return p + n * clearance_epsilon(R.eps, voxel);
+}
+
+// March endpoint of a VPL: cleared, when it has a normal.
+__device__ __forceinline__ V3 vpl_endpoint(const DevScene& sc, const Grid& g, const SceneRefs& R, V3 pos, V3 nrm) {
+    if (!(dot(nrm, nrm) > .5f)) return pos;
+    return cleared(pos, nrm, query_closest(sc, g, R.nodes, R.objs, R.n_obj, pos), R);
+}
+
+__device__ __forceinline__ const irt_vpl* pool_vpl(const RaySetup& s, uint32_t v) {
+    const uint32_t n = s.vpl_count;
+    return v < n ? s.cur + v : v < 2u * n ? s.prev + (v - n) : s.arch + (v - 2u * n);
+}
+
+// VPL archive slot frame % slots (src/renderer.rs:1873-1884), the queue's
+// reset, and every VPL's march endpoint: entry v of the frame's pools.
+__device__ __forceinline__ void ray_pool_entry(const RaySetup& s, const DevScene& sc, const Grid& g,
+                                               const SceneRefs& R, uint32_t frame_index, uint32_t v) {
+    const uint32_t n = s.vpl_count, first = (2u + frame_index % s.slots) * n;
+    const bool fresh = v >= first && v < first + n;  // the archive slot this frame's pool goes to
+    const float4* src = reinterpret_cast<const float4*>(fresh ? s.cur + (v - first) : pool_vpl(s, v));
+    const float4 pos = __ldg(src), nrm = __ldg(src + 1);
+    if (fresh) {
+        float4* dst = reinterpret_cast<float4*>(s.arch + (v - 2u * n));
+        dst[0] = pos;
+        dst[1] = nrm;
+        dst[2] = __ldg(src + 2);
+    }
+    if (s.ends) {
+        const V3 e = vpl_endpoint(sc, g, R, xyz(pos), xyz(nrm));
+        s.ends[v] = make_float4(e.x, e.y, e.z, 0.f);
+    }
+}
+
+// One warp's 8x4 pixels of the ray set-up: the pixel's clearance, the
+// begin of its rays' marches, and their records appended to the queue (one
+// atomic per ray class and warp).  VPL rays fill the queue from the front and
+// light rays from the back (ray_slot), so the march takes whole runs of one
+// class; each ray's result slot is in its record, so the order changes no
+// result.  Rays resolved without a march step write their visibility here.
+constexpr uint32_t kTileW = 8, kTileH = 4;
+__device__ __forceinline__ void ray_setup_tile(const RaySetup& s, const DevScene& sc, const Grid& g,
+                                               const SceneRefs& R, uint32_t W, uint32_t H, uint32_t tile,
+                                               uint32_t lane) {
+    const unsigned full = 0xffffffffu;
+    const uint32_t across = (W + kTileW - 1) / kTileW;
+    const uint32_t x = (tile % across) * kTileW + lane % kTileW, y = (tile / across) * kTileH + lane / kTileW;
+    const uint32_t i = y * W + x;
+    uint32_t light = kNoRay, vpl = kNoRay, hint = kNone;
+    MarchState d, v;
+    if (x < W && y < H) {
+        const float4 prep = __ldg(s.prep + i);
+        light = __float_as_uint(prep.w);
+        vpl = __ldg(s.prep_vpl + i);
+        if (light != kNoRay || vpl != kNoRay) {
+            const V3 p = xyz(__ldg(s.guide + i));
+            hint = query_closest(sc, g, R.nodes, R.objs, R.n_obj, p);
+            d.origin = cleared(p, xyz(prep), hint, R);
+            v.origin = d.origin;
         }
-    } else if (phase == kEndpoint) {
-        phase = kMarch;
-        const V3 target = xyz(__ldg(rec + 2)), endn = xyz(__ldg(rec + 3));
-        out = march_begin(m, target + endn * clearance_epsilon(eps, voxel), eps, max_steps);
-    } else {
-        m.closest = qy.closest;
-        out = march_after(m, qy.best, eps, k, max_steps);
+        if (light != kNoRay) {
+            const float out = march_begin(d, xyz(__ldg(reinterpret_cast<const float4*>(s.lights + light))), R.eps,
+                                          R.max_steps);
+            if (out >= 0.f) {
+                s.vis[2 * (size_t)i] = out;
+                light = kNoRay;
+            }
+        }
+        if (vpl != kNoRay) {
+            V3 end;
+            if (s.ends) {
+                end = xyz(__ldg(s.ends + vpl));
+            } else {
+                const float4* src = reinterpret_cast<const float4*>(pool_vpl(s, vpl));
+                end = vpl_endpoint(sc, g, R, xyz(__ldg(src)), xyz(__ldg(src + 1)));
+            }
+            const float out = march_begin(v, end, R.eps, R.max_steps);
+            if (out >= 0.f) {
+                s.vis[2 * (size_t)i + 1] = out;
+                vpl = kNoRay;
+            }
+        }
     }
-    if (out < 0.f) {
-        const V3 q = phase == kEndpoint ? xyz(__ldg(rec + 2)) : march_point(m);
-        query_begin(qy, grid, q, phase == kMarch ? m.closest : kNone, n_obj);
+    const unsigned bd = __ballot_sync(full, light != kNoRay), bi = __ballot_sync(full, vpl != kNoRay);
+    uint32_t base_i = 0, base_d = 0;
+    if (lane == 0) {
+        if (bi) base_i = atomicAdd(s.counters, (uint32_t)__popc(bi));
+        if (bd) base_d = atomicAdd(s.counters + 2, (uint32_t)__popc(bd));
     }
-    return out;
+    base_i = __shfl_sync(full, base_i, 0);
+    base_d = __shfl_sync(full, base_d, 0);
+    const uint32_t cap = 2u * W * H;
+    const unsigned below = (1u << lane) - 1u;
+    auto emit = [&](const MarchState& m, uint32_t at, uint32_t slot) {
+        if (!index_ok(sc.error, at, cap)) return;
+        s.rays[at].a = make_float4(m.origin.x, m.origin.y, m.origin.z, __uint_as_float(slot));
+        s.rays[at].b = make_float4(m.dir.x, m.dir.y, m.dir.z, m.limit);
+        s.hints[at] = (uint16_t)hint;
+    };
+    if (vpl != kNoRay) emit(v, base_i + (uint32_t)__popc(bi & below), 2u * i + 1u);
+    if (light != kNoRay) emit(d, cap - 1u - (base_d + (uint32_t)__popc(bd & below)), 2u * i);
 }
 
 // A warp's reserved slice [next, end) of a ray queue; `drained` once the
@@ -256,193 +357,249 @@ __device__ __forceinline__ uint32_t slice_take(RaySlice& s, unsigned need, uint3
     return idx;
 }
 
-__device__ __forceinline__ void march_reset(MarchState& m) {
-    m.closest = kNone;
-    m.origin = V3{0.f, 0.f, 0.f};
-    m.dir = V3{0.f, 0.f, 0.f};
-    m.t = m.limit = 0.f;
-    m.result = 1.f;
-    m.previous = 1e20f;
-    m.step = 0;
+// One lane's ray and the query of its current march step.
+struct Lane {
+    MarchState m;
+    Query qy;
+    uint32_t slot;
+    bool active;
+};
+__device__ __forceinline__ void lane_reset(Lane& L) {
+    L.m.closest = kNone;
+    L.m.origin = V3{0.f, 0.f, 0.f};
+    L.m.dir = V3{0.f, 0.f, 0.f};
+    L.m.t = L.m.limit = 0.f;
+    L.m.result = 1.f;
+    L.m.previous = 1e20f;
+    L.m.step = 0;
+    L.qy.cur = kQueryDone;
+    L.active = false;
+}
+// The ray of record `at`, as ray_setup_tile left it, and its first query.
+__device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t at, const Grid& grid,
+                                          const SceneRefs& R) {
+    const float4* r = reinterpret_cast<const float4*>(s.rays + at);
+    const float4 a = __ldg(r), b = __ldg(r + 1);
+    const uint32_t hint = __ldg(s.hints + at);
+    L.m.origin = V3{a.x, a.y, a.z};
+    L.m.dir = V3{b.x, b.y, b.z};
+    L.m.limit = b.w;
+    L.m.t = R.eps;
+    L.m.result = 1.f;
+    L.m.previous = 1e20f;
+    L.m.step = 0;
+    L.m.closest = hint;
+    L.slot = __float_as_uint(a.w);
+    L.active = true;
+    query_begin(L.qy, grid, march_point(L.m), hint, R.n_obj);
+}
+// One iteration of a warp's lanes, stage by stage: every active lane
+// evaluates its query's object; finds the next one; and where the query has
+// none left, completes its march step (sdf.wgsl:68-80) and begins the ray's
+// next query with its hint.  The lanes meet after each stage.
+__device__ __forceinline__ void lane_step(Lane& L, const DevScene& sc, const Grid& grid, const SceneRefs& R, float k,
+                                          float* vis, uint32_t cap) {
+    if (L.active && L.qy.oid != kNone) query_eval(L.qy, sc, R.objs, L.qy.oid);
+    __syncwarp();
+    if (L.active) L.qy.oid = query_next(L.qy, R.nodes, R.objs, R.n_obj, sc.error);
+    __syncwarp();
+    if (L.active && L.qy.oid == kNone) {
+        L.m.closest = L.qy.closest;
+        const float out = march_after(L.m, L.qy.best, R.eps, k, R.max_steps);
+        if (out >= 0.f) {
+            if (index_ok(sc.error, L.slot, cap)) vis[L.slot] = out;
+            L.active = false;
+        } else {
+            query_begin(L.qy, grid, march_point(L.m), L.m.closest, R.n_obj);
+        }
+    }
+    __syncwarp();
+}
+
+// Idle lanes a warp collects before it refills them, so that the refill's
+// instructions run for several lanes at once.
+constexpr int kRefill = 6;
+
+__global__ void __launch_bounds__(kMarchThreads) ray_pools_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
+                                                                  const float4* __restrict__ march_scene,
+                                                                  uint32_t scene_vec4, const Grid grid,
+                                                                  const __grid_constant__ RaySetup setup) {
+    extern __shared__ float4 smem[];
+    for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
+    __syncthreads();
+    const SceneRefs R = scene_refs(f, smem);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 4) setup.counters[t] = 0u;
+    const uint32_t n = (setup.slots + 2u) * setup.vpl_count;
+    for (uint32_t v = t; v < n; v += gridDim.x * blockDim.x) ray_pool_entry(setup, sc, grid, R, f.size[2], v);
+}
+
+__global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) ray_setup_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
+                                                                  const float4* __restrict__ march_scene,
+                                                                  uint32_t scene_vec4, const Grid grid,
+                                                                  const __grid_constant__ RaySetup setup) {
+    extern __shared__ float4 smem[];
+    for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
+    __syncthreads();
+    const SceneRefs R = scene_refs(f, smem);
+    const uint32_t W = f.size[0], H = f.size[1];
+    const uint32_t tiles = ((W + kTileW - 1) / kTileW) * ((H + kTileH - 1) / kTileH);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 32u; t < tiles; t += warps)
+        ray_setup_tile(setup, sc, grid, R, W, H, t, threadIdx.x & 31u);
 }
 
 __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) march_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
                                                     const float4* __restrict__ march_scene, uint32_t scene_vec4,
-                                                    const Grid grid, const RayRecord* __restrict__ rays,
-                                                    uint32_t* counters, float* __restrict__ vis) {
+                                                    const Grid grid, const __grid_constant__ RaySetup setup) {
     extern __shared__ float4 smem[];
     for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
     __syncthreads();
-    const uint32_t n_obj = f.counts[3];
-    const MNode* nodes = reinterpret_cast<const MNode*>(smem);
-    const MObj* objs = reinterpret_cast<const MObj*>(smem + 2 * (2 * n_obj - 1));
-
-    const uint32_t front = *(volatile uint32_t*)&counters[0];
-    const uint32_t n_rays = front + *(volatile uint32_t*)&counters[2];
+    const SceneRefs R = scene_refs(f, smem);
+    const uint32_t front = *(volatile uint32_t*)&setup.counters[0];
+    const uint32_t n_rays = front + *(volatile uint32_t*)&setup.counters[2];
     const uint32_t cap = 2u * f.size[0] * f.size[1];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const float eps = f.sdf[1];
-    const uint32_t max_steps = to_u32(f.sdf[0]);
 
-    bool active = false;
     bool exhausted = false;  // warp-uniform: the queue has no rays left
-    // A lane keeps its ray's index and re-reads the record's target, endpoint
-    // normal and output slot where a step needs them (L1/L2 hits), which
-    // keeps fewer values live across the loop.
-    uint32_t phase = kClear, ridx = 0;
-    MarchState m;
-    march_reset(m);
-    Query qy;
-    qy.cur = kQueryDone;
+    Lane L;
+    lane_reset(L);
     RaySlice slice{0u, 0u, false};
     const uint32_t keep = 2u * gridDim.x * (blockDim.x / 32u) * kRayChunk;
     for (;;) {
-        if (!exhausted) {
-            const unsigned need = __ballot_sync(full, !active);
-            if (need) {
-                const uint32_t idx = slice_take(slice, need, &counters[1], n_rays, keep, lane, rays, front, cap);
-                exhausted = slice.drained && slice.next >= slice.end;
-                if (!active) {
-                    if (idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap)) {
-                        ridx = ray_slot(idx, front, cap);
-                        const float4* r = reinterpret_cast<const float4*>(rays + ridx);
-                        float4 a = __ldg(r), b = __ldg(r + 1);
-                        m.origin = V3{a.x, a.y, a.z};  // surface point until the clearance query
-                        m.dir = V3{b.x, b.y, b.z};     // surface normal until the march begins
-                        phase = kClear;
-                        active = true;
-                        query_begin(qy, grid, m.origin, kNone, n_obj);
-                    }
-                }
-            }
+        const unsigned need = __ballot_sync(full, !L.active);
+        if (exhausted) {
+            if (need == full) break;
+        } else if (__popc(need) >= kRefill) {
+            const uint32_t idx = slice_take(slice, need, &setup.counters[1], n_rays, keep, lane, setup.rays, front, cap);
+            exhausted = slice.drained && slice.next >= slice.end;
+            if (!L.active && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap))
+                lane_take(L, setup, ray_slot(idx, front, cap), grid, R);
         }
-        if (!__any_sync(full, active)) break;
-        if (!active) continue;
-
-        uint32_t oid = query_next(qy, nodes, objs, n_obj, sc.error);
-        while (oid == kNone) {
-            const float4* rec = reinterpret_cast<const float4*>(rays + ridx);
-            const float out = query_finish(qy, m, phase, rec, grid, objs, n_obj, eps, f.sdf[2], max_steps);
-            if (out >= 0.f) {
-                const uint32_t slot = __float_as_uint(__ldg(rec).w);
-                if (index_ok(sc.error, slot, cap)) vis[slot] = out;
-                active = false;
-                break;
-            }
-            oid = query_next(qy, nodes, objs, n_obj, sc.error);
-        }
-        if (oid != kNone) query_eval(qy, sc, objs, oid);
+        lane_step(L, sc, grid, R, f.sdf[2], setup.vis, cap);
     }
 }
 
-// Batched march: for each scene group the CTA stages the group record and
-// its compact scene in shared memory, then its warps consume the group's ray
-// queues (one per view) in order with the same flattened loop; a lane keeps
-// the address of its ray record and the index of the queue it came from.
+// ---------------------------------------------------------------- batched views
+// For each scene group a CTA stages the group record and its compact scene in
+// shared memory, then runs the single-view bodies over the group's views.
 constexpr uint32_t kGroupVec4 = (uint32_t)((sizeof(MarchGroup) + 15) / 16);
 
+// Stages group g into smem; its scene follows the record.
+__device__ __forceinline__ const MarchGroup& stage_group(const MarchGroup* __restrict__ groups, uint32_t g,
+                                                         float4* smem) {
+    const MarchGroup& G = *reinterpret_cast<const MarchGroup*>(smem);
+    __syncthreads();  // every warp is done with the previous group's records
+    const float4* gsrc = reinterpret_cast<const float4*>(groups + g);
+    for (uint32_t i = threadIdx.x; i < kGroupVec4; i += blockDim.x) smem[i] = __ldg(gsrc + i);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < G.scene_vec4; i += blockDim.x) smem[kGroupVec4 + i] = __ldg(G.march_scene + i);
+    __syncthreads();
+    return G;
+}
+__device__ __forceinline__ DevScene group_scene(const MarchGroup& G) {
+    DevScene sc;
+    sc.objects = G.objects;
+    sc.meshes = G.meshes;
+    sc.nodes = G.nodes;
+    sc.lights = nullptr;
+    sc.atlas = G.atlas;
+    sc.sdf_f16 = G.sdf_f16;
+    sc.sdf_cells = G.sdf_cells;
+    sc.filter = G.field_filter;
+    sc.error = G.error;
+    return sc;
+}
+__device__ __forceinline__ Grid group_grid(const MarchGroup& G) {
+    return Grid{G.cells, G.grid_org[0], G.grid_org[1], G.grid_org[2], G.grid_inv[0], G.grid_inv[1], G.grid_inv[2]};
+}
+
+__global__ void __launch_bounds__(128) ray_pools_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
+                                                                const MarchQueue* __restrict__ queues) {
+    extern __shared__ float4 smem[];
+    for (uint32_t g = 0; g < n_groups; g++) {
+        const MarchGroup& G = stage_group(groups, g, smem);
+        const DevScene sc = group_scene(G);
+        const Grid grid = group_grid(G);
+        const SceneRefs R = scene_refs(G.f, smem + kGroupVec4);
+        // Entries of all the group's views in one run, so that small pools share the grid.
+        uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+        if (t < 4)
+            for (uint32_t q = G.q_begin; q < G.q_end; q++) queues[q].setup.counters[t] = 0u;
+        for (uint32_t q = G.q_begin; q < G.q_end; q++) {
+            const MarchQueue& Q = queues[q];
+            const uint32_t n = (Q.setup.slots + 2u) * Q.setup.vpl_count;
+            for (; t < n; t += gridDim.x * blockDim.x) ray_pool_entry(Q.setup, sc, grid, R, Q.frame->size[2], t);
+            t -= n;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(128, kMarchBlocksPerSm) ray_setup_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
+                                                            const MarchQueue* __restrict__ queues) {
+    extern __shared__ float4 smem[];
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t g = 0; g < n_groups; g++) {
+        const MarchGroup& G = stage_group(groups, g, smem);
+        const DevScene sc = group_scene(G);
+        const Grid grid = group_grid(G);
+        const SceneRefs R = scene_refs(G.f, smem + kGroupVec4);
+        uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
+        for (uint32_t q = G.q_begin; q < G.q_end; q++) {
+            const MarchQueue& Q = queues[q];
+            const uint32_t tiles = ((Q.width + kTileW - 1) / kTileW) * ((Q.height + kTileH - 1) / kTileH);
+            const RaySetup s = Q.setup;
+            for (; t < tiles; t += warps) ray_setup_tile(s, sc, grid, R, Q.width, Q.height, t, threadIdx.x & 31u);
+            t -= tiles;
+        }
+    }
+}
+
+// The march over a group's queues in order; a lane keeps its queue's index.
 __global__ void __launch_bounds__(128, kMarchBlocksPerSm) march_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
                                                             const MarchQueue* __restrict__ queues) {
     extern __shared__ float4 smem[];
-    const MarchGroup& G = *reinterpret_cast<const MarchGroup*>(smem);
-    float4* scene_smem = smem + kGroupVec4;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     for (uint32_t g = 0; g < n_groups; g++) {
-        __syncthreads();  // every warp is done with the previous group's records
-        const float4* gsrc = reinterpret_cast<const float4*>(groups + g);
-        for (uint32_t i = threadIdx.x; i < kGroupVec4; i += blockDim.x) smem[i] = __ldg(gsrc + i);
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < G.scene_vec4; i += blockDim.x) scene_smem[i] = __ldg(G.march_scene + i);
-        __syncthreads();
-        const irt_frame& f = G.f;
-        DevScene sc;
-        sc.objects = G.objects;
-        sc.meshes = G.meshes;
-        sc.nodes = G.nodes;
-        sc.lights = nullptr;
-        sc.atlas = G.atlas;
-        sc.sdf_f16 = G.sdf_f16;
-        sc.sdf_cells = G.sdf_cells;
-        sc.filter = G.field_filter;
-        sc.error = G.error;
-        Grid grid;
-        grid.cells = G.cells;
-        grid.ox = G.grid_org[0];
-        grid.oy = G.grid_org[1];
-        grid.oz = G.grid_org[2];
-        grid.ix = G.grid_inv[0];
-        grid.iy = G.grid_inv[1];
-        grid.iz = G.grid_inv[2];
-        const uint32_t n_obj = f.counts[3];
-        const MNode* nodes = reinterpret_cast<const MNode*>(scene_smem);
-        const MObj* objs = reinterpret_cast<const MObj*>(scene_smem + 2 * (2 * n_obj - 1));
-        const float eps = f.sdf[1];
-        const uint32_t max_steps = to_u32(f.sdf[0]);
-
+        const MarchGroup& G = stage_group(groups, g, smem);
+        const DevScene sc = group_scene(G);
+        const Grid grid = group_grid(G);
+        const SceneRefs R = scene_refs(G.f, smem + kGroupVec4);
         uint32_t q = G.q_begin;
         bool exhausted = q >= G.q_end;
-        uint32_t front = exhausted ? 0u : *(volatile const uint32_t*)&queues[q].counters[0];
-        uint32_t n_rays = exhausted ? 0u : front + *(volatile const uint32_t*)&queues[q].counters[2];
-        bool active = false;
-        uint32_t phase = kClear, lq = 0;
-        const float4* rec = nullptr;
-        MarchState m;
-        march_reset(m);
-        Query qy;
-        qy.cur = kQueryDone;
+        uint32_t front = exhausted ? 0u : *(volatile const uint32_t*)&queues[q].setup.counters[0];
+        uint32_t n_rays = exhausted ? 0u : front + *(volatile const uint32_t*)&queues[q].setup.counters[2];
+        uint32_t lq = 0;
+        Lane L;
+        lane_reset(L);
         RaySlice slice{0u, 0u, false};
         const uint32_t keep = 2u * gridDim.x * (blockDim.x / 32u) * kRayChunk;
         for (;;) {
-            if (!exhausted) {
-                const unsigned need = __ballot_sync(full, !active);
-                if (need) {
-                    const MarchQueue& Q = queues[q];
-                    const uint32_t idx = slice_take(slice, need, &Q.counters[1], n_rays, keep, lane, Q.rays, front,
-                                                    Q.cap);
-                    if (!active) {
-                        if (idx < n_rays && index_ok(sc.error, ray_slot(idx, front, Q.cap), Q.cap)) {
-                            rec = reinterpret_cast<const float4*>(Q.rays + ray_slot(idx, front, Q.cap));
-                            float4 a = __ldg(rec), b = __ldg(rec + 1);
-                            m.origin = V3{a.x, a.y, a.z};
-                            m.dir = V3{b.x, b.y, b.z};
-                            phase = kClear;
-                            lq = q;
-                            active = true;
-                            query_begin(qy, grid, m.origin, kNone, n_obj);
-                        }
-                    }
-                    if (slice.drained && slice.next >= slice.end) {  // this queue is used up: the next view's
-                        slice = RaySlice{0u, 0u, false};
-                        q++;
-                        if (q >= G.q_end) exhausted = true;
-                        else {
-                            front = *(volatile const uint32_t*)&queues[q].counters[0];
-                            n_rays = front + *(volatile const uint32_t*)&queues[q].counters[2];
-                        }
+            const unsigned need = __ballot_sync(full, !L.active);
+            if (exhausted) {
+                if (need == full) break;
+            } else if (__popc(need) >= kRefill) {
+                const MarchQueue& Q = queues[q];
+                const uint32_t cap = 2u * Q.width * Q.height;
+                const uint32_t idx = slice_take(slice, need, &Q.setup.counters[1], n_rays, keep, lane, Q.setup.rays,
+                                                front, cap);
+                if (!L.active && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap)) {
+                    lane_take(L, Q.setup, ray_slot(idx, front, cap), grid, R);
+                    lq = q;
+                }
+                if (slice.drained && slice.next >= slice.end) {  // this queue is used up: the next view's
+                    slice = RaySlice{0u, 0u, false};
+                    q++;
+                    if (q >= G.q_end) exhausted = true;
+                    else {
+                        front = *(volatile const uint32_t*)&queues[q].setup.counters[0];
+                        n_rays = front + *(volatile const uint32_t*)&queues[q].setup.counters[2];
                     }
                 }
             }
-            if (!__any_sync(full, active)) {
-                if (exhausted) break;
-                continue;
-            }
-            if (!active) continue;
-
-            uint32_t oid = query_next(qy, nodes, objs, n_obj, sc.error);
-            while (oid == kNone) {
-                const float out = query_finish(qy, m, phase, rec, grid, objs, n_obj, eps, f.sdf[2], max_steps);
-                if (out >= 0.f) {
-                    float* vis = queues[lq].vis;
-                    const uint32_t slot = __float_as_uint(__ldg(rec).w);
-                    if (index_ok(sc.error, slot, queues[lq].cap)) vis[slot] = out;
-                    active = false;
-                    break;
-                }
-                oid = query_next(qy, nodes, objs, n_obj, sc.error);
-            }
-            if (oid != kNone) query_eval(qy, sc, objs, oid);
+            lane_step(L, sc, grid, R, G.f.sdf[2], queues[lq].setup.vis, 2u * queues[lq].width * queues[lq].height);
         }
     }
 }
@@ -452,10 +609,8 @@ __global__ void __launch_bounds__(128, kMarchBlocksPerSm) march_batched_kernel(c
 
 #if IRT_MARCH_FAST
 #define IRT_MARCH_NS irtd::fast
-#define IRT_MARCH_LAUNCH irt_launch_march_fast
 #else
 #define IRT_MARCH_NS irtd::exact
-#define IRT_MARCH_LAUNCH irt_launch_march_exact
 #endif
 
 // The carveout (percent of the SM's shared-memory maximum) that holds
@@ -475,27 +630,33 @@ static cudaError_t march_prefer_l1(const void* kernel, uint32_t smem, int blocks
     return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-cudaError_t IRT_MARCH_LAUNCH(const MarchLaunch& M, cudaStream_t st) {
-    using namespace irtd;
-    using namespace IRT_MARCH_NS;
-    const uint32_t smem = irt_march_scene_bytes(M.frame->counts[3]);
-    thread_local int configured_device = -1;
-    thread_local uint32_t configured_smem = 0;
-    thread_local int blocks_per_sm = 0;
-    int device = 0;
-    cudaGetDevice(&device);
-    if (smem != configured_smem || device != configured_device) {
-        configured_device = device;
-        cudaError_t e = cudaFuncSetAttribute(march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+namespace {
+
+// Per thread and device: a kernel's dynamic shared memory attribute and its
+// resident CTAs per SM for that size.
+struct KernelFit {
+    int device = -1;
+    uint32_t smem = 0;
+    int per_sm = 0;
+
+    cudaError_t set(const void* kernel, int threads, uint32_t bytes, int prefer_blocks) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev == device && bytes == smem) return cudaSuccess;
+        device = dev;
+        smem = 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) e = march_prefer_l1(kernel, bytes, prefer_blocks);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes);
         if (e != cudaSuccess) return e;
-        e = march_prefer_l1((const void*)march_kernel, smem, kMarchCtasPerSm);
-        if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, march_kernel, kMarchThreads, smem);
-        if (e != cudaSuccess) return e;
-        if (blocks_per_sm < 1) return cudaErrorInvalidConfiguration;
-        configured_smem = smem;
+        if (per_sm < 1) return cudaErrorInvalidConfiguration;
+        smem = bytes;
+        return cudaSuccess;
     }
-    DevScene sc;
+};
+
+irtd::DevScene launch_scene(const MarchLaunch& M) {
+    irtd::DevScene sc;
     sc.objects = M.objects;
     sc.meshes = M.meshes;
     sc.nodes = M.nodes;
@@ -505,65 +666,95 @@ cudaError_t IRT_MARCH_LAUNCH(const MarchLaunch& M, cudaStream_t st) {
     sc.sdf_cells = M.sdf_cells;
     sc.filter = M.field_filter;
     sc.error = M.error;
-    Grid g;
-    g.cells = M.cells;
-    g.ox = M.grid_org[0];
-    g.oy = M.grid_org[1];
-    g.oz = M.grid_org[2];
-    g.ix = M.grid_inv[0];
-    g.iy = M.grid_inv[1];
-    g.iz = M.grid_inv[2];
-    march_kernel<<<M.num_sms * blocks_per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g, M.rays,
-                                                                M.ray_counters, M.vis);
+    return sc;
+}
+IRT_MARCH_NS::Grid launch_grid(const MarchLaunch& M) {
+    return IRT_MARCH_NS::Grid{M.cells,        M.grid_org[0], M.grid_org[1], M.grid_org[2],
+                              M.grid_inv[0], M.grid_inv[1], M.grid_inv[2]};
+}
+
+}  // namespace
+
+#if IRT_MARCH_FAST
+#define IRT_MARCH_FN(name) name##_fast
+#else
+#define IRT_MARCH_FN(name) name##_exact
+#endif
+
+cudaError_t IRT_MARCH_FN(irt_launch_ray_pools)(const MarchLaunch& M, cudaStream_t st) {
+    using namespace IRT_MARCH_NS;
+    const uint32_t smem = irt_march_scene_bytes(M.frame->counts[3]);
+    thread_local KernelFit fit;
+    cudaError_t e = fit.set((const void*)ray_pools_kernel, kMarchThreads, smem, 1);
+    if (e != cudaSuccess) return e;
+    const uint32_t entries = (M.setup.slots + 2u) * M.setup.vpl_count;
+    const uint32_t blocks = std::min((uint32_t)M.num_sms, (entries + kMarchThreads - 1) / kMarchThreads);
+    ray_pools_kernel<<<blocks, kMarchThreads, smem, st>>>(*M.frame, launch_scene(M), M.march_scene, smem / 16,
+                                                          launch_grid(M), M.setup);
     return cudaGetLastError();
 }
 
-#if IRT_MARCH_FAST
-#define IRT_MARCH_BATCHED_LAUNCH irt_launch_march_batched_fast
-#else
-#define IRT_MARCH_BATCHED_LAUNCH irt_launch_march_batched_exact
-#endif
+cudaError_t IRT_MARCH_FN(irt_launch_march)(const MarchLaunch& M, cudaStream_t st) {
+    using namespace IRT_MARCH_NS;
+    const uint32_t smem = irt_march_scene_bytes(M.frame->counts[3]);
+    thread_local KernelFit set_up, march;
+    cudaError_t e = set_up.set((const void*)ray_setup_kernel, kMarchThreads, smem, kMarchCtasPerSm);
+    if (e == cudaSuccess) e = march.set((const void*)march_kernel, kMarchThreads, smem, kMarchCtasPerSm);
+    if (e != cudaSuccess) return e;
+    const irtd::DevScene sc = launch_scene(M);
+    const Grid g = launch_grid(M);
+    ray_setup_kernel<<<M.num_sms * set_up.per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
+                                                                             M.setup);
+    march_kernel<<<M.num_sms * march.per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
+                                                                        M.setup);
+    return cudaGetLastError();
+}
 
-cudaError_t IRT_MARCH_BATCHED_LAUNCH(const MarchBatch& M, cudaStream_t st) {
-    using namespace irtd;
+cudaError_t IRT_MARCH_FN(irt_launch_ray_pools_batched)(const MarchBatch& M, cudaStream_t st) {
     using namespace IRT_MARCH_NS;
     if (M.n_groups == 0) return cudaSuccess;
     const uint32_t smem = kGroupVec4 * 16 + M.max_scene_bytes;
-    thread_local int configured_device = -1;
-    thread_local uint32_t configured_smem = 0;
-    thread_local int max_blocks = 0;
-    int device = 0;
-    cudaGetDevice(&device);
-    if (smem != configured_smem || device != configured_device) {
-        configured_device = device;
-        cudaError_t e = cudaFuncSetAttribute(march_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        e = march_prefer_l1((const void*)march_batched_kernel, smem, kMarchBlocksPerSm);
-        if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_blocks, march_batched_kernel, 128, smem);
-        if (e != cudaSuccess) return e;
-        if (max_blocks < 1) return cudaErrorInvalidConfiguration;
-        configured_smem = smem;
-    }
-    const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < max_blocks ? M.blocks_per_sm : max_blocks;
+    thread_local KernelFit fit;
+    cudaError_t e = fit.set((const void*)ray_pools_batched_kernel, 128, smem, 1);
+    if (e != cudaSuccess) return e;
+    ray_pools_batched_kernel<<<M.num_sms * std::min(fit.per_sm, 2), 128, smem, st>>>(M.groups, M.n_groups, M.queues);
+    return cudaGetLastError();
+}
+
+cudaError_t IRT_MARCH_FN(irt_launch_march_batched)(const MarchBatch& M, cudaStream_t st) {
+    using namespace IRT_MARCH_NS;
+    if (M.n_groups == 0) return cudaSuccess;
+    const uint32_t smem = kGroupVec4 * 16 + M.max_scene_bytes;
+    thread_local KernelFit set_up, march;
+    cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, 128, smem, kMarchBlocksPerSm);
+    if (e == cudaSuccess) e = march.set((const void*)march_batched_kernel, 128, smem, kMarchBlocksPerSm);
+    if (e != cudaSuccess) return e;
+    const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < march.per_sm ? M.blocks_per_sm : march.per_sm;
+    ray_setup_batched_kernel<<<M.num_sms * set_up.per_sm, 128, smem, st>>>(M.groups, M.n_groups, M.queues);
     march_batched_kernel<<<M.num_sms * bps, 128, smem, st>>>(M.groups, M.n_groups, M.queues);
     return cudaGetLastError();
 }
 
 #if !IRT_MARCH_FAST
+cudaError_t irt_launch_ray_pools_fast(const MarchLaunch& M, cudaStream_t st);
+cudaError_t irt_launch_march_fast(const MarchLaunch& M, cudaStream_t st);
+cudaError_t irt_launch_ray_pools_batched_fast(const MarchBatch& M, cudaStream_t st);
 cudaError_t irt_launch_march_batched_fast(const MarchBatch& M, cudaStream_t st);
 
+cudaError_t irt_launch_ray_pools(const MarchLaunch& M, cudaStream_t st) {
+    return M.fast ? irt_launch_ray_pools_fast(M, st) : irt_launch_ray_pools_exact(M, st);
+}
+cudaError_t irt_launch_march(const MarchLaunch& M, cudaStream_t st) {
+    return M.fast ? irt_launch_march_fast(M, st) : irt_launch_march_exact(M, st);
+}
+cudaError_t irt_launch_ray_pools_batched(const MarchBatch& M, cudaStream_t st) {
+    return M.fast ? irt_launch_ray_pools_batched_fast(M, st) : irt_launch_ray_pools_batched_exact(M, st);
+}
 cudaError_t irt_launch_march_batched(const MarchBatch& M, cudaStream_t st) {
     return M.fast ? irt_launch_march_batched_fast(M, st) : irt_launch_march_batched_exact(M, st);
 }
 
 uint32_t irt_march_scene_bytes(uint32_t object_count) {
     return (2 * object_count - 1) * (uint32_t)sizeof(irtd::MNode) + object_count * (uint32_t)sizeof(irtd::MObj);
-}
-
-cudaError_t irt_launch_march_fast(const MarchLaunch& M, cudaStream_t st);
-
-cudaError_t irt_launch_march(const MarchLaunch& M, cudaStream_t st) {
-    return M.fast ? irt_launch_march_fast(M, st) : irt_launch_march_exact(M, st);
 }
 #endif
