@@ -308,6 +308,7 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
             for (int a = 0; a < 3; a++) {
                 G.grid_org[a] = sc->grid_org[a];
                 G.grid_inv[a] = sc->grid_inv[a];
+                G.grid_size[a] = sc->grid_size[a];
             }
             groups.push_back(G);
         }

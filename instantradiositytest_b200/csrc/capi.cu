@@ -255,20 +255,15 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
         ctx->in_use += added;
     }
     sc->march_host.assign(mbytes / 16, make_float4(0.f, 0.f, 0.f, 0.f));
-    irtd::MNode* mn = reinterpret_cast<irtd::MNode*>(sc->march_host.data());
-    irtd::MObj* mo = reinterpret_cast<irtd::MObj*>(mn + node_count);
+    irtd::MObj* mo = reinterpret_cast<irtd::MObj*>(sc->march_host.data());
     auto bits = [](uint32_t u) {
         float f;
         std::memcpy(&f, &u, 4);
         return f;
     };
     std::vector<uint32_t> leaf_of(object_count, 0);
-    for (uint32_t i = 0; i < node_count; i++) {
-        const irt_node& n = nodes[i];
-        mn[i].a = make_float4(n.lo[0], n.lo[1], n.lo[2], bits(n.info[3]));
-        mn[i].b = make_float4(n.hi[0], n.hi[1], n.hi[2], bits(n.info[2] == 1u ? n.info[0] : 0xffffffffu));
-        if (n.info[2] == 1u) leaf_of[n.info[0]] = i;
-    }
+    for (uint32_t i = 0; i < node_count; i++)
+        if (nodes[i].info[2] == 1u) leaf_of[nodes[i].info[0]] = i;
     for (uint32_t i = 0; i < object_count; i++) {
         const irt_object& o = objects[i];
         const irt_mesh& m = sc->host_meshes[o.info[0]];
@@ -276,13 +271,22 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
         mo[i].rx = make_float4(inv[0], inv[4], inv[8], inv[12]);
         mo[i].ry = make_float4(inv[1], inv[5], inv[9], inv[13]);
         mo[i].rz = make_float4(inv[2], inv[6], inv[10], inv[14]);
-        mo[i].meta = make_float4(bits(o.info[2]), bits(o.info[3]), bits(o.info[0]), bits(leaf_of[i]));
+        const uint32_t res = m.field[3];
+        uint32_t first_cell;  // hi[3]: first corner cell of the mesh
+        std::memcpy(&first_cell, &m.hi[3], 4);
+        float scale, voxel;
+        std::memcpy(&scale, &o.info[2], 4);
+        std::memcpy(&voxel, &o.info[3], 4);
+        mo[i].meta = make_float4(scale, voxel, (float)(res - 2u), bits(irtd::cell_bias(first_cell, res)));
         mo[i].lo = make_float4(m.lo[0], m.lo[1], m.lo[2], m.lo[3]);
-        mo[i].hi = make_float4(m.hi[0], m.hi[1], m.hi[2], m.hi[3]);
-        mo[i].field = make_uint4(m.field[0], m.field[1], m.field[2], m.field[3]);
+        mo[i].hi = make_float4(m.hi[0], m.hi[1], m.hi[2], bits(res - 1u));
         mo[i].grid = make_float4(m.grid[0], m.grid[1], m.grid[2], m.grid[3]);
         mo[i].glo = make_float4(m.geometry_lo[0], m.geometry_lo[1], m.geometry_lo[2], m.geometry_lo[3]);
         mo[i].ghi = make_float4(m.geometry_hi[0], m.geometry_hi[1], m.geometry_hi[2], m.geometry_hi[3]);
+        mo[i].field = make_float4((float)m.field[0], (float)m.field[1], (float)m.field[2], 0.f);
+        const irt_node& leaf = nodes[leaf_of[i]];
+        mo[i].leaf_lo = make_float4(leaf.lo[0], leaf.lo[1], leaf.lo[2], 0.f);
+        mo[i].leaf_hi = make_float4(leaf.hi[0], leaf.hi[1], leaf.hi[2], 0.f);
         mo[i].sphere = make_float4(m.enclosing_sphere[0], m.enclosing_sphere[1], m.enclosing_sphere[2],
                                    m.enclosing_sphere[3]);
     }
@@ -310,18 +314,6 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
             sc->bytes += added;
             ctx->in_use += added;
         }
-        const uint32_t R = kGridRes + 1;
-        const size_t corner_floats = (size_t)R * R * R * object_count;
-        if (object_count <= kMaxCornerObjects && sc->corner_cap < corner_floats) {
-            if (sc->corners) cudaFree(sc->corners);
-            sc->corners = nullptr;
-            uint64_t added = 0;
-            irt_status s1 = dev_alloc(ctx, &sc->corners, corner_floats * 4, added);
-            if (s1) return s1;
-            sc->corner_cap = corner_floats;
-            sc->bytes += added;
-            ctx->in_use += added;
-        }
         LeafCacheLaunch LC{};
         LC.march_scene = sc->march_scene;
         LC.n = object_count;
@@ -334,12 +326,10 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
             double ext = (double)nodes[0].hi[a] - (double)nodes[0].lo[a];
             double lo = (double)nodes[0].lo[a] - 1e-3 * ext - 1e-3;
             double hi = (double)nodes[0].hi[a] + 1e-3 * ext + 1e-3;
-            LC.grid_org_d[a] = lo;
-            LC.grid_size_d[a] = (hi - lo) / kGridRes;
-            sc->grid_org[a] = (float)lo;
+            sc->grid_org[a] = LC.grid_org[a] = (float)lo;
+            sc->grid_size[a] = LC.grid_size[a] = (float)((hi - lo) / kGridRes);
             sc->grid_inv[a] = (float)(kGridRes / (hi - lo));
         }
-        LC.corners = object_count <= kMaxCornerObjects ? sc->corners : nullptr;
         LC.cells = reinterpret_cast<uint32_t*>(sc->cells);
         CK(irt_launch_leaf_cache(LC, st), "leaf cache");
         sc->cached_nodes.assign(nodes, nodes + node_count);
@@ -428,7 +418,6 @@ void irt_scene_destroy(irt_scene* sc) {
     if (sc->lights_prep) cudaFree(sc->lights_prep);
     if (sc->march_scene) cudaFree(sc->march_scene);
     if (sc->cells) cudaFree(sc->cells);
-    if (sc->corners) cudaFree(sc->corners);
     for (int k = 0; k < 2; k++) {
         if (sc->pinned_free[k]) {
             cudaEventSynchronize(sc->pinned_free[k]);
@@ -683,6 +672,7 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
         for (int a = 0; a < 3; a++) {
             M.grid_org[a] = sc->grid_org[a];
             M.grid_inv[a] = sc->grid_inv[a];
+            M.grid_size[a] = sc->grid_size[a];
         }
         M.setup = session_ray_setup(s, sc, cur, prev);
         M.num_sms = s->num_sms;

@@ -61,11 +61,9 @@ struct irt_scene {
     uint32_t updates = 0;
     // leaf-order cache (rebuilt when the BVH changes)
     uint4* cells = nullptr;
-    float* corners = nullptr;
-    size_t corner_cap = 0;
     std::vector<irt_node> cached_nodes;
     std::vector<irt_object> cached_objects;
-    float grid_org[3] = {0, 0, 0}, grid_inv[3] = {0, 0, 0};
+    float grid_org[3] = {0, 0, 0}, grid_inv[3] = {0, 0, 0}, grid_size[3] = {0, 0, 0};
     uint32_t object_count = 0, light_count = 0;
     uint64_t bytes = 0;
 };
@@ -76,6 +74,7 @@ inline irtd::FieldFilter scene_field_filter(const irt_scene* sc) {
     irtd::FieldFilter f{};
     f.linear = sc->field_linear ? sc->atlas_linear : 0;
     for (int a = 0; a < 3; a++) f.dims[a] = (float)sc->atlas_dims[a];
+    f.bound_slack = sc->field_linear ? 1.f / 32.f : 0.f;
     return f;
 }
 

@@ -15,6 +15,9 @@ namespace irtd {
 struct FieldFilter {
     cudaTextureObject_t linear;  // the atlas: texel coordinates, linear filter, clamp
     float dims[3];               // atlas extent in texels
+    // Voxels by which a sampled distance may miss the trilinear value (three
+    // axes of 8-bit weights), for the leaf-order cache's bounds; 0 unfiltered.
+    float bound_slack;
 };
 }  // namespace irtd
 
@@ -105,12 +108,12 @@ struct MarchLaunch {
     const void* sdf_cells;  // corner cells of the field meshes (dev_sdf.cuh), or null
     irtd::FieldFilter field_filter;
     uint32_t* error;
-    const float4* march_scene;  // compact nodes + objects (irt_march_scene_bytes)
+    const float4* march_scene;  // object records (irt_march_scene_bytes)
     // Leaf-order cache: a kGridRes^3 grid over the root box; per cell the
-    // first kCellEntries objects by increasing distance from the cell to their
-    // BVH leaf box, with those distances and the next one as a sentinel.
+    // first kCellEntries objects by increasing lower bound of their distance
+    // from the cell's centre, those bounds and the next one as a sentinel.
     const uint4* cells;
-    float grid_org[3], grid_inv[3];
+    float grid_org[3], grid_inv[3], grid_size[3];
     RaySetup setup;
     int num_sms;
     int fast;  // 1: approximate division / square root build (march_fast.cu)
@@ -119,29 +122,32 @@ struct MarchLaunch {
 // the lighting passes); the ray set-up and the march (after them).
 cudaError_t irt_launch_ray_pools(const MarchLaunch& M, cudaStream_t st);
 cudaError_t irt_launch_march(const MarchLaunch& M, cudaStream_t st);
-// Bytes of the compact march scene of `object_count` objects: 2N-1 nodes of
-// 32 bytes, then N object records of 176 bytes (mesh folded in).
+// Bytes of the compact march scene of `object_count` objects: records of 208
+// bytes (dev_sdf.cuh: MObj).
 uint32_t irt_march_scene_bytes(uint32_t object_count);
 constexpr uint32_t kMaxMarchObjects = 1024;  // the march scene lives in shared memory
 constexpr uint32_t kGridRes = 32;
 constexpr uint32_t kCellEntries = 8;
-// One cell: 4 x uint4 = ids (8 x u16 in words 0-3), lower bounds (f32 words
-// 4-11), sentinel bound of the first object left out (word 12), pad.
-constexpr uint32_t kCellWords = 16;
+// One cell, 3 x uint4: [ids 0-3 (u16), bounds 1, 2], [ids 4-7, bounds 3, 4],
+// [bounds 5-7, bound of the first object left out].  The first vector is all
+// a query reads when its hint is the cell's first entry and the second is
+// farther than the best; bound 0 is never needed (entry 0's box is tested).
+constexpr uint32_t kCellWords = 12;
+constexpr __host__ __device__ uint32_t cell_id_word(uint32_t k) { return (k >> 1) + (k >= 4 ? 2u : 0u); }
+constexpr __host__ __device__ uint32_t cell_bound_word(uint32_t k) { return k + (k < 3 ? 1u : 3u); }
 // Leaf-order cache build (leafcache.cu) from the staged march scene.
 struct LeafCacheLaunch {
-    const float4* march_scene;  // nodes + object records on the device
+    const float4* march_scene;  // object records on the device
     uint32_t n;                 // objects
     cudaTextureObject_t atlas;
     int sdf_f16;
     const void* sdf_cells;  // corner cells of the field meshes (dev_sdf.cuh), or null
     irtd::FieldFilter field_filter;
-    double grid_org_d[3], grid_size_d[3];
-    float* corners;             // (kGridRes+1)^3 * n floats, or null: box bounds only
+    float grid_org[3], grid_size[3];  // as the march reads them
     uint32_t* cells;            // kGridRes^3 * kCellWords words
 };
 cudaError_t irt_launch_leaf_cache(const LeafCacheLaunch& L, cudaStream_t st);
-constexpr uint32_t kMaxCornerObjects = 256;  // corner bounds for scenes up to this many objects
+constexpr uint32_t kMaxBoundObjects = 256;  // distance bounds for scenes up to this many objects, else box bounds
 
 struct SvgfLaunch {
     const irt_frame* frame;
@@ -242,7 +248,7 @@ struct alignas(16) MarchGroup {
     const float4* march_scene;
     uint32_t scene_vec4;
     const uint4* cells;
-    float grid_org[3], grid_inv[3];
+    float grid_org[3], grid_inv[3], grid_size[3];
     uint32_t q_begin, q_end;    // the group's queues in the queue table
 };
 struct MarchBatch {

@@ -2,22 +2,28 @@
 //
 // The cache is a kGridRes^3 grid over the root box of the BVH.  Per cell it
 // keeps the kCellEntries objects with the smallest lower bound on their
-// distance over the cell, sorted, plus the next bound as a sentinel.  A
-// bound is the larger of
-//   * the box bound: distance from the cell (grown by a rounding margin) to
-//     the object's BVH leaf box, x 0.9998 — the walk's own pruning bound;
-//   * the corner bound: the smallest object distance at the cell's eight
-//     corners minus the cell's half diagonal and a margin, when all eight
-//     are positive.  Positive object distances are 1-Lipschitz in world
-//     space (signed box and sphere distances are; the field term is scaled by
-//     the reciprocal of its trilinear gradient bound, its Pythagorean
-//     extension keeps that, and the object scale and 0.9999 factor do not
-//     raise it), so no point of the cell lies closer.
-// The march visits a cell's objects in this order and stops at the first
-// bound above its best distance; every object it skips has a distance above
-// that best, so the minimum, the closest object and its voxel are those of
-// the reference walk.  Corner distances use the same device code as the
-// march (object_distance on the staged records and the SDF texture).
+// distance from the cell's CENTRE, sorted, plus the next bound as a sentinel.
+// Positive object distances are 1-Lipschitz in world space (signed box and
+// sphere distances are; the field term is scaled by the reciprocal of its
+// trilinear gradient bound, its Pythagorean extension keeps that, and the
+// object scale and 0.9999 factor do not raise it), so for a point p of the
+// cell, centre c, an object with bound B > |p - c| lies at least B - |p - c|
+// away.  A bound is the larger of
+//   * the box bound: distance from c to the object's BVH leaf box, x 0.9998;
+//   * the object's own distance at c, where positive;
+// less a margin for the f32 evaluation of either side, of f16 texels (rounded
+// down by up to 2^-10 of a distance) and of the filtered sampler's 8-bit
+// weights.  The march visits a cell's objects in this order and stops at the
+// first bound above its best distance + |p - c|; every object it skips has a
+// distance above that best, so the minimum, the closest object and its voxel
+// are those of the reference walk.  Distances use the march's own device code.
+//
+// Against bounds over the whole cell (smallest corner distance less the half
+// diagonal), which for a flat surface are up to three cell half-widths lower
+// still than the distance at the centre, the centre's bound less |p - c| gives
+// away one half-width on average: 2.41 -> 2.11 ms of march at 1920x1200, 24
+// objects.  One evaluation a cell and object, taken and sorted by a warp,
+// replaces a corner pass and an f64 insertion sort per thread.
 #include <cuda_runtime.h>
 
 #include "dev_sdf.cuh"
@@ -26,94 +32,70 @@
 namespace irtd {
 
 struct CacheGrid {
-    double org[3], size[3];
-    double margin, half_diag;
+    float org[3], size[3];
+    float margin, slope;  // bound = distance * slope - margin
 };
+constexpr uint32_t kBuildWarps = 8;
 
-__device__ __forceinline__ float object_distance_global(const DevScene& sc, V3 p, const MObj* objs, uint32_t o) {
-    const float4* r = reinterpret_cast<const float4*>(objs + o);
-    DMesh m;
-    m.lo = __ldg(r + 4);
-    m.hi = __ldg(r + 5);
-    m.field = __ldg(reinterpret_cast<const uint4*>(r + 6));
-    m.grid = __ldg(r + 7);
-    m.glo = __ldg(r + 8);
-    m.ghi = __ldg(r + 9);
-    m.sphere = __ldg(r + 10);
-    return object_distance_rows(sc, p, __ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3).x, m);
-}
-
-// Object distance at every grid corner: D[corner * n + object].
-__global__ void corner_distance_kernel(const DevScene sc, const MObj* objs, uint32_t n, const CacheGrid g,
-                                       float* D) {
-    const uint32_t R = kGridRes + 1;
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)R * R * R * n) return;
-    uint32_t o = (uint32_t)(i % n);
-    uint32_t c = (uint32_t)(i / n);
-    uint32_t x = c % R, y = (c / R) % R, z = c / (R * R);
-    V3 p = V3{(float)(g.org[0] + x * g.size[0]), (float)(g.org[1] + y * g.size[1]), (float)(g.org[2] + z * g.size[2])};
-    D[i] = object_distance_global(sc, p, objs, o);
-}
-
-__global__ void cell_build_kernel(const MNode* nodes, const MObj* objs, uint32_t n, const CacheGrid g,
-                                  const float* D, int use_corners, uint32_t* cells) {
-    const uint32_t G = kGridRes, R = kGridRes + 1;
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= G * G * G) return;
-    uint32_t ix = c % G, iy = (c / G) % G, iz = c / (G * G);
-    double clo[3] = {g.org[0] + ix * g.size[0] - g.margin, g.org[1] + iy * g.size[1] - g.margin,
-                     g.org[2] + iz * g.size[2] - g.margin};
-    double chi[3] = {g.org[0] + (ix + 1) * g.size[0] + g.margin, g.org[1] + (iy + 1) * g.size[1] + g.margin,
-                     g.org[2] + (iz + 1) * g.size[2] + g.margin};
-    // the K+1 smallest (bound, object) pairs, ascending
-    float best_lb[kCellEntries + 1];
-    uint32_t best_id[kCellEntries + 1];
+// One warp per cell: lanes take the objects in turn, then the warp extracts
+// the kCellEntries + 1 smallest (bound, object) pairs in ascending order.
+__global__ void __launch_bounds__(kBuildWarps * 32) cell_build_kernel(const DevScene sc, const MObj* __restrict__ objs,
+                                                                      uint32_t n, const CacheGrid g, int use_distance,
+                                                                      uint32_t* __restrict__ cells) {
+    extern __shared__ uint32_t keys_smem[];
+    const unsigned full = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x / 32u;
+    uint32_t* keys = keys_smem + warp * n;
+    const uint32_t c = blockIdx.x * kBuildWarps + warp;  // the grid covers kGridRes^3 cells exactly
+    const uint32_t ix = c % kGridRes, iy = (c / kGridRes) % kGridRes, iz = c / (kGridRes * kGridRes);
+    const V3 p = V3{g.org[0] + (ix + .5f) * g.size[0], g.org[1] + (iy + .5f) * g.size[1],
+                    g.org[2] + (iz + .5f) * g.size[2]};
+    for (uint32_t o = lane; o < n; o += 32) {
+        const MObj& obj = objs[o];
+        const V3 gap = fmax3(fmax3(xyz(obj.leaf_lo) - p, p - xyz(obj.leaf_hi)), V3{0.f, 0.f, 0.f});
+        float lb = length(gap) * .9998f;
+        if (use_distance) {
+            const float d = object_distance(sc, p, obj);
+            if (d > lb) lb = d;
+        }
+        lb = lb * g.slope - (g.margin + obj.meta.y * sc.filter.bound_slack);
+        // order-preserving bits: the smallest float has the smallest key
+        const uint32_t b = __float_as_uint(lb);
+        keys[o] = b & 0x80000000u ? ~b : b | 0x80000000u;
+    }
+    __syncwarp();
+    uint32_t ids[kCellEntries + 1], bounds[kCellEntries + 1];
+    uint32_t last_key = 0u, last_id = 0u;
+#pragma unroll
     for (uint32_t k = 0; k <= kCellEntries; k++) {
-        best_lb[k] = INFINITY;
-        best_id[k] = 0xffffu;
+        uint32_t key = 0xffffffffu, id = 0xffffu;
+        for (uint32_t o = lane; o < n; o += 32) {
+            const uint32_t q = keys[o];
+            const bool after = k == 0u || q > last_key || (q == last_key && o > last_id);
+            if (after && q < key) {
+                key = q;
+                id = o;
+            }
+        }
+        const uint32_t best = __reduce_min_sync(full, key);
+        id = __reduce_min_sync(full, key == best ? id : 0xffffu);
+        last_key = best;
+        last_id = id;
+        ids[k] = id;
+        const uint32_t bits = best & 0x80000000u ? best & 0x7fffffffu : ~best;
+        bounds[k] = id == 0xffffu ? 0x7f800000u : bits;  // nothing left: +infinity
     }
-    for (uint32_t o = 0; o < n; o++) {
-        const uint32_t leaf = __float_as_uint(objs[o].meta.w);
-        const float4 a = nodes[leaf].a, b = nodes[leaf].b;
-        const double blo[3] = {a.x, a.y, a.z}, bhi[3] = {b.x, b.y, b.z};
-        double s = 0.0;
-        for (int k = 0; k < 3; k++) {
-            double gap = fmax(0.0, fmax(blo[k] - chi[k], clo[k] - bhi[k]));
-            s += gap * gap;
-        }
-        double lb = sqrt(s) * 0.9998 * (1.0 - 1e-6);
-        if (use_corners) {
-            double mn = INFINITY;
-            for (uint32_t k = 0; k < 8; k++) {
-                uint32_t cx = ix + (k & 1), cy = iy + ((k >> 1) & 1), cz = iz + (k >> 2);
-                mn = fmin(mn, (double)D[(size_t)((cz * R + cy) * R + cx) * n + o]);
-            }
-            if (mn > 0.0) {
-                double cb = mn - g.half_diag - 1e-3 * g.half_diag - 1e-4 - 1e-4 * mn;
-                lb = fmax(lb, cb);
-            }
-        }
-        float lbf = __double2float_rd(lb);
-        if (lbf < best_lb[kCellEntries] || (lbf == best_lb[kCellEntries] && o < best_id[kCellEntries])) {
-            // insert, keeping (bound, id) ascending
-            int k = (int)kCellEntries;
-            while (k > 0 && (best_lb[k - 1] > lbf || (best_lb[k - 1] == lbf && best_id[k - 1] > o))) {
-                best_lb[k] = best_lb[k - 1];
-                best_id[k] = best_id[k - 1];
-                k--;
-            }
-            best_lb[k] = lbf;
-            best_id[k] = o;
-        }
+    uint32_t out[kCellWords];
+#pragma unroll
+    for (uint32_t k = 0; k < kCellEntries; k += 2) out[cell_id_word(k)] = ids[k] | (ids[k + 1] << 16);
+#pragma unroll
+    for (uint32_t k = 1; k <= kCellEntries; k++) out[cell_bound_word(k)] = bounds[k];
+    if (lane < kCellWords / 4) {
+        uint4 v = make_uint4(out[0], out[1], out[2], out[3]);
+        if (lane == 1) v = make_uint4(out[4], out[5], out[6], out[7]);
+        if (lane == 2) v = make_uint4(out[8], out[9], out[10], out[11]);
+        reinterpret_cast<uint4*>(cells)[c * (kCellWords / 4) + lane] = v;
     }
-    uint32_t* w = cells + (size_t)c * kCellWords;
-    uint32_t idw[4] = {0, 0, 0, 0};
-    for (uint32_t k = 0; k < kCellEntries; k++) idw[k >> 1] |= (best_id[k] & 0xffffu) << ((k & 1) * 16);
-    for (uint32_t k = 0; k < 4; k++) w[k] = idw[k];
-    for (uint32_t k = 0; k < kCellEntries; k++) w[4 + k] = __float_as_uint(best_lb[k]);
-    w[12] = __float_as_uint(best_lb[kCellEntries]);
-    w[13] = w[14] = w[15] = 0u;
 }
 
 }  // namespace irtd
@@ -121,34 +103,25 @@ __global__ void cell_build_kernel(const MNode* nodes, const MObj* objs, uint32_t
 cudaError_t irt_launch_leaf_cache(const LeafCacheLaunch& L, cudaStream_t st) {
     using namespace irtd;
     CacheGrid g;
-    double maxsize = 0;
+    double d2 = 0, far = 0;
     for (int a = 0; a < 3; a++) {
-        g.org[a] = L.grid_org_d[a];
-        g.size[a] = L.grid_size_d[a];
-        maxsize = fmax(maxsize, g.size[a]);
+        g.org[a] = L.grid_org[a];
+        g.size[a] = L.grid_size[a];
+        d2 += (double)g.size[a] * g.size[a];
+        far = fmax(far, fmax(fabs((double)g.org[a]), fabs((double)g.org[a] + g.size[a] * (double)kGridRes)));
     }
-    // A point is filed by f32 arithmetic; growing each cell by this margin
-    // keeps the point inside the cell box its bounds are computed for.
-    g.margin = 1e-4 + 1e-5 * maxsize * kGridRes;
-    double d2 = 0;
-    for (int a = 0; a < 3; a++) d2 += (g.size[a] + 2 * g.margin) * (g.size[a] + 2 * g.margin);
-    g.half_diag = 0.5 * sqrt(d2);
+    // The f32 error of a point's place in its cell and of the distances there.
+    g.margin = (float)(1e-4 + 1e-3 * 0.5 * sqrt(d2) + 1e-6 * far);
+    g.slope = L.sdf_f16 ? 1.f - 2e-3f : 1.f - 2e-4f;
     DevScene sc{};
     sc.atlas = L.atlas;
     sc.sdf_f16 = L.sdf_f16;
     sc.sdf_cells = L.sdf_cells;
     sc.filter = L.field_filter;
-    const MObj* objs = reinterpret_cast<const MObj*>(L.march_scene + 2 * (2 * L.n - 1));
-    const MNode* nodes = reinterpret_cast<const MNode*>(L.march_scene);
-    const int use_corners = L.corners != nullptr;
-    if (use_corners) {
-        const uint64_t R = kGridRes + 1;
-        uint64_t total = R * R * R * L.n;
-        corner_distance_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(sc, objs, L.n, g, L.corners);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
+    const MObj* objs = reinterpret_cast<const MObj*>(L.march_scene);
+    static_assert((kGridRes * kGridRes * kGridRes) % kBuildWarps == 0, "whole blocks of cells");
     const uint32_t cells = kGridRes * kGridRes * kGridRes;
-    cell_build_kernel<<<(cells + 127) / 128, 128, 0, st>>>(nodes, objs, L.n, g, L.corners, use_corners, L.cells);
+    cell_build_kernel<<<cells / kBuildWarps, kBuildWarps * 32, kBuildWarps * L.n * 4, st>>>(
+        sc, objs, L.n, g, L.n <= kMaxBoundObjects, L.cells);
     return cudaGetLastError();
 }

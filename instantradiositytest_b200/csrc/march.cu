@@ -11,11 +11,15 @@
 // restates them as a per-lane state machine; lanes that finish their rays
 // refill together from their warp's reserved slice of the queue.  The march
 // is bound by instruction issue under divergence (79 % issue active, DRAM
-// idle), so what counts is lanes per instruction.  Per 1920x1200 frame (24
+// idle) and the latency of the field's corner cells, so what counts is lanes
+// per instruction, instructions, and resident warps.  Per 1920x1200 frame (24
 // meshes, f32, set-up included): clearances and endpoints as phases of the
 // march 3.22 ms at 14 lanes an instruction; as kernels of their own, and the
 // march's stages rejoined by __syncwarp (lane_step), 2.42 ms at 19.4 lanes,
-// of which the set-up is 0.14 ms.
+// of which the set-up is 0.14 ms; leaf bounds taken at the query point
+// (leafcache.cu; 1.31 -> 1.13 evaluations a query, fewer entries tested)
+// 2.11; short divides, flushed denormals, 256-bit cell loads 2.05; the cell
+// found anew per candidate search instead of kept, 1.98; 36 warps 1.89.
 //
 // scene_distance (sdf.wgsl:42-60) returns the minimum object distance: the
 // walk skips a subtree only when its box bound exceeds the current best, and
@@ -24,9 +28,10 @@
 // distance is clamped to).  So visiting the same leaves in another order and
 // skipping those whose box bound exceeds the current best yields the same
 // best, the same closest object (ties aside) and the same voxel.  The march
-// visits leaves in the order of a per-frame leaf-order cache: for the grid
-// cell holding the query point, the leaves sorted by their box distance to
-// the cell, stopping at the first whose bound exceeds the best so far.
+// visits leaves in the order of a per-frame leaf-order cache (leafcache.cu):
+// for the grid cell holding the query point, the leaves sorted by a lower
+// bound of their distance from the cell's centre, stopping at the first whose
+// bound exceeds the best so far plus the point's distance from the centre.
 // Points outside the grid, or past the cached entries, test every leaf.
 // Per object the arithmetic is object_distance()'s, evaluated on records
 // staged in shared memory.
@@ -55,14 +60,15 @@ namespace fast {
 namespace exact {
 #endif
 
-// Resident warps: 64 registers a thread, no spills, 32 warps per SM.  In
-// CTAs of 128 threads (the batched march): 9 CTAs at 56 registers spill and
-// measured 3.82 ms, 7 CTAs 3.78 ms, 8 CTAs 3.56 ms per 1920x1200 frame.  The
-// single-view march runs them as 4 CTAs of 256 threads, each staging the
-// scene records once for 8 warps: 3.392 -> 3.371 ms against 8 CTAs of 128.
+// Resident warps, set-up and march at 1920x1200: the single-view march at 56
+// registers in CTAs of 192 threads, 6 per SM (36 warps, no spills), 1.89 ms;
+// 4 CTAs of 256 (64 registers, 32 warps) 1.98, 5 (48 registers, spills) 2.14,
+// 6 (40 registers) 2.47, 3 (24 warps) 2.39 before the query was slimmed.  The
+// batched march, whose lanes also keep their queue, spills at 56 registers: 8
+// CTAs of 128 (64 registers) 4.36 ms over 5.2 Mpixel of views, 9 CTAs 4.75.
 constexpr int kMarchBlocksPerSm = 8;
-constexpr int kMarchThreads = 256;
-constexpr int kMarchCtasPerSm = 4;
+constexpr int kMarchThreads = 192;
+constexpr int kMarchCtasPerSm = 6;
 // Queue entries a warp reserves per atomic (one per lane): the queue counter
 // then sees one atomic per ~30 warp iterations instead of about one per
 // iteration (1920x1200 room: 3.51 -> 3.43 ms with the L2 prefetch of the
@@ -70,111 +76,104 @@ constexpr int kMarchCtasPerSm = 4;
 constexpr uint32_t kRayChunk = 32;
 constexpr uint32_t kNone = 0xffffffffu;
 
-__device__ __forceinline__ float object_distance_rec(const DevScene& sc, V3 p, const MObj& o) {
-    DMesh m;
-    m.lo = o.lo;
-    m.hi = o.hi;
-    m.field = o.field;
-    m.grid = o.grid;
-    m.glo = o.glo;
-    m.ghi = o.ghi;
-    m.sphere = o.sphere;
-    return object_distance_rows(sc, p, o.rx, o.ry, o.rz, o.meta.x, m);
-}
-
 struct Grid {
     const uint4* cells;
     float ox, oy, oz, ix, iy, iz;
+    float sx, sy, sz;  // cell size
 };
 
-// The march as one flattened loop: every iteration each lane evaluates at
-// most one object, the next candidate of its current distance query — the
-// hint object first (the previous closest, as scene_distance seeds it), then
-// the leaf-order cache entries of the query point's cell that survive the
-// walk's pruning tests (stopping at the first entry whose bound exceeds the
-// best), then every leaf when the cached entries may not hold the minimum
-// or the point is outside the grid.  A lane whose query has no candidate
-// left completes it (the step of sdf.wgsl:61-81 it feeds), starts its ray's
-// next query or takes a new ray, and finds that query's first candidate in
-// the same iteration.  So the object evaluations of lanes at different
-// stages of their queries (a hint, a second leaf, the first leaf of a new
-// ray) issue together instead of in separate divergent sections; per query
-// the candidates and their order are the same as a walk of one query at a
-// time, so the results are too.
+// A distance query.  Its candidates are the hint object first (the previous
+// closest, as scene_distance seeds it), then the leaf-order cache entries of
+// the query point's cell that survive the walk's pruning tests (stopping at
+// the first entry whose bound exceeds the best), then every leaf when the
+// cached entries may not hold the minimum or the point is outside the grid.
+// The march runs the queries of a warp's lanes as one flattened loop, one
+// object per lane and iteration, so the evaluations of lanes at different
+// stages (a hint, a second leaf) issue together; per query the candidates and
+// their order are the same as a walk of one query at a time, so the results
+// are too.
 struct Query {
-    V3 p;
     float best;
     uint32_t closest, hint;
-    uint32_t oid;         // the object to evaluate next, or kNone
-    int32_t cur;          // the candidate after it: 0..7 cache entries, 8 after them, >= kAll all leaves
-    const uint32_t* cw;   // the point's cache cell, or null outside the grid
+    uint32_t oid;  // the object to evaluate next, or kNone
+    uint32_t cur;  // the candidate after it: 0..7 cache entries, 8 after them, >= kAll all leaves
 };
-constexpr int32_t kAfterEntries = (int32_t)kCellEntries;
-constexpr int32_t kAll = 16;
-constexpr int32_t kQueryDone = 0x7fffffff;
+constexpr uint32_t kAll = 16;
 
-__device__ __forceinline__ void query_begin(Query& qy, const Grid& g, V3 p, uint32_t hint, uint32_t n) {
-    qy.p = p;
+__device__ __forceinline__ void query_begin(Query& qy, uint32_t hint, uint32_t n) {
     qy.best = 1e20f;
     qy.closest = hint;
     qy.hint = hint;
-    const float fx = (p.x - g.ox) * g.ix, fy = (p.y - g.oy) * g.iy, fz = (p.z - g.oz) * g.iz;
-    const float G = (float)kGridRes;
-    const bool inside = fx >= 0.f && fy >= 0.f && fz >= 0.f && fx < G && fy < G && fz < G;
-    qy.cw = nullptr;
-    if (inside) {
-        const uint32_t cell = ((uint32_t)fz * kGridRes + (uint32_t)fy) * kGridRes + (uint32_t)fx;
-        qy.cw = reinterpret_cast<const uint32_t*>(g.cells + (size_t)cell * (kCellWords / 4));
-    }
-    qy.cur = inside ? 0 : kAll;
-    qy.oid = hint < n ? hint : kNone;  // the hint first, unconditionally
+    qy.cur = 0u;
+    qy.oid = hint < n ? hint : kNone;
 }
 
-// The walk's pruning test of leaf `oid`'s box against the best so far.
-__device__ __forceinline__ bool leaf_may_hold_best(const MNode* nodes, const MObj* objs, V3 p, uint32_t oid,
-                                                   float best) {
-    const uint32_t leaf = __float_as_uint(objs[oid].meta.w);
-    const float4 a = nodes[leaf].a, b = nodes[leaf].b;
-    V3 delta = vmax(vmax(V3{a.x, a.y, a.z} - p, p - V3{b.x, b.y, b.z}), V3{0.f, 0.f, 0.f});
+// The cache cell of a point (or kNone outside the grid) and the point's
+// distance from the cell's centre.
+__device__ __forceinline__ uint32_t cell_of(const Grid& g, V3 p, float& off_centre) {
+    static_assert((kGridRes & (kGridRes - 1)) == 0, "the inside test takes the or of the three coordinates");
+    const V3 f = {(p.x - g.ox) * g.ix, (p.y - g.oy) * g.iy, (p.z - g.oz) * g.iz};
+    const V3 m = {__fadd_rd(f.x, kFloorMagic), __fadd_rd(f.y, kFloorMagic), __fadd_rd(f.z, kFloorMagic)};
+    const uint32_t x = __float_as_uint(m.x) - kFloorBits, y = __float_as_uint(m.y) - kFloorBits,
+                   z = __float_as_uint(m.z) - kFloorBits;
+    const float half = kFloorMagic - .5f;  // m - half = the cell's centre; exact
+    const V3 r = {(f.x - (m.x - half)) * g.sx, (f.y - (m.y - half)) * g.sy, (f.z - (m.z - half)) * g.sz};
+    off_centre = sqrtf(dot(r, r));
+    return (x | y | z) < kGridRes ? (z * kGridRes + y) * kGridRes + x : kNone;
+}
+
+// The walk's pruning test of an object's leaf box against the best so far.
+__device__ __forceinline__ bool leaf_may_hold_best(const MObj& o, V3 p, float bound) {
+    V3 delta = fmax3(fmax3(xyz(o.leaf_lo) - p, p - xyz(o.leaf_hi)), V3{0.f, 0.f, 0.f});
     V3 lb = delta * .9998f;
-    float bb = wmax(best, 0.f);
-    return !(dot(lb, lb) > bb * bb);
+    return !(dot(lb, lb) > bound * bound);
 }
 
-// Next object to evaluate for the query, or kNone when the query is complete.
-__device__ __forceinline__ uint32_t query_next(Query& qy, const MNode* nodes, const MObj* objs, uint32_t n,
+// Next object to evaluate for the query at p, or kNone when it is complete.
+// The cell is found anew on each call (1.13 a query): kept in the query, it
+// and the point would live through the evaluation.
+__device__ __forceinline__ uint32_t query_next(Query& qy, V3 p, const Grid& g, const MObj* objs, uint32_t n,
                                                uint32_t* err) {
-    for (;;) {
-        const int32_t c = qy.cur;
-        if (c < kAfterEntries) {
-            const uint32_t oid = (__ldg(qy.cw + (c >> 1)) >> ((c & 1) * 16)) & 0xffffu;
-            if (__uint_as_float(__ldg(qy.cw + 4 + c)) > wmax(qy.best, 0.f) || oid == 0xffffu) {
-                qy.cur = kQueryDone;
-                return kNone;
-            }
-            qy.cur = c + 1;
-            if (oid != qy.hint && index_ok(err, oid, n) && leaf_may_hold_best(nodes, objs, qy.p, oid, qy.best))
-                return oid;
-            continue;
+    float off_centre;
+    const uint32_t cell = cell_of(g, p, off_centre);
+    const float bound = fmaxf(qy.best, 0.f), reach = bound + off_centre;
+    const uint32_t* cw = reinterpret_cast<const uint32_t*>(g.cells) + (size_t)cell * kCellWords;
+    uint32_t c = qy.cur;
+    if (cell == kNone) {
+        if (c == 0u) c = kAll;
+    } else if (c == 0u) {  // usually the hint is the cell's first entry and the second one is farther
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(cw));
+        if ((w.x & 0xffffu) == qy.hint) {
+            if (__uint_as_float(w.z) > reach) return kNone;
+            c = 1u;
         }
-        if (c == kAfterEntries) {  // every cached entry fits: the ones left out may too
-            qy.cur = __uint_as_float(__ldg(qy.cw + 12)) <= wmax(qy.best, 0.f) ? kAll : kQueryDone;
+    }
+    for (;; c++) {
+        uint32_t oid;
+        if (c < kCellEntries) {
+            if (c > 0u && __uint_as_float(__ldg(cw + cell_bound_word(c))) > reach) return kNone;
+            oid = (__ldg(cw + cell_id_word(c)) >> ((c & 1u) * 16u)) & 0xffffu;
+            if (oid == 0xffffu) return kNone;
+            if (!index_ok(err, oid, n)) continue;
+        } else if (c < kAll) {  // every cached entry fits: the ones left out may too
+            if (__uint_as_float(__ldg(cw + cell_bound_word(kCellEntries))) > reach) return kNone;
+            c = kAll - 1u;
             continue;
+        } else {
+            oid = c - kAll;
+            if (oid >= n) return kNone;
         }
-        if (c < kAll + (int32_t)n) {
-            const uint32_t oid = (uint32_t)(c - kAll);
-            qy.cur = c + 1;
-            if (oid != qy.hint && leaf_may_hold_best(nodes, objs, qy.p, oid, qy.best)) return oid;
-            continue;
+        if (oid != qy.hint && leaf_may_hold_best(objs[oid], p, bound)) {
+            qy.cur = c + 1u;
+            return oid;
         }
-        return kNone;
     }
 }
 
 // Object `oid`'s distance folded into the query (the hint sets the best
 // unconditionally, as scene_distance seeds it).
-__device__ __forceinline__ void query_eval(Query& qy, const DevScene& sc, const MObj* objs, uint32_t oid) {
-    const float d = object_distance_rec(sc, qy.p, objs[oid]);
+__device__ __forceinline__ void query_eval(Query& qy, V3 p, const DevScene& sc, const MObj* objs, uint32_t oid) {
+    const float d = object_distance(sc, p, objs[oid]);
     if (oid == qy.hint || d < qy.best) {
         qy.best = d;
         qy.closest = oid;
@@ -183,30 +182,27 @@ __device__ __forceinline__ void query_eval(Query& qy, const DevScene& sc, const 
 
 // One distance query from p without a hint, walked to its end: the nearest
 // object, or kNone.
-__device__ __forceinline__ uint32_t query_closest(const DevScene& sc, const Grid& g, const MNode* nodes,
-                                                  const MObj* objs, uint32_t n, V3 p) {
+__device__ __forceinline__ uint32_t query_closest(const DevScene& sc, const Grid& g, const MObj* objs, uint32_t n,
+                                                  V3 p) {
     Query qy;
-    query_begin(qy, g, p, kNone, n);
+    query_begin(qy, kNone, n);
     for (;;) {
-        const uint32_t oid = query_next(qy, nodes, objs, n, sc.error);
+        const uint32_t oid = query_next(qy, p, g, objs, n, sc.error);
         if (oid == kNone) break;
-        query_eval(qy, sc, objs, oid);
+        query_eval(qy, p, sc, objs, oid);
     }
     return qy.closest;
 }
 
 // The scene as a kernel's CTA reads it.
 struct SceneRefs {
-    const MNode* nodes;
     const MObj* objs;
     uint32_t n_obj;
     float eps;
     uint32_t max_steps;
 };
 __device__ __forceinline__ SceneRefs scene_refs(const irt_frame& f, const float4* smem) {
-    const uint32_t n = f.counts[3];
-    return SceneRefs{reinterpret_cast<const MNode*>(smem), reinterpret_cast<const MObj*>(smem + 2 * (2 * n - 1)), n,
-                     f.sdf[1], to_u32(f.sdf[0])};
+    return SceneRefs{reinterpret_cast<const MObj*>(smem), f.counts[3], f.sdf[1], to_u32(f.sdf[0])};
 }
 
 // A point moved off the surface along its normal (sdf.wgsl:63, :66).
@@ -218,7 +214,7 @@ __device__ __forceinline__ V3 cleared(V3 p, V3 n, uint32_t closest, const SceneR
 // March endpoint of a VPL: cleared, when it has a normal.
 __device__ __forceinline__ V3 vpl_endpoint(const DevScene& sc, const Grid& g, const SceneRefs& R, V3 pos, V3 nrm) {
     if (!(dot(nrm, nrm) > .5f)) return pos;
-    return cleared(pos, nrm, query_closest(sc, g, R.nodes, R.objs, R.n_obj, pos), R);
+    return cleared(pos, nrm, query_closest(sc, g, R.objs, R.n_obj, pos), R);
 }
 
 __device__ __forceinline__ const irt_vpl* pool_vpl(const RaySetup& s, uint32_t v) {
@@ -268,7 +264,7 @@ __device__ __forceinline__ void ray_setup_tile(const RaySetup& s, const DevScene
         vpl = __ldg(s.prep_vpl + i);
         if (light != kNoRay || vpl != kNoRay) {
             const V3 p = xyz(__ldg(s.guide + i));
-            hint = query_closest(sc, g, R.nodes, R.objs, R.n_obj, p);
+            hint = query_closest(sc, g, R.objs, R.n_obj, p);
             d.origin = cleared(p, xyz(prep), hint, R);
             v.origin = d.origin;
         }
@@ -378,12 +374,11 @@ __device__ __forceinline__ void lane_reset(Lane& L) {
     L.m.result = 1.f;
     L.m.previous = 1e20f;
     L.m.step = 0;
-    L.qy.cur = kQueryDone;
+    L.qy.oid = kNone;
     L.active = false;
 }
 // The ray of record `at`, as ray_setup_tile left it, and its first query.
-__device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t at, const Grid& grid,
-                                          const SceneRefs& R) {
+__device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t at, const SceneRefs& R) {
     const float4* r = reinterpret_cast<const float4*>(s.rays + at);
     const float4 a = __ldg(r), b = __ldg(r + 1);
     const uint32_t hint = __ldg(s.hints + at);
@@ -397,7 +392,7 @@ __device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t a
     L.m.closest = hint;
     L.slot = __float_as_uint(a.w);
     L.active = true;
-    query_begin(L.qy, grid, march_point(L.m), hint, R.n_obj);
+    query_begin(L.qy, hint, R.n_obj);
 }
 // One iteration of a warp's lanes, stage by stage: every active lane
 // evaluates its query's object; finds the next one; and where the query has
@@ -408,9 +403,9 @@ __device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t a
 // an instruction, 760 against 531 million warp instructions at 960x600).
 __device__ __forceinline__ void lane_step(Lane& L, const DevScene& sc, const Grid& grid, const SceneRefs& R, float k,
                                           float* vis, uint32_t cap) {
-    if (L.active && L.qy.oid != kNone) query_eval(L.qy, sc, R.objs, L.qy.oid);
+    if (L.active && L.qy.oid != kNone) query_eval(L.qy, march_point(L.m), sc, R.objs, L.qy.oid);
     __syncwarp();
-    if (L.active) L.qy.oid = query_next(L.qy, R.nodes, R.objs, R.n_obj, sc.error);
+    if (L.active) L.qy.oid = query_next(L.qy, march_point(L.m), grid, R.objs, R.n_obj, sc.error);
     __syncwarp();
     if (L.active && L.qy.oid == kNone) {
         L.m.closest = L.qy.closest;
@@ -419,7 +414,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const DevScene& sc, const Gri
             if (index_ok(sc.error, L.slot, cap)) vis[L.slot] = out;
             L.active = false;
         } else {
-            query_begin(L.qy, grid, march_point(L.m), L.m.closest, R.n_obj);
+            query_begin(L.qy, L.m.closest, R.n_obj);
         }
     }
     __syncwarp();
@@ -485,7 +480,7 @@ __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) march_kernel(c
             const uint32_t idx = slice_take(slice, need, &setup.counters[1], n_rays, keep, lane, setup.rays, front, cap);
             exhausted = slice.drained && slice.next >= slice.end;
             if (!L.active && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap))
-                lane_take(L, setup, ray_slot(idx, front, cap), grid, R);
+                lane_take(L, setup, ray_slot(idx, front, cap), R);
         }
         lane_step(L, sc, grid, R, f.sdf[2], setup.vis, cap);
     }
@@ -522,7 +517,8 @@ __device__ __forceinline__ DevScene group_scene(const MarchGroup& G) {
     return sc;
 }
 __device__ __forceinline__ Grid group_grid(const MarchGroup& G) {
-    return Grid{G.cells, G.grid_org[0], G.grid_org[1], G.grid_org[2], G.grid_inv[0], G.grid_inv[1], G.grid_inv[2]};
+    return Grid{G.cells,        G.grid_org[0],  G.grid_org[1],  G.grid_org[2],  G.grid_inv[0],
+                G.grid_inv[1], G.grid_inv[2], G.grid_size[0], G.grid_size[1], G.grid_size[2]};
 }
 
 __global__ void __launch_bounds__(128) ray_pools_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
@@ -596,7 +592,7 @@ __global__ void __launch_bounds__(128, kMarchBlocksPerSm) march_batched_kernel(c
                 const uint32_t idx = slice_take(slice, need, &Q.setup.counters[1], n_rays, keep, lane, Q.setup.rays,
                                                 front, cap);
                 if (!L.active && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap)) {
-                    lane_take(L, Q.setup, ray_slot(idx, front, cap), grid, R);
+                    lane_take(L, Q.setup, ray_slot(idx, front, cap), R);
                     lq = q;
                 }
                 if (slice.drained && slice.next >= slice.end) {  // this queue is used up: the next view's
@@ -679,8 +675,8 @@ irtd::DevScene launch_scene(const MarchLaunch& M) {
     return sc;
 }
 IRT_MARCH_NS::Grid launch_grid(const MarchLaunch& M) {
-    return IRT_MARCH_NS::Grid{M.cells,        M.grid_org[0], M.grid_org[1], M.grid_org[2],
-                              M.grid_inv[0], M.grid_inv[1], M.grid_inv[2]};
+    return IRT_MARCH_NS::Grid{M.cells,        M.grid_org[0],  M.grid_org[1],  M.grid_org[2],  M.grid_inv[0],
+                              M.grid_inv[1], M.grid_inv[2], M.grid_size[0], M.grid_size[1], M.grid_size[2]};
 }
 
 }  // namespace
@@ -765,6 +761,6 @@ cudaError_t irt_launch_march_batched(const MarchBatch& M, cudaStream_t st) {
 }
 
 uint32_t irt_march_scene_bytes(uint32_t object_count) {
-    return (2 * object_count - 1) * (uint32_t)sizeof(irtd::MNode) + object_count * (uint32_t)sizeof(irtd::MObj);
+    return object_count * (uint32_t)sizeof(irtd::MObj);
 }
 #endif
