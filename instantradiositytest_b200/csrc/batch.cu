@@ -247,7 +247,6 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
                 A.in = in;
                 A.out = out;
                 A.out2 = out2;
-                A.step = 1 << i;
                 in = out;
             }
             irt_svgf_view_fill(A, hs[2 + i].data() + sv * v);
@@ -407,7 +406,7 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
     mark(1);
     for (size_t w = 0; w < waves; w++) {
         CK(irt_launch_svgf_batched(batch_launch(b, w, t.sviews[6], sv, -1),
-                                   b->desc.gbuffer_format == IRT_GBUFFER_F32 ? 3 : 6, st),
+                                   6, st),
            "batch guides");
         CK(irt_launch_svgf_batched(batch_launch(b, w, t.sviews[7], sv, -1), 4, st), "batch previous guides");
         mark(2);
@@ -439,8 +438,11 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
         mark(9);
         const uint32_t iters = b->desc.settings.svgf_iterations;
         for (uint32_t i = 0; i < iters && i < 4; i++)
-            CK(irt_launch_svgf_batched(batch_launch(b, w, t.sviews[2 + i], sv, shape_of[kTAtrous]), 2, st),
-               "batch atrous");
+        {
+            BatchLaunch A = batch_launch(b, w, t.sviews[2 + i], sv, shape_of[kTAtrous]);
+            A.step = 1 << i;
+            CK(irt_launch_svgf_batched(A, 2, st), "batch atrous");
+        }
         mark(10);
         CK(irt_launch_svgf_batched(batch_launch(b, w, t.history, sv, -1), 5, st), "batch history");
     }

@@ -609,8 +609,8 @@ static cudaError_t compute_guides(irt_session* s, const irt_frame* f, const irt_
     G.out = s->guide[0];
     G.out2 = s->feat;
     G.radiance_f16 = s->desc.radiance_format == IRT_RADIANCE_F16;
-    // positions, and for decoded G-buffer formats the edge-stopping features
-    cudaError_t e = irt_launch_svgf(G, s->desc.gbuffer_format == IRT_GBUFFER_F32 ? 3 : 6, st);
+    // positions and edge-stopping features
+    cudaError_t e = irt_launch_svgf(G, 6, st);
     if (e != cudaSuccess) return e;
     G.out = s->guide[1];
     e = irt_launch_svgf(G, 4, st);

@@ -215,12 +215,13 @@ struct BatchLaunch {
     int gbuffer_format;
     int radiance_f16, moments_f16;
     int keep;
+    int step;  // a-trous: 1 << iteration
 };
 size_t irt_lighting_args_size(int gbuffer_format);
 void irt_lighting_args_fill(const LightingLaunch& L, void* out);
 cudaError_t irt_launch_lighting_batched(const BatchLaunch& B, int stage, cudaStream_t st);
-// SVGF stages of a batch: 0 temporal, 1 variance, 2 a-trous (records carry
-// the step), 3 guides of this frame, 4 guides of the previous frame, 5 depth
+// SVGF stages of a batch: 0 temporal, 1 variance, 2 a-trous (BatchLaunch::
+// step), 3 guides of this frame, 4 guides of the previous frame, 5 depth
 // and normal history copy, 6 guides and features of this frame.
 size_t irt_svgf_view_size(int gbuffer_format);
 void irt_svgf_view_fill(const SvgfLaunch& L, void* out);

@@ -292,7 +292,6 @@ static void fill_view(const SvgfLaunch& L, void* out) {
     w.out = L.out;
     w.out2 = L.out2;
     w.moments_out = L.moments_out;
-    w.step = L.step;
     *static_cast<SView<G>*>(out) = w;
 }
 

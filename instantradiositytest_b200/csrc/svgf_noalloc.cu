@@ -112,12 +112,11 @@ extern "C" irt_status irt_svgf_spatial_noalloc(const irt_frame* frame, const irt
     L.gbuffer = *gbuffer;
     L.radiance_f16 = radiance_format == IRT_RADIANCE_F16;
     L.moments_f16 = moments_format == IRT_MOMENTS_F16;
-    // The frame's per-pixel positions (and, for the F16 and packed G-buffers,
-    // decoded edge-stopping features), written by the same kernels a session
+    // The frame's per-pixel positions and edge-stopping features, written by the same kernels a session
     // runs before its SVGF passes, so the results equal a session's.
     L.out = guide;
     L.out2 = feat;
-    cudaError_t e = irt_launch_svgf(L, gbuffer->format == IRT_GBUFFER_F32 ? 3 : 6, st);
+    cudaError_t e = irt_launch_svgf(L, 6, st);
     L.guide = guide;
     L.feat = feat;
     // svgf_variance (svgf.wgsl:77-89): temporal radiance + moments -> ping.

@@ -62,78 +62,170 @@ __global__ void __launch_bounds__(256) svgf_variance_kernel(const __grid_constan
                            blockIdx.y * blockDim.y + threadIdx.y);
 }
 
-__device__ __forceinline__ float wavelet_kernel(int32_t x) {
-    if (x == 0) return 1.f;
-    if (x == 1 || x == -1) return 2.f / 3.f;
-    return 1.f / 6.f;
+// A-trous: 25 taps a pixel, bound by L1 bandwidth (64 bytes a tap with f32
+// radiance) and load latency.  Per 1920x1200 pass, f32 / mixed storage, 256 / 246 us
+// before: a tap reads the guide and the feature record (one 128-bit and one
+// 256-bit load, also for f32 planes, whose five loads a tap cost 197 us with
+// all of the following), the wavelet step is a template constant so that the
+// taps of a row are immediate offsets, interior pixels test no bounds, the
+// three exponentials of a tap are one exp2 of the summed exponents with the
+// two divisors inverted once a pixel, no branch stands between the loads of
+// one tap and the next, and the 25 taps are unrolled (179 / 166 us with the
+// rows rolled): 173 / 156 us.  Two pixels a step apart per thread (30 taps
+// read instead of 50) 182 / 180; blocks of 32x4 176 us for step 1, 194-215 for
+// the others.
+//
+// What an a-trous tap reads of a pixel besides its radiance: position (w < 0:
+// background), normal and roughness, colour and metal.
+struct TapGeometry {
+    float4 position, normal, color;
+};
+// The planes of a row of pixels, from which a tap at a constant distance is
+// an immediate offset.
+template <class G>
+struct TapRow {
+    const float4* guide;
+    const float4* feat;
+    __device__ __forceinline__ TapRow(const SvgfCtx<G>& c, ptrdiff_t i) : guide(c.guide + i), feat(c.feat + 2 * i) {}
+    __device__ __forceinline__ TapGeometry at(int32_t dx) const {
+        TapGeometry t;
+        t.position = __ldg(guide + dx);
+        asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(t.normal.x), "=f"(t.normal.y), "=f"(t.normal.z), "=f"(t.normal.w), "=f"(t.color.x),
+              "=f"(t.color.y), "=f"(t.color.z), "=f"(t.color.w)
+            : "l"(feat + 2 * dx));
+        return t;
+    }
+};
+
+constexpr __device__ __host__ float wavelet_kernel(int32_t x) {
+    return x == 0 ? 1.f : (x == 1 || x == -1) ? 2.f / 3.f : 1.f / 6.f;
 }
 
-// svgf.wgsl:91-110; `out2` (optional) receives a second copy of the result.
-template <class G, class R>
-__device__ __forceinline__ void atrous_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* input,
-                                            typename R::T* out, typename R::T* out2, int32_t step, int32_t x,
-                                            int32_t y) {
-    Sv<G> sv(f, c);
-    if (x >= sv.W || y >= sv.H) return;
-    size_t i = sv.idx(x, y);
-    float4 c4 = R::load(input, i);
-    if (c.g.d(i) >= 1.f) {
-        R::store(out, i, c4);
-        if (out2) R::store(out2, i, c4);
-        return;
-    }
-    float variance = 0.f, guide_weight = 0.f;
-    Guide a = sv.guide(x, y);
-#pragma unroll
-    for (int32_t yy = -1; yy <= 1; yy++)
-#pragma unroll
-        for (int32_t xx = -1; xx <= 1; xx++) {
-            int32_t qx = min(max(x + xx, 0), sv.W - 1);
-            int32_t qy = min(max(y + yy, 0), sv.H - 1);
-            float w = (xx == 0 ? 2.f : 1.f) * (yy == 0 ? 2.f : 1.f);
-            float s = R::load(input, sv.idx(qx, qy)).w;
-            variance += s * s * w;
-            guide_weight += w;
-        }
-    float phi = 4.f * sqrtf(variance / wmax(guide_weight, .00001f)) + .0001f;
-    V3 sum = V3{0.f, 0.f, 0.f};
-    float total = 0.f, v = 0.f;
-    float lc = luminance(V3{c4.x, c4.y, c4.z});
-    auto tap = [&](int32_t xx, int32_t yy) {
-        int32_t qx = x + xx * step, qy = y + yy * step;
-        float geom = sv.geometry_weight(a, qx, qy, (float)step);
-        if (geom <= 0.f) return;
-        float4 smp = R::load(input, sv.idx(qx, qy));
-        float w = wavelet_kernel(xx) * wavelet_kernel(yy) * geom *
-                  expf(-fabsf(luminance(V3{smp.x, smp.y, smp.z}) - lc) / phi);
-        sum = sum + V3{smp.x, smp.y, smp.z} * w;
+// One pixel of svgf_atrous with its sums.
+struct Atrous {
+    V3 position, normal, color;
+    float rough, metal, lum;
+    float kz, kl;  // log2(e) over the plane-distance tolerance and over phi
+    V3 sum;
+    float total, v;
+    // svgf.wgsl:32-44, :99-105: the tap's weight, the exponentials of the
+    // plane distance, colour, parameter and luminance terms as one exp2 of
+    // their sum with the divisors' reciprocals taken once a pixel.
+    // Without a branch before the sums, so that the loads of later taps issue
+    // ahead of this one's arithmetic.
+    __device__ __forceinline__ void tap(const TapGeometry& t, float4 smp, float kernel) {
+        const float kc = 8.f * 1.44269504f;
+        const float wn = pow64(wmax(dot(normal, xyz(t.normal)), 0.f));
+        const V3 dc = color - xyz(t.color);
+        const float d0 = rough - t.normal.w, d1 = metal - t.color.w;
+        const float geom = fabsf(dot(xyz(t.position) - position, normal)) * kz +
+                           (length(dc) + sqrtf(d0 * d0 + d1 * d1)) * kc;
+        const float w = wn * kernel * exp2f(-(geom + fabsf(luminance(xyz(smp)) - lum) * kl));
+        // background (depth >= 1), or a geometry weight of 0
+        if (t.position.w < 0.f || !(wn > 0.f) || geom > 126.f) return;
+        sum = sum + xyz(smp) * w;
         v += smp.w * smp.w * w * w;
         total += w;
-    };
-    // Taps in row order.  With feature records (three 128-bit loads a tap)
-    // a row's five taps are unrolled so their loads issue together (a-trous
-    // 1.12 -> 1.03 ms at 1920x1200); on f32 planes (six loads a tap) the
-    // unrolled row needs more registers than it saves (1.08 -> 1.23 ms).
-    if constexpr (Sv<G>::kFeatures) {
-        for (int32_t yy = -2; yy <= 2; yy++)
-#pragma unroll
-            for (int32_t xx = -2; xx <= 2; xx++) tap(xx, yy);
-    } else {
-        for (int32_t yy = -2; yy <= 2; yy++)
-            for (int32_t xx = -2; xx <= 2; xx++) tap(xx, yy);
     }
-    float dn = wmax(total, .00001f);
-    float4 o = make_float4(sum.x / dn, sum.y / dn, sum.z / dn, wmin(sqrtf(v) / dn, 65000.f));
+};
+
+// The pixel's own terms; false: background, whose radiance passes through.
+template <class G, class R>
+__device__ __forceinline__ bool atrous_begin(Atrous& a, const SvgfCtx<G>& c, const typename R::T* input,
+                                             typename R::T* out, typename R::T* out2, int32_t W, int32_t H,
+                                             int32_t x, int32_t y, float step) {
+    const ptrdiff_t i = (ptrdiff_t)y * W + x;
+    const float4 c4 = R::load(input, i);
+    const TapGeometry own = TapRow<G>(c, i).at(0);
+    if (own.position.w < 0.f) {  // depth >= 1
+        R::store(out, i, c4);
+        if (out2) R::store(out2, i, c4);
+        return false;
+    }
+    float variance = 0.f;
+#pragma unroll
+    for (int32_t yy = -1; yy <= 1; yy++) {
+        const int32_t qy = min(max(y + yy, 0), H - 1);
+#pragma unroll
+        for (int32_t xx = -1; xx <= 1; xx++) {
+            const int32_t qx = min(max(x + xx, 0), W - 1);
+            const float s = R::load(input, (size_t)qy * W + qx).w;
+            variance += s * s * ((xx == 0 ? 2.f : 1.f) * (yy == 0 ? 2.f : 1.f));
+        }
+    }
+    const float log2e = 1.44269504f;
+    a.position = xyz(own.position);
+    a.normal = xyz(own.normal);
+    a.color = xyz(own.color);
+    a.rough = own.normal.w;
+    a.metal = own.color.w;
+    a.lum = luminance(xyz(c4));
+    a.kz = log2e / wmax(.0001f, own.position.w * (step * .5f));
+    a.kl = log2e / (4.f * sqrtf(variance * (1.f / 16.f)) + .0001f);
+    a.sum = V3{0.f, 0.f, 0.f};
+    a.total = a.v = 0.f;
+    return true;
+}
+template <class R>
+__device__ __forceinline__ void atrous_end(const Atrous& a, typename R::T* out, typename R::T* out2, ptrdiff_t i) {
+    const float dn = 1.f / wmax(a.total, .00001f);
+    const float4 o = make_float4(a.sum.x * dn, a.sum.y * dn, a.sum.z * dn, wmin(sqrtf(a.v) * dn, 65000.f));
     R::store(out, i, o);
     if (out2) R::store(out2, i, o);
 }
 
-template <class G, class R>
-__global__ void __launch_bounds__(256) svgf_atrous_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
-                                                          const typename R::T* input, typename R::T* out,
-                                                          typename R::T* out2, int32_t step) {
-    atrous_body<G, R>(f, c, input, out, out2, step, blockIdx.x * blockDim.x + threadIdx.x,
-                      blockIdx.y * blockDim.y + threadIdx.y);
+// svgf.wgsl:91-110 with the wavelet's step as a constant; `out2` (optional)
+// receives a second copy of the result.
+template <class G, class R, int32_t Step>
+__device__ __forceinline__ void atrous_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* input,
+                                            typename R::T* out, typename R::T* out2, int32_t x, int32_t y) {
+    const int32_t W = (int32_t)f.size[0], H = (int32_t)f.size[1];
+    if (x >= W || y >= H) return;
+    const ptrdiff_t i = (ptrdiff_t)y * W + x;
+    Atrous a;
+    if (!atrous_begin<G, R>(a, c, input, out, out2, W, H, x, y, (float)Step)) return;
+    if (x >= 2 * Step && y >= 2 * Step && x < W - 2 * Step && y < H - 2 * Step) {
+#pragma unroll
+        for (int32_t yy = -2; yy <= 2; yy++) {
+            const TapRow<G> row(c, i + (ptrdiff_t)(yy * Step) * W);
+            const typename R::T* in = input + i + (ptrdiff_t)(yy * Step) * W;
+#pragma unroll
+            for (int32_t xx = -2; xx <= 2; xx++)
+                a.tap(row.at(xx * Step), R::load(in, xx * Step), wavelet_kernel(xx) * wavelet_kernel(yy));
+        }
+    } else {
+#pragma unroll 1
+        for (int32_t k = 0; k < 25; k++) {
+            const int32_t xx = k % 5 - 2, yy = k / 5 - 2, qx = x + xx * Step, qy = y + yy * Step;
+            if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
+            const ptrdiff_t q = (ptrdiff_t)qy * W + qx;
+            a.tap(TapRow<G>(c, q).at(0), R::load(input, q), wavelet_kernel(xx) * wavelet_kernel(yy));
+        }
+    }
+    atrous_end<R>(a, out, out2, i);
+}
+
+template <class G, class R, int32_t Step>
+__global__ void __launch_bounds__(256, 4) svgf_atrous_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
+                                                          const typename R::T* __restrict__ input, typename R::T* __restrict__ out,
+                                                          typename R::T* __restrict__ out2) {
+    atrous_body<G, R, Step>(f, c, input, out, out2, blockIdx.x * blockDim.x + threadIdx.x,
+                            blockIdx.y * blockDim.y + threadIdx.y);
+}
+
+// Calls fn(integral_constant) for a wavelet step 1, 2, 4, 8 or 16 (at most 5 iterations).
+template <class Fn>
+static cudaError_t with_step(int step, Fn&& fn) {
+    switch (step) {
+    case 1: fn(std::integral_constant<int32_t, 1>{}); break;
+    case 2: fn(std::integral_constant<int32_t, 2>{}); break;
+    case 4: fn(std::integral_constant<int32_t, 4>{}); break;
+    case 8: fn(std::integral_constant<int32_t, 8>{}); break;
+    case 16: fn(std::integral_constant<int32_t, 16>{}); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
 }
 
 template <class G, class R, class M>
@@ -152,8 +244,8 @@ __global__ void __launch_bounds__(256, 5) svgf_variance_batched(const irt_frame*
     variance_body<G, R, M>(f, w.c, (const T*)w.in, (const typename M::T*)w.moments_in, (T*)w.out, x, y);
 }
 
-template <class G, class R>
-__global__ void __launch_bounds__(256, 5) svgf_atrous_batched(const irt_frame* __restrict__ frames,
+template <class G, class R, int32_t Step>
+__global__ void __launch_bounds__(256, 4) svgf_atrous_batched(const irt_frame* __restrict__ frames,
                                                            const SView<G>* __restrict__ views,
                                                            const uint32_t* __restrict__ tile_start, uint32_t n) {
     const uint32_t v = svgf_find_view(tile_start, n, blockIdx.x);
@@ -165,7 +257,7 @@ __global__ void __launch_bounds__(256, 5) svgf_atrous_batched(const irt_frame* _
     int32_t x, y;
     svgf_tile_xy(f.size[0], blockIdx.x - __ldg(tile_start + v), x, y);
     typedef typename R::T T;
-    atrous_body<G, R>(f, w.c, (const T*)w.in, (T*)w.out, (T*)w.out2, w.step, x, y);
+    atrous_body<G, R, Step>(f, w.c, (const T*)w.in, (T*)w.out, (T*)w.out2, x, y);
 }
 
 template <class G, class R, class M>
@@ -179,12 +271,14 @@ static cudaError_t spatial_typed(const SvgfLaunch& L, int stage, cudaStream_t st
         svgf_variance_kernel<G, R, M><<<grid, block, 0, st>>>(f, c, (const T*)L.in,
                                                               (const typename M::T*)L.moments_in, (T*)L.out);
     } else if (stage == 2) {
-        // Blocks of 256 pixels of one row: per 1920x1200 frame (4 passes, f32 / mixed storage)
-        // 1.077 / 1.021 ms in 32x8 blocks, 1.062 / 1.018 in 128x2, 1.063 / 1.010 in 64x4,
-        // 1.025 / 0.985 in 256x1 (the variance pass is fastest in 32x8: 0.061 against 0.068 ms).
+        // Blocks of 256 pixels of one row (4 passes at 1920x1200 f32: 0.72 ms; 64x2 0.77, 32x4
+        // 0.77); the variance pass is fastest in 32x8 (0.061 against 0.068 ms in 256x1).
         dim3 block(256, 1);
         dim3 grid((f.size[0] + 255) / 256, f.size[1]);
-        svgf_atrous_kernel<G, R><<<grid, block, 0, st>>>(f, c, (const T*)L.in, (T*)L.out, (T*)L.out2, L.step);
+        return with_step(L.step, [&](auto step) {
+            svgf_atrous_kernel<G, R, decltype(step)::value><<<grid, block, 0, st>>>(f, c, (const T*)L.in, (T*)L.out,
+                                                                                   (T*)L.out2);
+        });
     } else {
         return cudaErrorInvalidValue;
     }
@@ -198,7 +292,10 @@ static cudaError_t spatial_batched_typed(const BatchLaunch& B, int stage, cudaSt
     if (stage == 1)
         svgf_variance_batched<G, R, M><<<B.tiles, block, 0, st>>>(B.frames, views, B.tile_start, B.n);
     else if (stage == 2)
-        svgf_atrous_batched<G, R><<<B.tiles, block, 0, st>>>(B.frames, views, B.tile_start, B.n);
+        return with_step(B.step, [&](auto step) {
+            svgf_atrous_batched<G, R, decltype(step)::value><<<B.tiles, block, 0, st>>>(B.frames, views, B.tile_start,
+                                                                                       B.n);
+        });
     else
         return cudaErrorInvalidValue;
     return cudaGetLastError();
