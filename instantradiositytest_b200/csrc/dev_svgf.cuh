@@ -11,11 +11,9 @@ namespace irtd {
 template <class G>
 struct SvgfCtx {
     G g;
-    const float* old_depth;
     const typename G::NormalT* old_normal;
-    // Per-pixel world positions of this frame and the previous one
-    // (guide_kernel), or null to evaluate world() per tap; both give the
-    // same values.
+    // Per-pixel world positions of this frame and the previous one, w < 0
+    // where depth >= 1 (guide_kernel).
     const float4* guide;
     const float4* old_guide;
     // Per-pixel edge-stopping features of this frame (feature_kernel), two
@@ -95,8 +93,7 @@ struct Sv {
     __device__ __forceinline__ float uvy(int32_t y) const { return ((float)(uint32_t)y + .5f) / (float)H; }
     // svgf.wgsl:19
     __device__ __forceinline__ V3 position(int32_t x, int32_t y) const {
-        if (c.guide) return xyz(__ldg(c.guide + idx(x, y)));
-        return world(uvx(x), uvy(y), c.g.d(idx(x, y)), f.inv_vp);
+        return xyz(__ldg(c.guide + idx(x, y)));
     }
     // svgf.wgsl:20-26
     // `a`, `n`: the pixel's position and (decoded) normal, `reach` =
@@ -104,9 +101,9 @@ struct Sv {
     __device__ __forceinline__ bool history_ok(V3 a, V3 n, float reach, int32_t qx, int32_t qy) const {
         if (f.flags[0] == 0u || f.flags[1] != f.size[3] || !inside(qx, qy)) return false;
         size_t q = idx(qx, qy);
-        float d = __ldg(c.old_depth + q);
-        if (d >= 1.f) return false;
-        V3 b = c.old_guide ? xyz(__ldg(c.old_guide + q)) : world(uvx(qx), uvy(qy), d, f.previous_inv_vp);
+        const float4 guide = __ldg(c.old_guide + q);
+        if (guide.w < 0.f) return false;  // depth >= 1
+        V3 b = xyz(guide);
         return distance(a, b) < reach && dot(n, G::decode_normal(__ldg(c.old_normal + q))) > f.temporal[2];
     }
     __device__ __forceinline__ float history_reach(V3 a) const {
@@ -155,11 +152,11 @@ struct Sv {
                 return wn * wz * wc;
             }
         }
-        float dq = c.g.d(q);
-        if (dq >= 1.f) return 0.f;
+        const float4 guide = __ldg(c.guide + q);
+        if (guide.w < 0.f) return 0.f;  // depth >= 1
         V3 nq = c.g.n(q);
         float wn = pow64(wmax(dot(a.normal, nq), 0.f));
-        V3 wq = c.guide ? xyz(__ldg(c.guide + q)) : world(uvx(qx), uvy(qy), dq, f.inv_vp);
+        V3 wq = xyz(guide);
         float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
         float wz = expf(-fabsf(dot(wq - a.position, a.normal)) / tolerance);
         V3 dc = a.color - c.g.c(q);
@@ -233,7 +230,6 @@ __host__ inline SvgfCtx<G> make_ctx(const SvgfLaunch& L) {
     c.g.color = reinterpret_cast<decltype(c.g.color)>(L.gbuffer.color);
     c.g.params = reinterpret_cast<decltype(c.g.params)>(L.gbuffer.params);
     c.g.motion = reinterpret_cast<decltype(c.g.motion)>(L.gbuffer.motion);
-    c.old_depth = L.old_depth;
     c.old_normal = reinterpret_cast<const typename G::NormalT*>(L.old_normal);
     c.guide = L.guide;
     c.old_guide = L.old_guide;

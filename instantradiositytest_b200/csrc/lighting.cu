@@ -65,7 +65,8 @@ struct Px {
     __device__ __forceinline__ V3 camera() const { return V3{f.camera[0], f.camera[1], f.camera[2]}; }
     __device__ __forceinline__ float uvx(uint32_t qx) const { return ((float)qx + .5f) / (float)f.size[0]; }
     __device__ __forceinline__ float uvy(uint32_t qy) const { return ((float)qy + .5f) / (float)f.size[1]; }
-    __device__ __forceinline__ bool valid() const { return a.g.d(id) < 1.f; }
+    // depth < 1: the guide's w is negative elsewhere.
+    __device__ __forceinline__ bool valid() const { return !(__ldg(&a.guide[id].w) < 0.f); }
     // lighting.wgsl:30-34
     // world(pixel_uv(p), depth, inv_vp) of pixel i, precomputed per frame.
     __device__ __forceinline__ V3 position(size_t i) const { return xyz(__ldg(a.guide + i)); }
@@ -102,9 +103,9 @@ struct Px {
     // lighting.wgsl:36-40
     __device__ __forceinline__ bool compatible(const Surface& s, uint32_t qx, uint32_t qy) const {
         size_t q = (size_t)qy * f.size[0] + qx;
-        float d = a.g.d(q);
-        if (d >= 1.f) return false;
-        V3 p = position(q);
+        const float4 guide = __ldg(a.guide + q);
+        if (guide.w < 0.f) return false;  // depth >= 1
+        V3 p = xyz(guide);
         V3 n = normalize(normal_of(q));
         return dot(s.n, n) > f.temporal[2] && distance(s.p, p) < f.temporal[1] * wmax(distance(s.p, camera()), 1.f);
     }
@@ -122,11 +123,11 @@ struct Px {
             return false;
         size_t q = (size_t)qy * f.size[0] + (size_t)qx;
         if (!index_ok(a.sc.error, q, (size_t)f.size[0] * f.size[1])) return false;
-        float d = __ldg(a.prev_depth + q);
-        if (d >= 1.f) return false;
         // world((q + .5) / size, d, previous_inv_vp): the previous frame's
         // position of q, which is that frame's guide entry.
-        V3 oldp = xyz(__ldg(a.old_guide + q));
+        const float4 guide = __ldg(a.old_guide + q);
+        if (guide.w < 0.f) return false;  // depth >= 1
+        V3 oldp = xyz(guide);
         V3 pn = G::decode_normal(__ldg(a.prev_normal + q));
         return dot(s.n, pn) > f.temporal[2] && distance(s.p, oldp) < f.temporal[1] * wmax(distance(s.p, camera()), 1.f);
     }
@@ -153,8 +154,10 @@ struct Px {
     __device__ __forceinline__ void neighbor(uint32_t& rng, int32_t& qx, int32_t& qy) const {
         float angle = 2.f * kPI * rnd(rng);
         float radius = sqrtf(rnd(rng)) * (float)f.restir[3];
-        qx = (int32_t)x + to_i32(rintf(cosf(angle) * radius));
-        qy = (int32_t)y + to_i32(rintf(sinf(angle) * radius));
+        float sn, cs;  // one range reduction for both
+        sincosf(angle, &sn, &cs);
+        qx = (int32_t)x + to_i32(rintf(cs * radius));
+        qy = (int32_t)y + to_i32(rintf(sn * radius));
     }
 
     // ---------------------------------------------------------------- passes
@@ -222,8 +225,10 @@ struct Px {
                 if (qx < 0 || qy < 0 || qx >= (int32_t)f.size[0] || qy >= (int32_t)f.size[1]) continue;
                 if (!index_ok(a.sc.error, (size_t)qy * f.size[0] + (size_t)qx, (size_t)f.size[0] * f.size[1]))
                     continue;
-                if (!compatible(s, (uint32_t)qx, (uint32_t)qy)) continue;
+                // The reservoir is loaded beside the compatibility test's reads
+                // (spatial 0.455 -> 0.438 ms at 1920x1200).
                 Res previous = res_load(in, (size_t)qy * f.size[0] + (size_t)qx);
+                if (!compatible(s, (uint32_t)qx, (uint32_t)qy)) continue;
                 if (Dom == 0) {
                     if (previous.target > 0.f && index_ok(a.sc.error, previous.id, f.counts[0])) {
                         float target = luminance(direct(s, load_light(a.sc.lights, previous.id)));

@@ -6,6 +6,7 @@
 // One thread per pixel in 32x8 blocks.
 #include <cuda_runtime.h>
 
+#define IRT_PLAIN_SUMS 1
 #include "dev_svgf.cuh"
 #include "kernels.h"
 
@@ -31,7 +32,7 @@ __device__ __forceinline__ void temporal_body(const irt_frame& f, const SvgfCtx<
     V3 history = V3{0.f, 0.f, 0.f};
     float hm0 = 0.f, hm1 = 0.f, length_history = 0.f, total = 0.f;
     float tap_w[4] = {0.f, 0.f, 0.f, 0.f}, tap_mean[4], tap_dev[4];  // MomF16 only
-    if (c.g.d(i) < 1.f) {
+    if (!(__ldg(&c.guide[i].w) < 0.f)) {  // depth < 1
         float2 mv = c.g.mv(i);
         float px = (sv.uvx(x) - mv.x) * (float)sv.W - .5f;
         float py = (sv.uvy(y) - mv.y) * (float)sv.H - .5f;

@@ -26,7 +26,7 @@ __device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<
     Moments centre = M::load(moments, i);
     float age = centre.age;
     float sigma = in.w;
-    if (age < 4.f && c.g.d(i) < 1.f) {
+    if (age < 4.f && !(__ldg(&c.guide[i].w) < 0.f)) {  // young, depth < 1
         float s0 = 0.f, s1 = 0.f, total = 0.f;
         const float K = M::central ? centre.mean : 0.f;
         Guide a = sv.guide(x, y);

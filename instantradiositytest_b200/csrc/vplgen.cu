@@ -9,6 +9,7 @@
 // runs against the workload's primitive table (dev_prims.cuh).
 #include <cuda_runtime.h>
 
+#define IRT_PLAIN_SUMS 1
 #include "dev_common.cuh"
 #include "dev_prims.cuh"
 #include "kernels.h"
