@@ -62,6 +62,7 @@ struct ParityTables {
     MarchQueue* queues = nullptr;  // device
     std::vector<uint32_t> wave_groups;  // groups of wave w: [wave_groups[w], wave_groups[w + 1])
     uint32_t max_scene_bytes = 0;
+    int sampler = 0;               // of every group, or 3 where they differ
     cudaGraphExec_t graph = nullptr;
     int renders = 0;               // direct renders of this parity since the tables were built
 };
@@ -194,11 +195,13 @@ std::vector<uintptr_t> signature_of(const irt_batch* b, irt_scene* const* scenes
                             (uintptr_t)sc->lights_prep, (uintptr_t)sc->atlas, (uintptr_t)sc->march_scene,
                             (uintptr_t)sc->cells, sc->object_count, (uintptr_t)g[v].depth, (uintptr_t)g[v].normal,
                             (uintptr_t)g[v].color, (uintptr_t)g[v].params, (uintptr_t)g[v].motion,
-                            (uintptr_t)cur[v], (uintptr_t)prev[v], frames[v].counts[0], frames[v].counts[3]};
+                            (uintptr_t)cur[v], (uintptr_t)prev[v], frames[v].counts[0], frames[v].counts[3],
+                            (uintptr_t)sc->field_linear};
         sig.insert(sig.end(), std::begin(vals), std::end(vals));
-        uint32_t gi[6];
+        uint32_t gi[7];
         std::memcpy(gi, sc->grid_org, 12);
         std::memcpy(gi + 3, sc->grid_inv, 12);
+        std::memcpy(gi + 6, &sc->grid_slack, 4);
         sig.insert(sig.end(), std::begin(gi), std::end(gi));
     }
     return sig;
@@ -309,6 +312,9 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
                 G.grid_inv[a] = sc->grid_inv[a];
                 G.grid_size[a] = sc->grid_size[a];
             }
+            G.grid_slack = sc->grid_slack;
+            const int sampler = march_sampler(G.field_filter, G.sdf_f16);
+            t.sampler = groups.empty() || t.sampler == sampler ? sampler : 3;
             groups.push_back(G);
         }
         t.wave_groups.push_back((uint32_t)groups.size());
@@ -418,6 +424,7 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
         M.num_sms = b->num_sms;
         M.blocks_per_sm = kMarchBps[march_choice];
         M.fast = 1;
+        M.sampler = t.sampler;
         CK(irt_launch_ray_pools_batched(M, st), "batch ray pools");
         mark(3);
         CK(irt_launch_lighting_batched(batch_launch(b, w, t.largs, la, shape_of[kTReuse]), kStageReuse, st),

@@ -3,7 +3,9 @@
 // Svgf::encode (src/svgf.rs:140-261).  No exception crosses the boundary.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -330,6 +332,20 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
             sc->grid_size[a] = LC.grid_size[a] = (float)((hi - lo) / kGridRes);
             sc->grid_inv[a] = (float)(kGridRes / (hi - lo));
         }
+        // The f32 error of a distance and of a point's place in its cell; for
+        // the filtered sampler also what its weights may miss by.
+        double d2 = 0, far = 0, voxel = 0;
+        for (int a = 0; a < 3; a++) {
+            d2 += (double)sc->grid_size[a] * sc->grid_size[a];
+            far = std::max(far, std::max(std::fabs((double)nodes[0].lo[a]), std::fabs((double)nodes[0].hi[a])));
+        }
+        for (uint32_t i = 0; i < object_count; i++) {
+            float v;
+            std::memcpy(&v, &objects[i].info[3], 4);
+            voxel = std::max(voxel, (double)v);
+        }
+        LC.margin = (float)(1e-4 + 1e-3 * 0.5 * std::sqrt(d2) + 1e-6 * far);
+        sc->grid_slack = LC.margin + (float)voxel * LC.field_filter.bound_slack;
         LC.cells = reinterpret_cast<uint32_t*>(sc->cells);
         CK(irt_launch_leaf_cache(LC, st), "leaf cache");
         sc->cached_nodes.assign(nodes, nodes + node_count);
@@ -674,6 +690,7 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
             M.grid_inv[a] = sc->grid_inv[a];
             M.grid_size[a] = sc->grid_size[a];
         }
+        M.grid_slack = sc->grid_slack;
         M.setup = session_ray_setup(s, sc, cur, prev);
         M.num_sms = s->num_sms;
         M.fast = s->desc.exact_march ? 0 : 1;

@@ -64,6 +64,7 @@ struct irt_scene {
     std::vector<irt_node> cached_nodes;
     std::vector<irt_object> cached_objects;
     float grid_org[3] = {0, 0, 0}, grid_inv[3] = {0, 0, 0}, grid_size[3] = {0, 0, 0};
+    float grid_slack = 0;  // error of an evaluated object distance
     uint32_t object_count = 0, light_count = 0;
     uint64_t bytes = 0;
 };

@@ -87,7 +87,7 @@ __device__ __forceinline__ float sample_linear(const DevScene& sc, V3 origin, fl
     const float v = __fadd_rn(__fadd_rn(origin.y, q.y), .5f);
     const float w = __fadd_rn(__fadd_rn(origin.z, q.z), .5f);
     const float value = tex3D<float>(sc.filter.linear, u, v, w);
-    return sc.sdf_f16 ? value * f16_scale : value;
+    return sc.sdf_f16 ? __fmul_rn(value, f16_scale) : value;  // rounded before the bound is taken off
 }
 
 // common.wgsl:31-38 — the cell's 8 texels, weights in z, y, x order as the
@@ -120,7 +120,7 @@ __device__ __forceinline__ float sample_cell(const DevScene& sc, uint32_t cell, 
     const float x2 = fmaf(fx, t[5] - t[4], t[4]), x3 = fmaf(fx, t[7] - t[6], t[6]);
     const float y0 = fmaf(fy, x1 - x0, x0), y1 = fmaf(fy, x3 - x2, x2);
     const float value = fmaf(fz, y1 - y0, y0);
-    return sc.sdf_f16 ? value * f16_scale : value;
+    return sc.sdf_f16 ? __fmul_rn(value, f16_scale) : value;  // rounded before the bound is taken off
 #else
     if (sc.sdf_f16) {
         float s = f16_scale;

@@ -113,7 +113,7 @@ struct MarchLaunch {
     // first kCellEntries objects by increasing lower bound of their distance
     // from the cell's centre, those bounds and the next one as a sentinel.
     const uint4* cells;
-    float grid_org[3], grid_inv[3], grid_size[3];
+    float grid_org[3], grid_inv[3], grid_size[3], grid_slack;
     RaySetup setup;
     int num_sms;
     int fast;  // 1: approximate division / square root build (march_fast.cu)
@@ -144,6 +144,7 @@ struct LeafCacheLaunch {
     const void* sdf_cells;  // corner cells of the field meshes (dev_sdf.cuh), or null
     irtd::FieldFilter field_filter;
     float grid_org[3], grid_size[3];  // as the march reads them
+    float margin;               // f32 error of a distance and of a point's place in its cell
     uint32_t* cells;            // kGridRes^3 * kCellWords words
 };
 cudaError_t irt_launch_leaf_cache(const LeafCacheLaunch& L, cudaStream_t st);
@@ -249,7 +250,7 @@ struct alignas(16) MarchGroup {
     const float4* march_scene;
     uint32_t scene_vec4;
     const uint4* cells;
-    float grid_org[3], grid_inv[3], grid_size[3];
+    float grid_org[3], grid_inv[3], grid_size[3], grid_slack;
     uint32_t q_begin, q_end;    // the group's queues in the queue table
 };
 struct MarchBatch {
@@ -260,7 +261,11 @@ struct MarchBatch {
     int num_sms;
     int blocks_per_sm;          // 0 = occupancy maximum
     int fast;
+    int sampler;                // march_sampler() of every group, or 3 where they differ
 };
+// Which build of the march kernel a scene's fields take: point-sampled f32 (0)
+// or f16 (1) corner cells, or the filtered atlas (2, f32 only).
+inline int march_sampler(const irtd::FieldFilter& filter, int sdf_f16) { return filter.linear ? 2 : sdf_f16 ? 1 : 0; }
 cudaError_t irt_launch_ray_pools_batched(const MarchBatch& M, cudaStream_t st);
 cudaError_t irt_launch_march_batched(const MarchBatch& M, cudaStream_t st);
 // Lights with the spot direction normalised and cos(angle / 2) in

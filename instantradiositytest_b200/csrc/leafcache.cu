@@ -103,15 +103,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32) cell_build_kernel(const DevS
 cudaError_t irt_launch_leaf_cache(const LeafCacheLaunch& L, cudaStream_t st) {
     using namespace irtd;
     CacheGrid g;
-    double d2 = 0, far = 0;
     for (int a = 0; a < 3; a++) {
         g.org[a] = L.grid_org[a];
         g.size[a] = L.grid_size[a];
-        d2 += (double)g.size[a] * g.size[a];
-        far = fmax(far, fmax(fabs((double)g.org[a]), fabs((double)g.org[a] + g.size[a] * (double)kGridRes)));
     }
-    // The f32 error of a point's place in its cell and of the distances there.
-    g.margin = (float)(1e-4 + 1e-3 * 0.5 * sqrt(d2) + 1e-6 * far);
+    g.margin = L.margin;
     g.slope = L.sdf_f16 ? 1.f - 2e-3f : 1.f - 2e-4f;
     DevScene sc{};
     sc.atlas = L.atlas;
