@@ -19,7 +19,8 @@
 // of which the set-up is 0.14 ms; leaf bounds taken at the query point
 // (leafcache.cu; 1.31 -> 1.13 evaluations a query, fewer entries tested)
 // 2.11; short divides, flushed denormals, 256-bit cell loads 2.05; the cell
-// found anew per candidate search instead of kept, 1.98; 36 warps 1.89.
+// found anew per candidate search instead of kept, 1.98; 36 warps 1.89; a
+// kernel per field sampler 1.84; rays sorted by end (ray_setup_block) 1.68.
 //
 // scene_distance (sdf.wgsl:42-60) returns the minimum object distance: the
 // walk skips a subtree only when its box bound exceeds the current best, and
@@ -266,21 +267,45 @@ __device__ __forceinline__ void ray_pool_entry(const RaySetup& s, const DevScene
     }
 }
 
-// One warp's 8x4 pixels of the ray set-up: the pixel's clearance, the
-// begin of its rays' marches, and their records appended to the queue (one
-// atomic per ray class and warp).  VPL rays fill the queue from the front and
+// The ray set-up of a block's 32x16 pixels (a warp takes 8x4 of them): each
+// pixel's clearance, the begin of its rays' marches, and their records
+// appended to the queue, the block's rays of a class sorted by where they end
+// (one atomic per class and block).  The pixels of a block see nearly the same
+// point, so rays to neighbouring ends stay together all the way: the march's
+// warps meet the same objects.  VPL rays fill the queue from the front and
 // light rays from the back (ray_slot), so the march takes whole runs of one
 // class; each ray's result slot is in its record, so the order changes no
 // result.  Rays resolved without a march step write their visibility here.
-constexpr uint32_t kTileW = 8, kTileH = 4;
-__device__ __forceinline__ void ray_setup_tile(const RaySetup& s, const DevScene& sc, const Grid& g,
-                                               const SceneRefs& R, uint32_t W, uint32_t H, uint32_t tile,
-                                               uint32_t lane) {
+constexpr uint32_t kSetupThreads = 512, kSetupW = 32, kSetupH = 16;
+constexpr uint32_t kEndBins = 512;  // 8x8x8 over the cache grid, in Morton order
+struct SetupShared {
+    uint32_t bins[kEndBins];  // rays per end: VPL rays in the low half, light rays in the high half
+    uint32_t warp_total[kSetupThreads / 32];
+    uint32_t base[2];
+};
+static_assert(kEndBins == kSetupThreads, "one bin a thread in the scan");
+
+__device__ __forceinline__ uint32_t end_bin(const Grid& g, V3 p) {
+    auto axis = [](float f) {  // 0..7, spread to every third bit
+        const uint32_t c = (uint32_t)fminf(fmaxf(f, 0.f), (float)(kGridRes - 1)) / (kGridRes / 8);
+        return (c & 1u) | (c & 2u) << 2 | (c & 4u) << 4;
+    };
+    return axis((p.x - g.ox) * g.ix) | axis((p.y - g.oy) * g.iy) << 1 | axis((p.z - g.oz) * g.iz) << 2;
+}
+
+__device__ __forceinline__ void ray_setup_block(const RaySetup& s, const DevScene& sc, const Grid& g,
+                                                const SceneRefs& R, uint32_t W, uint32_t H, uint32_t tile,
+                                                SetupShared& sh) {
     const unsigned full = 0xffffffffu;
-    const uint32_t across = (W + kTileW - 1) / kTileW;
-    const uint32_t x = (tile % across) * kTileW + lane % kTileW, y = (tile / across) * kTileH + lane / kTileW;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t / 32u;
+    const uint32_t across = (W + kSetupW - 1) / kSetupW;
+    const uint32_t x = (tile % across) * kSetupW + (warp & 3u) * 8u + (lane & 7u);
+    const uint32_t y = (tile / across) * kSetupH + (warp >> 2) * 4u + (lane >> 3);
     const uint32_t i = y * W + x;
-    uint32_t light = kNoRay, vpl = kNoRay, hint = kNone;
+    __syncthreads();  // the previous tile's bins are read
+    sh.bins[t] = 0u;
+    __syncthreads();
+    uint32_t light = kNoRay, vpl = kNoRay, hint = kNone, bin_d = 0, bin_v = 0, rank_d = 0, rank_v = 0;
     MarchState d, v;
     if (x < W && y < H) {
         const float4 prep = __ldg(s.prep + i);
@@ -293,11 +318,14 @@ __device__ __forceinline__ void ray_setup_tile(const RaySetup& s, const DevScene
             v.origin = d.origin;
         }
         if (light != kNoRay) {
-            const float out = march_begin(d, xyz(__ldg(reinterpret_cast<const float4*>(s.lights + light))), R.eps,
-                                          R.max_steps);
+            const V3 end = xyz(__ldg(reinterpret_cast<const float4*>(s.lights + light)));
+            const float out = march_begin(d, end, R.eps, R.max_steps);
             if (out >= 0.f) {
                 s.vis[2 * (size_t)i] = out;
                 light = kNoRay;
+            } else {
+                bin_d = end_bin(g, end);
+                rank_d = atomicAdd(&sh.bins[bin_d], 1u << 16) >> 16;
             }
         }
         if (vpl != kNoRay) {
@@ -312,27 +340,42 @@ __device__ __forceinline__ void ray_setup_tile(const RaySetup& s, const DevScene
             if (out >= 0.f) {
                 s.vis[2 * (size_t)i + 1] = out;
                 vpl = kNoRay;
+            } else {
+                bin_v = end_bin(g, end);
+                rank_v = atomicAdd(&sh.bins[bin_v], 1u) & 0xffffu;
             }
         }
     }
-    const unsigned bd = __ballot_sync(full, light != kNoRay), bi = __ballot_sync(full, vpl != kNoRay);
-    uint32_t base_i = 0, base_d = 0;
-    if (lane == 0) {
-        if (bi) base_i = atomicAdd(s.counters, (uint32_t)__popc(bi));
-        if (bd) base_d = atomicAdd(s.counters + 2, (uint32_t)__popc(bd));
+    __syncthreads();
+    // Exclusive prefix sums of both classes at once (at most 512 rays each).
+    const uint32_t own = sh.bins[t];
+    uint32_t sum = own;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(full, sum, o);
+        if (lane >= o) sum += up;
     }
-    base_i = __shfl_sync(full, base_i, 0);
-    base_d = __shfl_sync(full, base_d, 0);
+    if (lane == 31u) sh.warp_total[warp] = sum;
+    __syncthreads();
+    uint32_t before = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kSetupThreads / 32; k++) before += k < warp ? sh.warp_total[k] : 0u;
+    sh.bins[t] = before + sum - own;
+    if (t == kSetupThreads - 1) {
+        const uint32_t total = before + sum;
+        sh.base[0] = total & 0xffffu ? atomicAdd(s.counters, total & 0xffffu) : 0u;
+        sh.base[1] = total >> 16 ? atomicAdd(s.counters + 2, total >> 16) : 0u;
+    }
+    __syncthreads();
     const uint32_t cap = 2u * W * H;
-    const unsigned below = (1u << lane) - 1u;
     auto emit = [&](const MarchState& m, uint32_t at, uint32_t slot) {
         if (!index_ok(sc.error, at, cap)) return;
         s.rays[at].a = make_float4(m.origin.x, m.origin.y, m.origin.z, __uint_as_float(slot));
         s.rays[at].b = make_float4(m.dir.x, m.dir.y, m.dir.z, m.limit);
         s.hints[at] = (uint16_t)hint;
     };
-    if (vpl != kNoRay) emit(v, base_i + (uint32_t)__popc(bi & below), 2u * i + 1u);
-    if (light != kNoRay) emit(d, cap - 1u - (base_d + (uint32_t)__popc(bd & below)), 2u * i);
+    if (vpl != kNoRay) emit(v, sh.base[0] + (sh.bins[bin_v] & 0xffffu) + rank_v, 2u * i + 1u);
+    if (light != kNoRay) emit(d, cap - 1u - (sh.base[1] + (sh.bins[bin_d] >> 16) + rank_d), 2u * i);
 }
 
 // A warp's reserved slice [next, end) of a ray queue; `drained` once the
@@ -474,19 +517,18 @@ __global__ void __launch_bounds__(kMarchThreads) ray_pools_kernel(const __grid_c
     for (uint32_t v = t; v < n; v += gridDim.x * blockDim.x) ray_pool_entry(setup, sc, grid, R, f.size[2], v);
 }
 
-__global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) ray_setup_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
+__global__ void __launch_bounds__(kSetupThreads, 2) ray_setup_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
                                                                   const float4* __restrict__ march_scene,
                                                                   uint32_t scene_vec4, const Grid grid,
                                                                   const __grid_constant__ RaySetup setup) {
     extern __shared__ float4 smem[];
+    __shared__ SetupShared sh;
     for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
     __syncthreads();
     const SceneRefs R = scene_refs(f, smem);
     const uint32_t W = f.size[0], H = f.size[1];
-    const uint32_t tiles = ((W + kTileW - 1) / kTileW) * ((H + kTileH - 1) / kTileH);
-    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
-    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 32u; t < tiles; t += warps)
-        ray_setup_tile(setup, sc, grid, R, W, H, t, threadIdx.x & 31u);
+    const uint32_t tiles = ((W + kSetupW - 1) / kSetupW) * ((H + kSetupH - 1) / kSetupH);
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) ray_setup_block(setup, sc, grid, R, W, H, t, sh);
 }
 
 template <int S>
@@ -579,21 +621,21 @@ __global__ void __launch_bounds__(128) ray_pools_batched_kernel(const MarchGroup
     }
 }
 
-__global__ void __launch_bounds__(128, kMarchBlocksPerSm) ray_setup_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
+__global__ void __launch_bounds__(kSetupThreads, 2) ray_setup_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
                                                             const MarchQueue* __restrict__ queues) {
     extern __shared__ float4 smem[];
-    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    __shared__ SetupShared sh;
     for (uint32_t g = 0; g < n_groups; g++) {
         const MarchGroup& G = stage_group(groups, g, smem);
         const DevScene sc = group_scene(G);
         const Grid grid = group_grid(G);
         const SceneRefs R = scene_refs(G.f, smem + kGroupVec4);
-        uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
+        uint32_t t = blockIdx.x;
         for (uint32_t q = G.q_begin; q < G.q_end; q++) {
             const MarchQueue& Q = queues[q];
-            const uint32_t tiles = ((Q.width + kTileW - 1) / kTileW) * ((Q.height + kTileH - 1) / kTileH);
+            const uint32_t tiles = ((Q.width + kSetupW - 1) / kSetupW) * ((Q.height + kSetupH - 1) / kSetupH);
             const RaySetup s = Q.setup;
-            for (; t < tiles; t += warps) ray_setup_tile(s, sc, grid, R, Q.width, Q.height, t, threadIdx.x & 31u);
+            for (; t < tiles; t += gridDim.x) ray_setup_block(s, sc, grid, R, Q.width, Q.height, t, sh);
             t -= tiles;
         }
     }
@@ -747,12 +789,12 @@ cudaError_t IRT_MARCH_FN(irt_launch_march)(const MarchLaunch& M, cudaStream_t st
     const int sampler = march_sampler(M.field_filter, M.sdf_f16);
     thread_local KernelFit set_up, fits[3];
     KernelFit& march = fits[sampler];
-    cudaError_t e = set_up.set((const void*)ray_setup_kernel, kMarchThreads, smem, kMarchCtasPerSm);
+    cudaError_t e = set_up.set((const void*)ray_setup_kernel, kSetupThreads, smem, 2);
     if (e == cudaSuccess) e = march.set((const void*)kernels[sampler], kMarchThreads, smem, kMarchCtasPerSm);
     if (e != cudaSuccess) return e;
     const irtd::DevScene sc = launch_scene(M);
     const Grid g = launch_grid(M);
-    ray_setup_kernel<<<M.num_sms * set_up.per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
+    ray_setup_kernel<<<M.num_sms * set_up.per_sm, kSetupThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
                                                                              M.setup);
     kernels[sampler]<<<M.num_sms * march.per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
                                                                             M.setup);
@@ -780,11 +822,11 @@ cudaError_t IRT_MARCH_FN(irt_launch_march_batched)(const MarchBatch& M, cudaStre
     if (M.sampler < 0 || M.sampler > kAnySampler) return cudaErrorInvalidValue;
     thread_local KernelFit set_up, fits[4];
     KernelFit& march = fits[M.sampler];
-    cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, 128, smem, kMarchBlocksPerSm);
+    cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, kSetupThreads, smem, 2);
     if (e == cudaSuccess) e = march.set((const void*)kernels[M.sampler], 128, smem, kMarchBlocksPerSm);
     if (e != cudaSuccess) return e;
     const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < march.per_sm ? M.blocks_per_sm : march.per_sm;
-    ray_setup_batched_kernel<<<M.num_sms * set_up.per_sm, 128, smem, st>>>(M.groups, M.n_groups, M.queues);
+    ray_setup_batched_kernel<<<M.num_sms * set_up.per_sm, kSetupThreads, smem, st>>>(M.groups, M.n_groups, M.queues);
     kernels[M.sampler]<<<M.num_sms * bps, 128, smem, st>>>(M.groups, M.n_groups, M.queues);
     return cudaGetLastError();
 }
