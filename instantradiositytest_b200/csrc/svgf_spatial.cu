@@ -2,9 +2,8 @@
 // (svgf.wgsl:90-110) as sm_100a CUDA, built with fast math (approximate
 // exp, division and square root): these passes only weight and average
 // radiance, and their inputs (positions, history length) come exactly from
-// the guide and temporal kernels.  One thread per pixel (variance in 32x8
-// blocks, a-trous in blocks of 256 pixels of a row); neighbour taps read
-// through L1.
+// the guide and temporal kernels.  Variance in 32x8 blocks, a-trous one thread
+// per pixel in blocks of 256 pixels of a row; neighbour taps read through L1.
 #include <cuda_runtime.h>
 
 #include "dev_svgf.cuh"
@@ -12,70 +11,7 @@
 
 namespace irtd {
 
-// svgf.wgsl:77-89
-// With MomF16 (mean, deviation) moments the 7x7 sums are taken about the
-// centre pixel's mean (shifted data), so E[l^2] - E[l]^2 is formed from
-// small numbers: s0 = sum w (m - K), s1 = sum w (dev^2 + (m - K)^2).
-template <class G, class R, class M>
-__device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* input,
-                                              const typename M::T* moments, typename R::T* out, int32_t x, int32_t y) {
-    Sv<G> sv(f, c);
-    if (x >= sv.W || y >= sv.H) return;
-    size_t i = sv.idx(x, y);
-    float4 in = R::load(input, i);
-    Moments centre = M::load(moments, i);
-    float age = centre.age;
-    float sigma = in.w;
-    if (age < 4.f && !(__ldg(&c.guide[i].w) < 0.f)) {  // young, depth < 1
-        float s0 = 0.f, s1 = 0.f, total = 0.f;
-        const float K = M::central ? centre.mean : 0.f;
-        Guide a = sv.guide(x, y);
-        for (int32_t yy = -3; yy <= 3; yy++)
-            for (int32_t xx = -3; xx <= 3; xx++) {
-                int32_t qx = x + xx, qy = y + yy;
-                float w = sv.geometry_weight(a, qx, qy, 1.f);
-                if (w <= 0.f) continue;
-                Moments m = M::load(moments, sv.idx(qx, qy));
-                if constexpr (M::central) {
-                    float d = m.mean - K;
-                    s0 += d * w;
-                    s1 += (m.second * m.second + d * d) * w;
-                } else {
-                    s0 += m.mean * w;
-                    s1 += m.second * w;
-                }
-                total += w;
-            }
-        float dn = wmax(total, .00001f);
-        s0 /= dn;
-        s1 /= dn;
-        sigma = sqrtf(wmax(s1 - s0 * s0, 0.f) * 4.f / wmax(age, 1.f));
-    }
-    R::store(out, i, make_float4(in.x, in.y, in.z, wmin(sigma, 65000.f)));
-}
-
-template <class G, class R, class M>
-__global__ void __launch_bounds__(256) svgf_variance_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
-                                                            const typename R::T* input, const typename M::T* moments,
-                                                            typename R::T* out) {
-    variance_body<G, R, M>(f, c, input, moments, out, blockIdx.x * blockDim.x + threadIdx.x,
-                           blockIdx.y * blockDim.y + threadIdx.y);
-}
-
-// A-trous: 25 taps a pixel, bound by L1 bandwidth (64 bytes a tap with f32
-// radiance) and load latency.  Per 1920x1200 pass, f32 / mixed storage, 256 / 246 us
-// before: a tap reads the guide and the feature record (one 128-bit and one
-// 256-bit load, also for f32 planes, whose five loads a tap cost 197 us with
-// all of the following), the wavelet step is a template constant so that the
-// taps of a row are immediate offsets, interior pixels test no bounds, the
-// three exponentials of a tap are one exp2 of the summed exponents with the
-// two divisors inverted once a pixel, no branch stands between the loads of
-// one tap and the next, and the 25 taps are unrolled (179 / 166 us with the
-// rows rolled): 173 / 156 us.  Two pixels a step apart per thread (30 taps
-// read instead of 50) 182 / 180; blocks of 32x4 176 us for step 1, 194-215 for
-// the others.
-//
-// What an a-trous tap reads of a pixel besides its radiance: position (w < 0:
+// What a tap reads of a pixel besides its radiance or moments: position (w < 0:
 // background), normal and roughness, colour and metal.
 struct TapGeometry {
     float4 position, normal, color;
@@ -98,32 +34,205 @@ struct TapRow {
     }
 };
 
+// A pixel's own terms of the geometry weight of its taps (svgf.wgsl:32-44).
+struct TapCentre {
+    V3 position, normal, color;
+    float rough, metal;
+    float kz;  // log2(e) over the plane-distance tolerance
+    __device__ __forceinline__ void set(const TapGeometry& own, float step) {
+        position = xyz(own.position);
+        normal = xyz(own.normal);
+        color = xyz(own.color);
+        rough = own.normal.w;
+        metal = own.color.w;
+        kz = 1.44269504f / wmax(.0001f, own.position.w * (step * .5f));
+    }
+    // The tap's normal weight, and in `geom` the plane-distance, colour and
+    // parameter terms as one exponent of 2; false where the weight is 0
+    // (background, or one of its factors underflows).
+    __device__ __forceinline__ bool weigh(const TapGeometry& t, float& wn, float& geom) const {
+        const float kc = 8.f * 1.44269504f;
+        wn = pow64(wmax(dot(normal, xyz(t.normal)), 0.f));
+        const V3 dc = color - xyz(t.color);
+        const float d0 = rough - t.normal.w, d1 = metal - t.color.w;
+        geom = fmaf(length(dc) + sqrtf(fmaf(d0, d0, d1 * d1)), kc, fabsf(dot(xyz(t.position) - position, normal)) * kz);
+        return !(t.position.w < 0.f || !(wn > 0.f) || geom > 126.f);
+    }
+};
+
+// svgf.wgsl:77-89
+// With MomF16 (mean, deviation) moments the 7x7 sums are taken about the
+// centre pixel's mean (shifted data), so E[l^2] - E[l]^2 is formed from
+// small numbers: s0 = sum w (m - K), s1 = sum w (dev^2 + (m - K)^2).
+// The sums of svgf_variance over the taps of one pixel.
+template <class M>
+struct VarianceSums {
+    float s0 = 0.f, s1 = 0.f, total = 0.f;
+    // The row of taps py + yy; without a branch before the sums, so that its
+    // seven taps' loads issue together.
+    template <class G>
+    __device__ __forceinline__ void row(const SvgfCtx<G>& c, const TapCentre& a, const typename M::T* moments, float K,
+                                        int32_t W, int32_t H, int32_t px, int32_t py, int32_t yy) {
+        const int32_t qy = py + yy;
+        const bool row_in = yy <= 3 && qy >= 0 && qy < H;
+        const ptrdiff_t at = (ptrdiff_t)min(max(qy, 0), H - 1) * W;
+#pragma unroll
+        for (int32_t xx = -3; xx <= 3; xx++) {
+            const int32_t qx = px + xx;
+            const ptrdiff_t q = at + min(max(qx, 0), W - 1);
+            const TapGeometry g = TapRow<G>(c, q).at(0);
+            const Moments m = M::load(moments, q);
+            float wn, geom;
+            const bool counts = a.weigh(g, wn, geom) && row_in && qx >= 0 && qx < W;
+            const float w = wn * exp2f(-geom);
+            if (!counts) continue;
+            if constexpr (M::central) {
+                float d = m.mean - K;
+                s0 += d * w;
+                s1 += fmaf(m.second, m.second, d * d) * w;
+            } else {
+                s0 += m.mean * w;
+                s1 += m.second * w;
+            }
+            total += w;
+        }
+    }
+    __device__ __forceinline__ void add(const VarianceSums& o) {
+        s0 += o.s0;
+        s1 += o.s1;
+        total += o.total;
+    }
+    __device__ __forceinline__ float sigma(float age) const {
+        const float dn = wmax(total, .00001f);
+        const float m0 = s0 / dn, m1 = s1 / dn;
+        return sqrtf(wmax(m1 - m0 * m0, 0.f) * 4.f / wmax(age, 1.f));
+    }
+};
+
+// Only pixels with a young history (disocclusions; every pixel of the first
+// frames) take the 49 taps.  A block of 256 lists its young pixels.  Up to 64
+// of them: eight lanes take a pixel, a row of taps each, since what a few
+// young pixels cost is the latency of their loads one after the other.  More:
+// a thread a pixel, whose loads coalesce.  160x100 25 -> 12 us, 480x300 31 -> 18,
+// 960x600 with moving objects 44 -> 32, 1920x1200 f32 / mixed 96 / 101 -> 82 / 76;
+// all young at 1920x1200 355 -> 312 (1235 with eight lanes each).  Lists up to
+// 32 leave 160x100 at 14, up to 128 take 960x600 to 43.
+constexpr uint32_t kSpreadYoung = 64;
+template <class G, class R, class M>
+__device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* input,
+                                              const typename M::T* moments, typename R::T* out, int32_t x, int32_t y) {
+    __shared__ uint32_t list[256], listed;
+    const unsigned full = 0xffffffffu;
+    const int32_t W = (int32_t)f.size[0], H = (int32_t)f.size[1];
+    const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x, lane = t & 31u;
+    if (t == 0) listed = 0u;
+    __syncthreads();
+    bool young = false;
+    if (x < W && y < H) {
+        const ptrdiff_t i = (ptrdiff_t)y * W + x;
+        young = M::load(moments, i).age < 4.f && !(__ldg(&c.guide[i].w) < 0.f);  // depth < 1
+        if (!young) {
+            float4 in = R::load(input, i);
+            in.w = wmin(in.w, 65000.f);
+            R::store(out, i, in);
+        }
+    }
+    const unsigned in_warp = __ballot_sync(full, young);
+    uint32_t base = 0;
+    if (lane == 0u && in_warp) base = atomicAdd(&listed, (uint32_t)__popc(in_warp));
+    base = __shfl_sync(full, base, 0);
+    if (young) list[base + (uint32_t)__popc(in_warp & ((1u << lane) - 1u))] = (uint32_t)x | (uint32_t)y << 16;
+    __syncthreads();
+    const uint32_t n = listed;
+    auto pixel = [&](uint32_t k, auto&& sums) {
+        const int32_t px = (int32_t)(list[k] & 0xffffu), py = (int32_t)(list[k] >> 16);
+        const ptrdiff_t i = (ptrdiff_t)py * W + px;
+        const Moments centre = M::load(moments, i);
+        TapCentre a;
+        a.set(TapRow<G>(c, i).at(0), 1.f);
+        VarianceSums<M> v;
+        if (!sums(v, a, M::central ? centre.mean : 0.f, px, py)) return;
+        const float4 in = R::load(input, i);
+        R::store(out, i, make_float4(in.x, in.y, in.z, wmin(v.sigma(centre.age), 65000.f)));
+    };
+    if (n > kSpreadYoung) {
+        if (t < n)
+            pixel(t, [&](VarianceSums<M>& v, const TapCentre& a, float K, int32_t px, int32_t py) {
+                // rows added as the eight lanes' exchange adds them, so that a
+                // pixel's value does not depend on its block's list
+                VarianceSums<M> hold, half;
+#pragma unroll 1
+                for (int32_t k = 0; k < 7; k++) {
+                    VarianceSums<M> r;
+                    r.row(c, a, moments, K, W, H, px, py, k - 3);
+                    if ((k & 1) == 0) {
+                        hold = r;
+                        continue;
+                    }
+                    hold.add(r);
+                    if (k == 1) v = hold;
+                    if (k == 3) v.add(hold);
+                    if (k == 5) half = hold;
+                }
+                half.add(hold);
+                v.add(half);
+                return true;
+            });
+        return;
+    }
+    for (uint32_t k = t / 8u; k - lane / 8u < n; k += blockDim.x * blockDim.y / 8u)  // whole warps
+        pixel(min(k, n - 1u), [&](VarianceSums<M>& v, const TapCentre& a, float K, int32_t px, int32_t py) {
+            v.row(c, a, moments, K, W, H, px, py, (int32_t)(lane & 7u) - 3);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                v.s0 += __shfl_xor_sync(full, v.s0, o);
+                v.s1 += __shfl_xor_sync(full, v.s1, o);
+                v.total += __shfl_xor_sync(full, v.total, o);
+            }
+            return k < n && (lane & 7u) == 0u;
+        });
+}
+
+template <class G, class R, class M>
+__global__ void __launch_bounds__(256, 4) svgf_variance_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
+                                                            const typename R::T* input, const typename M::T* moments,
+                                                            typename R::T* out) {
+    variance_body<G, R, M>(f, c, input, moments, out, blockIdx.x * blockDim.x + threadIdx.x,
+                           blockIdx.y * blockDim.y + threadIdx.y);
+}
+
+// A-trous: 25 taps a pixel, bound by L1 bandwidth (64 bytes a tap with f32
+// radiance) and load latency.  Per 1920x1200 pass, f32 / mixed storage, 256 / 246 us
+// before: a tap reads the guide and the feature record (one 128-bit and one
+// 256-bit load, also for f32 planes, whose five loads a tap cost 197 us with
+// all of the following), the wavelet step is a template constant so that the
+// taps of a row are immediate offsets, interior pixels test no bounds, the
+// three exponentials of a tap are one exp2 of the summed exponents with the
+// two divisors inverted once a pixel, no branch stands between the loads of
+// one tap and the next, and the 25 taps are unrolled (179 / 166 us with the
+// rows rolled): 173 / 156 us.  Two pixels a step apart per thread (30 taps
+// read instead of 50) 182 / 180; blocks of 32x4 176 us for step 1, 194-215 for
+// the others.
+//
 constexpr __device__ __host__ float wavelet_kernel(int32_t x) {
     return x == 0 ? 1.f : (x == 1 || x == -1) ? 2.f / 3.f : 1.f / 6.f;
 }
 
 // One pixel of svgf_atrous with its sums.
 struct Atrous {
-    V3 position, normal, color;
-    float rough, metal, lum;
-    float kz, kl;  // log2(e) over the plane-distance tolerance and over phi
+    TapCentre c;
+    float lum, kl;  // log2(e) over phi
     V3 sum;
     float total, v;
-    // svgf.wgsl:32-44, :99-105: the tap's weight, the exponentials of the
-    // plane distance, colour, parameter and luminance terms as one exp2 of
-    // their sum with the divisors' reciprocals taken once a pixel.
+    // svgf.wgsl:99-105: the exponentials of the geometry and luminance terms
+    // as one exp2 of their sum, the divisors' reciprocals taken once a pixel.
     // Without a branch before the sums, so that the loads of later taps issue
     // ahead of this one's arithmetic.
     __device__ __forceinline__ void tap(const TapGeometry& t, float4 smp, float kernel) {
-        const float kc = 8.f * 1.44269504f;
-        const float wn = pow64(wmax(dot(normal, xyz(t.normal)), 0.f));
-        const V3 dc = color - xyz(t.color);
-        const float d0 = rough - t.normal.w, d1 = metal - t.color.w;
-        const float geom = fabsf(dot(xyz(t.position) - position, normal)) * kz +
-                           (length(dc) + sqrtf(d0 * d0 + d1 * d1)) * kc;
+        float wn, geom;
+        const bool counts = c.weigh(t, wn, geom);
         const float w = wn * kernel * exp2f(-(geom + fabsf(luminance(xyz(smp)) - lum) * kl));
-        // background (depth >= 1), or a geometry weight of 0
-        if (t.position.w < 0.f || !(wn > 0.f) || geom > 126.f) return;
+        if (!counts) return;
         sum = sum + xyz(smp) * w;
         v += smp.w * smp.w * w * w;
         total += w;
@@ -154,15 +263,9 @@ __device__ __forceinline__ bool atrous_begin(Atrous& a, const SvgfCtx<G>& c, con
             variance += s * s * ((xx == 0 ? 2.f : 1.f) * (yy == 0 ? 2.f : 1.f));
         }
     }
-    const float log2e = 1.44269504f;
-    a.position = xyz(own.position);
-    a.normal = xyz(own.normal);
-    a.color = xyz(own.color);
-    a.rough = own.normal.w;
-    a.metal = own.color.w;
+    a.c.set(own, step);
     a.lum = luminance(xyz(c4));
-    a.kz = log2e / wmax(.0001f, own.position.w * (step * .5f));
-    a.kl = log2e / (4.f * sqrtf(variance * (1.f / 16.f)) + .0001f);
+    a.kl = 1.44269504f / (4.f * sqrtf(variance * (1.f / 16.f)) + .0001f);
     a.sum = V3{0.f, 0.f, 0.f};
     a.total = a.v = 0.f;
     return true;
@@ -229,7 +332,7 @@ static cudaError_t with_step(int step, Fn&& fn) {
 }
 
 template <class G, class R, class M>
-__global__ void __launch_bounds__(256, 5) svgf_variance_batched(const irt_frame* __restrict__ frames,
+__global__ void __launch_bounds__(256, 4) svgf_variance_batched(const irt_frame* __restrict__ frames,
                                                              const SView<G>* __restrict__ views,
                                                              const uint32_t* __restrict__ tile_start, uint32_t n) {
     const uint32_t v = svgf_find_view(tile_start, n, blockIdx.x);
@@ -272,7 +375,7 @@ static cudaError_t spatial_typed(const SvgfLaunch& L, int stage, cudaStream_t st
                                                               (const typename M::T*)L.moments_in, (T*)L.out);
     } else if (stage == 2) {
         // Blocks of 256 pixels of one row (4 passes at 1920x1200 f32: 0.72 ms; 64x2 0.77, 32x4
-        // 0.77); the variance pass is fastest in 32x8 (0.061 against 0.068 ms in 256x1).
+        // 0.77).
         dim3 block(256, 1);
         dim3 grid((f.size[0] + 255) / 256, f.size[1]);
         return with_step(L.step, [&](auto step) {
