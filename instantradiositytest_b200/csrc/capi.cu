@@ -625,11 +625,9 @@ static cudaError_t compute_guides(irt_session* s, const irt_frame* f, const irt_
     G.out = s->guide[0];
     G.out2 = s->feat;
     G.radiance_f16 = s->desc.radiance_format == IRT_RADIANCE_F16;
-    // positions and edge-stopping features
+    // positions and edge-stopping features, and the previous pixels' positions
+    G.old_guide_out = s->guide[1];
     cudaError_t e = irt_launch_svgf(G, 6, st);
-    if (e != cudaSuccess) return e;
-    G.out = s->guide[1];
-    e = irt_launch_svgf(G, 4, st);
     if (e == cudaSuccess) s->guide_frame = f->size[2];
     return e;
 }
@@ -828,9 +826,12 @@ irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer*
         mark(s, 8, st);
     }
     // Depth/normal history for the next frame (src/renderer.rs:1951-1960).
-    CK(cudaMemcpyAsync(s->prev_depth, g->depth, s->P * 4, cudaMemcpyDeviceToDevice, st), "depth history");
-    CK(cudaMemcpyAsync(s->prev_normal, g->normal, s->P * s->normal_bytes, cudaMemcpyDeviceToDevice, st),
-       "normal history");
+    SvgfLaunch Hh{};
+    Hh.frame = f;
+    Hh.gbuffer = *g;
+    Hh.out = s->prev_depth;
+    Hh.out2 = s->prev_normal;
+    CK(irt_launch_svgf(Hh, 5, st), "depth and normal history");
     mark(s, 9, st);
     return IRT_OK;
 }

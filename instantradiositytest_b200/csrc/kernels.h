@@ -21,6 +21,39 @@ struct FieldFilter {
 };
 }  // namespace irtd
 
+// Launch of a frame's kernel behind the one before it in its stream
+// (programmatic dependent launch): its blocks may become resident once every
+// block of that kernel has started its work, and wait_for_previous() at the
+// kernel's start holds them until that kernel has completed and its writes are
+// visible; after it, let_next_start() opens the same to the next one.  Every
+// kernel launched so calls both, in this order, before it touches memory the
+// frame writes, so a kernel's completion implies that of all before it.  What
+// is saved is the launch and ramp-up between kernels.
+template <class... P, class... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+namespace irtd {
+__device__ __forceinline__ void wait_for_previous() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void frame_kernel_begin() {
+    wait_for_previous();
+    let_next_start();
+}
+}  // namespace irtd
+#endif
+
 // Lighting stages: 0..7 are the reference entry points in schedule order
 // (candidates_direct, candidates_indirect, temporal_direct, temporal_indirect,
 // spatial_direct, spatial_indirect, resolve_direct, resolve_indirect).
@@ -167,11 +200,13 @@ struct SvgfLaunch {
     const float4* guide;      // per-pixel positions of this frame (or null)
     const float4* old_guide;  // ... of the previous frame (or null)
     const float4* feat;       // per-pixel edge-stopping features (or null)
+    float4* old_guide_out;    // stage 6: also the guide of the previous frame's pixels (or null)
 };
-// irt_launch_svgf stages: 0 temporal, 1 variance, 2 a-trous, 3 position guide
-// of this frame (out = float4[W*H]), 4 guide of the previous frame (from
-// old_depth and previous_inv_vp), 6 guide of this frame (out) and its
-// edge-stopping features (out2 = float4[2*W*H]).
+// irt_launch_svgf stages: 0 temporal, 1 variance, 2 a-trous, 5 depth and
+// normal history (out = previous depth, out2 = previous normal), 6 position
+// guide of this frame (out = float4[W*H]) and its edge-stopping features (out2 =
+// float4[2*W*H]), and with old_guide_out the guide of the previous frame's
+// pixels from old_depth and previous_inv_vp.
 
 // VPL paths of one frame (vplgen.cu): lights on the device, ray casts
 // against a workload's primitive table.

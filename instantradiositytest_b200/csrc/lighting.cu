@@ -342,6 +342,7 @@ __device__ __forceinline__ void reuse_body(const irt_frame& f, const LightArgs<G
 template <class G>
 __global__ void __launch_bounds__(256, 4) reuse_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ LightArgs<G> a,
                                                     int keep_candidates) {
+    frame_kernel_begin();
     reuse_body<G>(f, a, keep_candidates, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
 
@@ -429,6 +430,7 @@ __device__ __forceinline__ void spatial_prep_body(const irt_frame& f, const Ligh
 template <class G, class R>
 __global__ void __launch_bounds__(256, 4) spatial_prep_kernel(const __grid_constant__ irt_frame f,
                                                            const __grid_constant__ LightArgs<G> a) {
+    frame_kernel_begin();
     spatial_prep_body<G, R>(f, a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
 
@@ -451,6 +453,7 @@ __device__ __forceinline__ void combine_body(const irt_frame& f, const float4* p
 template <class R>
 __global__ void __launch_bounds__(256) combine_kernel(const __grid_constant__ irt_frame f, const float4* pending,
                                                       const float* vis, float4* direct_out, void* noisy_out) {
+    frame_kernel_begin();
     combine_body<R>(f, pending, vis, direct_out, noisy_out, (size_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -612,13 +615,14 @@ static cudaError_t launch_typed(const LightingLaunch& L, int stage, cudaStream_t
     dim3 block(32, 8);
     dim3 grid((f.size[0] + 31) / 32, (f.size[1] + 7) / 8);
     switch (stage) {
-    case kStageReuse: reuse_kernel<G><<<grid, block, 0, st>>>(f, a, L.keep_candidates); break;
+    case kStageReuse: return launch_behind(reuse_kernel<G>, grid, block, 0, st, f, a, L.keep_candidates);
     case kStageShade: shade_kernel<G, R><<<grid, block, 0, st>>>(f, a); break;
-    case kStageSpatial: spatial_prep_kernel<G, R><<<grid, block, 0, st>>>(f, a); break;
+    case kStageSpatial: return launch_behind(spatial_prep_kernel<G, R>, grid, block, 0, st, f, a);
     case kStageCombine: {
         size_t P = (size_t)f.size[0] * f.size[1];
-        combine_kernel<R><<<(unsigned)((P + 255) / 256), 256, 0, st>>>(f, L.pending, L.vis, L.direct_out, L.noisy_out);
-    } break;
+        return launch_behind(combine_kernel<R>, dim3((unsigned)((P + 255) / 256)), dim3(256), 0, st, f, L.pending, L.vis,
+                             L.direct_out, L.noisy_out);
+    }
     case 0: pass_kernel<G, R, 0><<<grid, block, 0, st>>>(f, a); break;
     case 1: pass_kernel<G, R, 1><<<grid, block, 0, st>>>(f, a); break;
     case 2: pass_kernel<G, R, 2><<<grid, block, 0, st>>>(f, a); break;

@@ -505,6 +505,7 @@ __device__ __forceinline__ void assume_sampler(DevScene& sc) {
 // instructions run for several lanes at once: 1 lane 2.49 ms, 3 or 6 lanes
 // 2.43, 10 lanes 2.49, 16 lanes 2.68 (set-up and march at 1920x1200).
 constexpr int kRefill = 6;
+constexpr uint32_t kMinLanes = 4;
 
 __global__ void __launch_bounds__(kMarchThreads) ray_pools_kernel(const __grid_constant__ irt_frame f, const DevScene sc,
                                                                   const float4* __restrict__ march_scene,
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(kMarchThreads) ray_pools_kernel(const __grid_c
                                                                   const __grid_constant__ RaySetup setup) {
     extern __shared__ float4 smem[];
     for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
+    frame_kernel_begin();  // the records above are not the frame's to write
     __syncthreads();
     const SceneRefs R = scene_refs(f, smem);
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -527,6 +529,7 @@ __global__ void __launch_bounds__(kSetupThreads, 2) ray_setup_kernel(const __gri
     extern __shared__ float4 smem[];
     __shared__ SetupShared sh;
     for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
+    frame_kernel_begin();  // the records above are not the frame's to write
     __syncthreads();
     const SceneRefs R = scene_refs(f, smem);
     const uint32_t W = f.size[0], H = f.size[1];
@@ -540,6 +543,7 @@ __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) march_kernel(c
                                                     const Grid grid, const __grid_constant__ RaySetup setup) {
     extern __shared__ float4 smem[];
     for (uint32_t i = threadIdx.x; i < scene_vec4; i += blockDim.x) smem[i] = __ldg(march_scene + i);
+    frame_kernel_begin();  // the records above are not the frame's to write
     __syncthreads();
     assume_sampler<S>(sc);
     const SceneRefs R = scene_refs(f, smem);
@@ -549,19 +553,26 @@ __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm) march_kernel(c
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
 
+    // A queue shorter than the grid's lanes is spread over its warps, a few
+    // lanes each: a step then runs fewer lanes' ways (160x100: 32 000 rays).
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    const uint32_t lanes = min(max((n_rays + warps - 1u) / warps, kMinLanes), 32u);
+    const unsigned mine = lanes == 32u ? full : (1u << lanes) - 1u;
+    const int refill = min(kRefill, (int)lanes);
+
     bool exhausted = false;  // warp-uniform: the queue has no rays left
     Lane L;
     lane_reset(L);
     RaySlice slice{0u, 0u, false};
-    const uint32_t keep = 2u * gridDim.x * (blockDim.x / 32u) * kRayChunk;
+    const uint32_t keep = 2u * warps * kRayChunk;
     for (;;) {
-        const unsigned need = __ballot_sync(full, !L.active);
+        const unsigned idle = __ballot_sync(full, !L.active), need = idle & mine;
         if (exhausted) {
-            if (need == full) break;
-        } else if (__popc(need) >= kRefill) {
+            if (idle == full) break;
+        } else if (__popc(need) >= refill) {
             const uint32_t idx = slice_take(slice, need, &setup.counters[1], n_rays, keep, lane, setup.rays, front, cap);
             exhausted = slice.drained && slice.next >= slice.end;
-            if (!L.active && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap))
+            if ((need >> lane & 1u) && idx < n_rays && index_ok(sc.error, ray_slot(idx, front, cap), cap))
                 lane_take(L, setup, ray_slot(idx, front, cap), R);
         }
         lane_step(L, sc, grid, R, f.sdf[2], setup.vis, cap);
@@ -779,9 +790,8 @@ cudaError_t IRT_MARCH_FN(irt_launch_ray_pools)(const MarchLaunch& M, cudaStream_
     if (e != cudaSuccess) return e;
     const uint32_t entries = (M.setup.slots + 2u) * M.setup.vpl_count;
     const uint32_t blocks = std::min((uint32_t)M.num_sms, (entries + kMarchThreads - 1) / kMarchThreads);
-    ray_pools_kernel<<<blocks, kMarchThreads, smem, st>>>(*M.frame, launch_scene(M), M.march_scene, smem / 16,
-                                                          launch_grid(M), M.setup);
-    return cudaGetLastError();
+    return launch_behind(ray_pools_kernel, dim3(blocks), dim3(kMarchThreads), smem, st, *M.frame, launch_scene(M),
+                         M.march_scene, smem / 16, launch_grid(M), M.setup);
 }
 
 cudaError_t IRT_MARCH_FN(irt_launch_march)(const MarchLaunch& M, cudaStream_t st) {
@@ -797,11 +807,11 @@ cudaError_t IRT_MARCH_FN(irt_launch_march)(const MarchLaunch& M, cudaStream_t st
     if (e != cudaSuccess) return e;
     const irtd::DevScene sc = launch_scene(M);
     const Grid g = launch_grid(M);
-    ray_setup_kernel<<<M.num_sms * set_up.per_sm, kSetupThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
-                                                                             M.setup);
-    kernels[sampler]<<<M.num_sms * march.per_sm, kMarchThreads, smem, st>>>(*M.frame, sc, M.march_scene, smem / 16, g,
-                                                                            M.setup);
-    return cudaGetLastError();
+    e = launch_behind(ray_setup_kernel, dim3(M.num_sms * set_up.per_sm), dim3(kSetupThreads), smem, st, *M.frame, sc,
+                      M.march_scene, smem / 16, g, M.setup);
+    if (e != cudaSuccess) return e;
+    return launch_behind(kernels[sampler], dim3(M.num_sms * march.per_sm), dim3(kMarchThreads), smem, st, *M.frame, sc,
+                         M.march_scene, smem / 16, g, M.setup);
 }
 
 cudaError_t IRT_MARCH_FN(irt_launch_ray_pools_batched)(const MarchBatch& M, cudaStream_t st) {

@@ -197,6 +197,7 @@ template <class G, class R, class M>
 __global__ void __launch_bounds__(256, 4) svgf_variance_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
                                                             const typename R::T* input, const typename M::T* moments,
                                                             typename R::T* out) {
+    frame_kernel_begin();
     variance_body<G, R, M>(f, c, input, moments, out, blockIdx.x * blockDim.x + threadIdx.x,
                            blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -313,6 +314,7 @@ template <class G, class R, int32_t Step>
 __global__ void __launch_bounds__(256, 4) svgf_atrous_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
                                                           const typename R::T* __restrict__ input, typename R::T* __restrict__ out,
                                                           typename R::T* __restrict__ out2) {
+    frame_kernel_begin();
     atrous_body<G, R, Step>(f, c, input, out, out2, blockIdx.x * blockDim.x + threadIdx.x,
                             blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -321,14 +323,13 @@ __global__ void __launch_bounds__(256, 4) svgf_atrous_kernel(const __grid_consta
 template <class Fn>
 static cudaError_t with_step(int step, Fn&& fn) {
     switch (step) {
-    case 1: fn(std::integral_constant<int32_t, 1>{}); break;
-    case 2: fn(std::integral_constant<int32_t, 2>{}); break;
-    case 4: fn(std::integral_constant<int32_t, 4>{}); break;
-    case 8: fn(std::integral_constant<int32_t, 8>{}); break;
-    case 16: fn(std::integral_constant<int32_t, 16>{}); break;
-    default: return cudaErrorInvalidValue;
+    case 1: return fn(std::integral_constant<int32_t, 1>{});
+    case 2: return fn(std::integral_constant<int32_t, 2>{});
+    case 4: return fn(std::integral_constant<int32_t, 4>{});
+    case 8: return fn(std::integral_constant<int32_t, 8>{});
+    case 16: return fn(std::integral_constant<int32_t, 16>{});
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <class G, class R, class M>
@@ -371,16 +372,16 @@ static cudaError_t spatial_typed(const SvgfLaunch& L, int stage, cudaStream_t st
     if (stage == 1) {
         dim3 block(32, 8);
         dim3 grid((f.size[0] + 31) / 32, (f.size[1] + 7) / 8);
-        svgf_variance_kernel<G, R, M><<<grid, block, 0, st>>>(f, c, (const T*)L.in,
-                                                              (const typename M::T*)L.moments_in, (T*)L.out);
+        return launch_behind(svgf_variance_kernel<G, R, M>, grid, block, 0, st, f, c, (const T*)L.in,
+                             (const typename M::T*)L.moments_in, (T*)L.out);
     } else if (stage == 2) {
         // Blocks of 256 pixels of one row (4 passes at 1920x1200 f32: 0.72 ms; 64x2 0.77, 32x4
         // 0.77).
         dim3 block(256, 1);
         dim3 grid((f.size[0] + 255) / 256, f.size[1]);
         return with_step(L.step, [&](auto step) {
-            svgf_atrous_kernel<G, R, decltype(step)::value><<<grid, block, 0, st>>>(f, c, (const T*)L.in, (T*)L.out,
-                                                                                   (T*)L.out2);
+            return launch_behind(svgf_atrous_kernel<G, R, decltype(step)::value>, grid, block, 0, st, f, c,
+                                 (const T*)L.in, (T*)L.out, (T*)L.out2);
         });
     } else {
         return cudaErrorInvalidValue;
@@ -398,6 +399,7 @@ static cudaError_t spatial_batched_typed(const BatchLaunch& B, int stage, cudaSt
         return with_step(B.step, [&](auto step) {
             svgf_atrous_batched<G, R, decltype(step)::value><<<B.tiles, block, 0, st>>>(B.frames, views, B.tile_start,
                                                                                        B.n);
+            return cudaGetLastError();
         });
     else
         return cudaErrorInvalidValue;
