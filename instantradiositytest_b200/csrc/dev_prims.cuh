@@ -88,84 +88,111 @@ __device__ __forceinline__ bool cast_tris(const irt::TriNode* nodes, const irt::
     return true;
 }
 
-// Nearest hit t in (tmin, tmax) along o + t d over all primitives: front
-// entries of boxes (slab test; an origin inside a box is no hit) and spheres
-// (nearest root), and triangle hierarchies (back faces skipped when `cull`).
-// Returns the primitive index or -1, with t and the object-space normal in
-// nl (the entered face, or the interpolated vertex normal of a triangle).
-__device__ __forceinline__ int cast_prims(const irt::PrimTable& T, const float o[3], const float d[3], float tmin,
-                                          float tmax, bool cull, float& t_out, float nl[3]) {
-    const irt::GPrim* prims = T.prims;
+// One primitive's hit before `best`, as cast_prims takes it: updates best and
+// the object-space normal nl and returns true.
+__device__ __forceinline__ bool cast_prim(const irt::PrimTable& T, const irt::GPrim& p, const float o[3],
+                                          const float d[3], float tmin, bool cull, float& best, float nl[3]) {
+    float lo4[4], ld4[4];
+    xf4(p.inv_model, o[0], o[1], o[2], 1.f, lo4);
+    xf4(p.inv_model, d[0], d[1], d[2], 0.f, ld4);
+    float t = 0.f;
+    float nn[3] = {0, 0, 0};
+    bool h = false;
+    if (p.kind == irt::kPrimTriangles) {
+        const float inv[3] = {1.f / ld4[0], 1.f / ld4[1], 1.f / ld4[2]};
+        return slab(p.lo, p.hi, lo4, inv, tmin, best) &&
+               cast_tris(T.nodes + p.node_base, T.tris + p.tri_base, lo4, ld4, tmin, cull, best, nl);
+    }
+    if (p.kind == irt::kPrimSphere) {
+        float r = p.lo[0];
+        float b = lo4[0] * ld4[0] + lo4[1] * ld4[1] + lo4[2] * ld4[2];
+        float a = ld4[0] * ld4[0] + ld4[1] * ld4[1] + ld4[2] * ld4[2];
+        float c = lo4[0] * lo4[0] + lo4[1] * lo4[1] + lo4[2] * lo4[2] - r * r;
+        float disc = b * b - a * c;
+        if (disc >= 0.f) {
+            t = (-b - sqrtf(disc)) / a;
+            if (t >= tmin && t < best) {
+                h = true;
+                for (int q = 0; q < 3; q++) nn[q] = (lo4[q] + ld4[q] * t) / r;
+            }
+        }
+    } else {
+        float t0 = tmin, t1 = best;
+        int axis = -1;
+        float sign = 0.f;
+        bool miss = false;
+        for (int a = 0; a < 3 && !miss; a++) {
+            float inv = 1.f / ld4[a];
+            float ta = (p.lo[a] - lo4[a]) * inv, tb = (p.hi[a] - lo4[a]) * inv;
+            float s = -1.f;
+            if (ta > tb) {
+                float tmp = ta;
+                ta = tb;
+                tb = tmp;
+                s = 1.f;
+            }
+            if (ta > t0) {
+                t0 = ta;
+                axis = a;
+                sign = s;
+            }
+            t1 = fminf(t1, tb);
+            if (t0 > t1) miss = true;
+        }
+        if (!miss && axis >= 0 && t0 < best) {
+            h = true;
+            t = t0;
+            nn[axis] = sign;
+        }
+    }
+    if (!h) return false;
+    best = t;
+    nl[0] = nn[0];
+    nl[1] = nn[1];
+    nl[2] = nn[2];
+    return true;
+}
+
+// Nearest hit t in (tmin, tmax) along o + t d over the primitives that `at`
+// names (n of them, ascending): front entries of boxes (slab test; an origin
+// inside a box is no hit) and spheres (nearest root), and triangle hierarchies
+// (back faces skipped when `cull`).  Returns the primitive index or -1, with t
+// and the object-space normal in nl (the entered face, or the interpolated
+// vertex normal of a triangle).
+template <class At>
+__device__ __forceinline__ int cast_prims(const irt::PrimTable& T, uint32_t n, At&& at, const float o[3],
+                                          const float d[3], float tmin, float tmax, bool cull, float& t_out,
+                                          float nl[3]) {
     float best = tmax;
     int hit = -1;
-    for (uint32_t k = 0; k < T.n; k++) {
-        const irt::GPrim& p = prims[k];
-        float lo4[4], ld4[4];
-        xf4(p.inv_model, o[0], o[1], o[2], 1.f, lo4);
-        xf4(p.inv_model, d[0], d[1], d[2], 0.f, ld4);
-        float t = 0.f;
-        float nn[3] = {0, 0, 0};
-        bool h = false;
-        if (p.kind == irt::kPrimTriangles) {
-            const float inv[3] = {1.f / ld4[0], 1.f / ld4[1], 1.f / ld4[2]};
-            if (slab(p.lo, p.hi, lo4, inv, tmin, best) &&
-                cast_tris(T.nodes + p.node_base, T.tris + p.tri_base, lo4, ld4, tmin, cull, best, nl)) {
-                hit = (int)k;
-            }
-            continue;
-        }
-        if (p.kind == irt::kPrimSphere) {
-            float r = p.lo[0];
-            float b = lo4[0] * ld4[0] + lo4[1] * ld4[1] + lo4[2] * ld4[2];
-            float a = ld4[0] * ld4[0] + ld4[1] * ld4[1] + ld4[2] * ld4[2];
-            float c = lo4[0] * lo4[0] + lo4[1] * lo4[1] + lo4[2] * lo4[2] - r * r;
-            float disc = b * b - a * c;
-            if (disc >= 0.f) {
-                t = (-b - sqrtf(disc)) / a;
-                if (t >= tmin && t < best) {
-                    h = true;
-                    for (int q = 0; q < 3; q++) nn[q] = (lo4[q] + ld4[q] * t) / r;
-                }
-            }
-        } else {
-            float t0 = tmin, t1 = best;
-            int axis = -1;
-            float sign = 0.f;
-            bool miss = false;
-            for (int a = 0; a < 3 && !miss; a++) {
-                float inv = 1.f / ld4[a];
-                float ta = (p.lo[a] - lo4[a]) * inv, tb = (p.hi[a] - lo4[a]) * inv;
-                float s = -1.f;
-                if (ta > tb) {
-                    float tmp = ta;
-                    ta = tb;
-                    tb = tmp;
-                    s = 1.f;
-                }
-                if (ta > t0) {
-                    t0 = ta;
-                    axis = a;
-                    sign = s;
-                }
-                t1 = fminf(t1, tb);
-                if (t0 > t1) miss = true;
-            }
-            if (!miss && axis >= 0 && t0 < best) {
-                h = true;
-                t = t0;
-                nn[axis] = sign;
-            }
-        }
-        if (h) {
-            best = t;
-            hit = (int)k;
-            nl[0] = nn[0];
-            nl[1] = nn[1];
-            nl[2] = nn[2];
-        }
+    for (uint32_t j = 0; j < n; j++) {
+        const uint32_t k = at(j);
+        if (cast_prim(T, T.prims[k], o, d, tmin, cull, best, nl)) hit = (int)k;
     }
     t_out = best;
     return hit;
+}
+
+// The same hit found by a warp, every lane with the same ray: the lanes take
+// the primitives in turn and the nearest hit wins, the lowest index among
+// equals, as in the sequence (whether a primitive counts depends on the best
+// so far, its t does not).
+__device__ __forceinline__ int cast_prims_warp(const irt::PrimTable& T, const float o[3], const float d[3], float tmin,
+                                               float tmax, bool cull, float& t_out, float nl[3]) {
+    const unsigned full = 0xffffffffu;
+    float best = tmax;
+    uint32_t hit = 0xffffffffu;
+    for (uint32_t k = threadIdx.x & 31u; k < T.n; k += 32u)
+        if (cast_prim(T, T.prims[k], o, d, tmin, cull, best, nl)) hit = k;
+    float nearest = hit != 0xffffffffu ? best : tmax;
+#pragma unroll
+    for (int x = 16; x > 0; x >>= 1) nearest = fminf(nearest, __shfl_xor_sync(full, nearest, x));
+    const uint32_t k = __reduce_min_sync(full, hit != 0xffffffffu && best == nearest ? hit : 0xffffffffu);
+    t_out = nearest;
+    if (k == 0xffffffffu) return -1;
+    const int from = (int)(k & 31u);
+    for (int a = 0; a < 3; a++) nl[a] = __shfl_sync(full, nl[a], from);
+    return (int)k;
 }
 
 }  // namespace irtd

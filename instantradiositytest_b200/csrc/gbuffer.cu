@@ -36,24 +36,119 @@ __device__ __forceinline__ uint32_t oct_snorm16(float x, float y, float z) {
     return ((uint32_t)(uint16_t)(int16_t)qu) | ((uint32_t)(uint16_t)(int16_t)qv << 16);
 }
 
+// Ray of the image point (u, v): d spans near to far plane, t in [0, 1).
+__device__ __forceinline__ void primary_ray(const irt_frame& f, float u, float v, float o[3], float d[3]) {
+    float nx = u * 2.f - 1.f, ny = 1.f - v * 2.f;
+    float pn[4], pf[4];
+    xf(f.inv_vp.m, nx, ny, 0.f, 1.f, pn);
+    xf(f.inv_vp.m, nx, ny, 1.f, 1.f, pf);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        o[a] = pn[a] / pn[3];
+        d[a] = pf[a] / pf[3] - o[a];
+    }
+}
+
+// Primitives a block of pixels may see, in ascending order: those whose
+// bounding sphere is not wholly beyond one of the four planes through the
+// block's corner rays, by a margin well above the f32 error of the rays (a
+// far plane's corner is good to about 1e-4 of its distance).  Every pixel of
+// the block tests the same few primitives instead of all: 1280x720, 23
+// objects 97 -> 57 us, 2560x1600, 50 objects 816 -> 300.
+constexpr uint32_t kMaxListed = 2048;
+struct BlockPrims {
+    float corner_o[4][3], corner_d[4][3];
+    uint32_t count;
+    uint16_t index[kMaxListed];
+};
+__device__ __forceinline__ bool beyond(const BlockPrims& s, const GPrim& p) {
+    // bounding sphere in world space: the model's largest stretch is at most
+    // sqrt of the largest row sum of |A^T A|
+    float m[3], half;
+    if (p.kind == irt::kPrimSphere) {
+        m[0] = m[1] = m[2] = 0.f;
+        half = p.lo[0];
+    } else {
+        float h2 = 0.f;
+        for (int a = 0; a < 3; a++) {
+            m[a] = .5f * (p.lo[a] + p.hi[a]);
+            const float h = .5f * (p.hi[a] - p.lo[a]);
+            h2 += h * h;
+        }
+        half = sqrtf(h2);
+    }
+    float c[4];
+    xf(p.model, m[0], m[1], m[2], 1.f, c);
+    float stretch = 0.f;
+    for (int a = 0; a < 3; a++) {
+        float row = 0.f;
+        for (int b = 0; b < 3; b++) {
+            float dot = 0.f;
+            for (int k = 0; k < 3; k++) dot += p.model[4 * a + k] * p.model[4 * b + k];
+            row += fabsf(dot);
+        }
+        stretch = fmaxf(stretch, row);
+    }
+    const float r = half * sqrtf(stretch);
+    float centre[3];
+    for (int a = 0; a < 3; a++)
+        centre[a] = s.corner_d[0][a] + s.corner_d[1][a] + s.corner_d[2][a] + s.corner_d[3][a];
+    for (int k = 0; k < 4; k++) {
+        const float *da = s.corner_d[k], *db = s.corner_d[(k + 1) & 3], *o = s.corner_o[k];
+        float n[3] = {da[1] * db[2] - da[2] * db[1], da[2] * db[0] - da[0] * db[2], da[0] * db[1] - da[1] * db[0]};
+        const float len = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+        float side = n[0] * centre[0] + n[1] * centre[1] + n[2] * centre[2];
+        if (side < 0.f) {
+            n[0] = -n[0];
+            n[1] = -n[1];
+            n[2] = -n[2];
+        }
+        const float w[3] = {c[0] - o[0], c[1] - o[1], c[2] - o[2]};
+        const float away = sqrtf(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+        // parallel corner rays (len 0) and anything not a number keep the primitive
+        if (n[0] * w[0] + n[1] * w[1] + n[2] * w[2] < -len * (1.01f * r + .02f * away + 1e-3f)) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void list_block_prims(const irt_frame& f, const irt::PrimTable& T, BlockPrims& s) {
+    const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x;
+    if (t < 4u) {  // the corners of the block's pixels, in a cycle
+        const float W = (float)f.size[0], H = (float)f.size[1];
+        const float x = (float)((blockIdx.x + (t == 1u || t == 2u ? 1u : 0u)) * blockDim.x);
+        const float y = (float)((blockIdx.y + (t >= 2u ? 1u : 0u)) * blockDim.y);
+        primary_ray(f, fminf(x, W) / W, fminf(y, H) / H, s.corner_o[t], s.corner_d[t]);
+    }
+    __syncthreads();
+    if (t < 32u) {
+        uint32_t count = 0;
+        for (uint32_t first = 0; first < T.n; first += 32u) {
+            const bool keep = first + t < T.n && !beyond(s, T.prims[first + t]);
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (keep) s.index[count + __popc(kept & ((1u << t) - 1u))] = (uint16_t)(first + t);
+            count += (uint32_t)__popc(kept);
+        }
+        if (t == 0u) s.count = count;
+    }
+    __syncthreads();
+}
+
 __global__ void gbuffer_kernel(const __grid_constant__ irt_frame f, const irt::PrimTable T, int fmt,
                                float* depth, void* normal, void* color, void* params, void* motion) {
+    __shared__ BlockPrims listed;
+    const bool list = T.n <= kMaxListed;
+    if (list) list_block_prims(f, T, listed);
     uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
     uint32_t W = f.size[0], H = f.size[1];
     if (x >= W || y >= H) return;
     size_t i = (size_t)y * W + x;
     float u = ((float)x + .5f) / (float)W, v = ((float)y + .5f) / (float)H;
-    float nx = u * 2.f - 1.f, ny = 1.f - v * 2.f;
-    float pn[4], pf[4];
-    xf(f.inv_vp.m, nx, ny, 0.f, 1.f, pn);
-    xf(f.inv_vp.m, nx, ny, 1.f, 1.f, pf);
-    float o[3] = {pn[0] / pn[3], pn[1] / pn[3], pn[2] / pn[3]};
-    float d[3] = {pf[0] / pf[3] - o[0], pf[1] / pf[3] - o[1], pf[2] / pf[3] - o[2]};
-    // d spans near to far plane: t in [0, 1).
+    float o[3], d[3];
+    primary_ray(f, u, v, o, d);
     float best;
     float nl_best[3] = {0, 0, 0};
-    int hit = irtd::cast_prims(T, o, d, 0.f, 1.f, true, best, nl_best);
+    int hit = irtd::cast_prims(T, list ? listed.count : T.n, [&](uint32_t j) { return list ? (uint32_t)listed.index[j] : j; },
+                               o, d, 0.f, 1.f, true, best, nl_best);
     float dep = 1.f, nrm[3] = {0, 0, 0}, col[3] = {0, 0, 0}, par[2] = {0, 0}, mot[2] = {0, 0};
     if (hit >= 0) {
         const GPrim& p = T.prims[hit];
