@@ -114,7 +114,9 @@ cudaError_t upload(T** dst, const void* src, size_t bytes) {
         cudaError_t e = cudaMalloc(dst, bytes);
         if (e != cudaSuccess) return e;
     }
-    return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+    // the batch's stream does not wait for the default one
+    return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
 }
 
 void free_tables(ParityTables& t) {

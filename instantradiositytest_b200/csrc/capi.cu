@@ -155,6 +155,9 @@ irt_status irt_scene_create(irt_context* ctx, const irt_mesh* meshes, uint32_t m
             if (e != cudaSuccess) return fail(cuda_fail(ctx, e, "mesh upload"));
         }
     }
+    // Uploads from pageable memory may still be on their way to the device.
+    e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) return fail(cuda_fail(ctx, e, "scene upload"));
     ctx->in_use += sc->bytes;
     *out = sc;
     return IRT_OK;

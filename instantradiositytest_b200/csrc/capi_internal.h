@@ -205,7 +205,14 @@ irt_status dev_alloc(irt_context* ctx, T** p, size_t bytes, uint64_t& counter) {
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, bytes);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
-    e = cudaMemset(q, 0, bytes);
+    // Zeroed when this returns: a fill left on the default stream is not
+    // ordered with work that a caller's non-blocking stream does next and
+    // could wipe what it has written.
+    cudaStream_t fill = nullptr;
+    e = cudaStreamCreateWithFlags(&fill, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(q, 0, bytes, fill);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(fill);
+    if (fill) cudaStreamDestroy(fill);
     if (e != cudaSuccess) {
         cudaFree(q);
         return cuda_fail(ctx, e, "cudaMemset");

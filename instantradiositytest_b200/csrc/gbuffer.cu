@@ -275,7 +275,9 @@ cudaError_t irt_workload_prims(const irt_workload* wl_c, irt::PrimTable* out) {
             if (bytes == 0) return cudaSuccess;
             cudaError_t r = cudaMalloc(dst, bytes);
             if (r != cudaSuccess) return r;
-            return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+            r = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+            // a caller's non-blocking stream does not wait for the default one
+            return r == cudaSuccess ? cudaStreamSynchronize(nullptr) : r;
         };
         e = upload(&w.dev_prims, prims.data(), prims.size() * sizeof(GPrim));
         if (e == cudaSuccess) e = upload(&w.dev_nodes, nodes.data(), nodes.size() * sizeof(irt::TriNode));
