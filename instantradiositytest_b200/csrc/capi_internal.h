@@ -44,19 +44,19 @@ struct irt_scene {
     // cell index is in hi[3] of its rows (host_meshes and the device copy).
     void* sdf_cells = nullptr;
     std::vector<irt_mesh> host_meshes;
-    // per-frame data
+    // per-frame data: one device block, holding every buffer below up to `cells`
+    char* block = nullptr;
+    uint64_t block_bytes = 0;
     irt_object* objects = nullptr;
     irt_node* nodes = nullptr;
     irt_light* lights = nullptr;
     irt_light* lights_prep = nullptr;  // spot direction normalised, cos(angle / 2)
     uint32_t object_cap = 0, light_cap = 0;
-    // compact march scene (nodes + object records with their mesh folded in)
+    // compact march scene (object records with their mesh and leaf box folded in)
     float4* march_scene = nullptr;
-    std::vector<float4> march_host;
     // Pinned staging of the per-frame uploads, two slots used in turn, so an
     // update neither waits for the device nor races an earlier copy.
-    unsigned char* pinned[2] = {nullptr, nullptr};
-    size_t pinned_cap[2] = {0, 0};
+    unsigned char* pinned = nullptr;
     cudaEvent_t pinned_free[2] = {nullptr, nullptr};
     uint32_t updates = 0;
     // leaf-order cache (rebuilt when the BVH changes)
@@ -85,6 +85,7 @@ struct irt_session {
     uint32_t W = 0, H = 0;
     size_t P = 0;
     size_t rad_bytes = 0, normal_bytes = 0, mom_bytes = 0;
+    char* slab = nullptr;  // the session's device memory, holding every buffer below
     irt_reservoir* dres[3] = {nullptr, nullptr, nullptr};
     irt_reservoir* ires[3] = {nullptr, nullptr, nullptr};
     irt_vpl* archive = nullptr;
