@@ -3,7 +3,8 @@ IEEE march (which visits a cell's objects in the cache's order and stops at
 its bounds) equals the per-entry-point schedule (which walks the hierarchy)
 bit for bit — with fewer objects than a cell's 8 entries, with more, above
 the 256 objects up to which bounds are object distances, for f16 fields and
-the filtered sampler, and with objects that move."""
+the filtered sampler, with objects that move, and far from the origin, where
+the f32 error of positions and distances is hundreds of times larger."""
 import ctypes as C
 import math
 
@@ -44,12 +45,33 @@ def moved(objects, k):
     return out
 
 
+def shift(f, objects, lights, by):
+    """The same frame with the world moved: vp' = vp T(-by), inverse T(by) inv."""
+    t = np.eye(4)
+    t[:3, 3] = by
+    for vp, inv in (("vp", "inv_vp"), ("previous_vp", "previous_inv_vp")):
+        m = np.array(getattr(f, vp).m, np.float64).reshape(4, 4).T @ np.linalg.inv(t)
+        n = t @ np.array(getattr(f, inv).m, np.float64).reshape(4, 4).T
+        getattr(f, vp).m[:] = m.T.reshape(16).astype(np.float32).tolist()
+        getattr(f, inv).m[:] = n.T.reshape(16).astype(np.float32).tolist()
+    for a in range(3):
+        f.camera[a] += by[a]
+    objects, lights = objects.copy(), lights.copy()
+    for o in objects:
+        m = t @ o["model"].reshape(4, 4).T.astype(np.float64)
+        o["model"] = o["previous"] = m.T.reshape(16)
+        o["inverse"] = np.linalg.inv(m).T.reshape(16)
+    lights["position_strength"][:, :3] += np.float32(by)
+    return objects, lights
+
+
 CASES = {
     "few": dict(n_boxes=1, n_spheres=1),
     "room": dict(n_boxes=9, n_spheres=6, sdf_resolution=32),
     "f16": dict(n_boxes=9, n_spheres=6, sdf_resolution=24, sdf_format=L.SDF_F16),
     "linear": dict(n_boxes=9, n_spheres=6, sdf_resolution=24),
     "moving": dict(n_boxes=9, n_spheres=6, sdf_resolution=24),
+    "far": dict(n_boxes=9, n_spheres=6, sdf_resolution=24),
     "many": dict(n_boxes=200, n_spheres=90, sdf_resolution=12),
 }
 
@@ -70,13 +92,20 @@ def test_cached_march_equals_hierarchy_walk(cuda, name):
         if name == "moving":
             objects = moved(objects, i)
             nodes = boxes_of(objects, wl.meshes)
-        scene.update(objects, nodes, lights)
         L.check(L.lib.irt_gbuffer_render(ctx.handle, wl.handle, C.byref(f), None, L.GBUFFER_F32, g.depth, g.normal,
                                          g.color, g.params, g.motion, None), ctx.handle, "gbuffer")
+        scene.update(objects, nodes, lights)
         cur, prev = pools[i % 2], pools[(i + 1) % 2] if i else pools[2]
         L.check(L.lib.irt_vpl_generate(scene.handle, wl.handle, C.byref(f), C.c_void_p(cur.data_ptr()), None),
                 ctx.handle, "vpls")
         torch.cuda.synchronize()
+        if name == "far":
+            by = (700.0, -300.0, 200.0)
+            objects, lights = shift(f, objects, lights, by)
+            scene.update(objects, boxes_of(objects, wl.meshes), lights)
+            pool = cur.view(torch.float32).reshape(-1, 12)
+            pool[:, :3] += torch.tensor(by, device="cuda")
+            torch.cuda.synchronize()
         for s in sessions:
             s.render(scene, f, g, C.c_void_p(cur.data_ptr()), C.c_void_p(prev.data_ptr()))
         torch.cuda.synchronize()
