@@ -38,19 +38,20 @@ sys.path.insert(0, ROOT)
 # kernel that touches it; neighbour taps are cache traffic, not HBM).  With
 # G = G-buffer bytes read (depth, normal, colour, params, motion), Gs = G
 # without motion, prev = previous depth + normal, r = radiance texel,
-# m = moments texel, reservoirs 32 B, ray records 64 B:
+# m = moments texel, reservoirs 32 B, ray records 32 B with a 2 B hint:
 #   reuse   = G + prev + history reservoirs D/I 64 + reservoirs [1] written 64
 #   spatial = Gs + reservoirs [1] 64 + [2] written 64 + contributions 32
-#             + 2 ray records 128 written
-#   march   = 2 ray records 128 read + 2 visibilities 8 written       = 136
+#             + the names of the pixel's rays 20 written
+#   march   = ray set-up (position 16 + names 20 read, 2 records 68 written)
+#             + march (2 records 68 read, 2 visibilities 8 written)     = 180
 #   combine = contributions 32 + visibilities 8 + direct 16 + noisy r
 #   svgf_temporal = noisy r + G + feedback r + moments m + prev + temporal r + moments m
 #   svgf_variance = temporal r + moments m + Gs + output r
 #   atrous  = 4 x (input r + Gs + output r)
 #   history = previous depth/normal planes read + written
-# f32 storage: G = 4+12+12+8+8 = 44 -> 188, 324, 136, 72, 140, 84, 4x68, 40.
+# f32 storage: G = 4+12+12+8+8 = 44 -> 188, 216, 180, 72, 140, 84, 4x68, 40.
 # Mixed precision (packed G-buffer, f16 radiance and moments):
-#   G = 4+4+4+4+4 = 20 -> 156, 304, 136, 64, 68, 40, 4x32, 16.
+#   G = 4+4+4+4+4 = 20 -> 156, 196, 180, 64, 68, 40, 4x32, 16.
 GBUFFER_READ = {0: (4, 12, 12, 8, 8), 1: (4, 6, 6, 4, 4), 2: (4, 4, 4, 4, 4)}
 NORMAL_STORED = {0: 16, 1: 8, 2: 4}
 
@@ -62,7 +63,7 @@ def alg_bytes(gfmt, rfmt, mfmt):
     prev = d + n
     r = 8 if rfmt else 16
     m = 8 if mfmt else 16
-    return {"reuse": G + prev + 128, "spatial": Gs + 288, "march": 136, "combine": 56 + r,
+    return {"reuse": G + prev + 128, "spatial": Gs + 180, "march": 180, "combine": 56 + r,
             "svgf_temporal": 3 * r + G + 2 * m + prev, "svgf_variance": 2 * r + m + Gs, "atrous": 4 * (2 * r + Gs),
             "history": 2 * (d + NORMAL_STORED[gfmt])}
 
@@ -81,11 +82,11 @@ def storage_of(config):
 
 STAGES = ["prep", "reuse", "spatial", "march", "combine", "svgf_temporal", "svgf_variance", "atrous", "history"]
 KERNELS = ["reuse", "spatial", "march", "combine", "svgf_temporal", "svgf_variance", "atrous"]
-# Kernels launched per frame: light preparation (scene update), 2 position
-# guides, then per schedule the lighting kernels (1: reuse, spatial, march,
-# combine; 2: reuse, shade; 0: the 8 reference passes), then SVGF temporal,
-# variance and 4 a-trous.
-KERNELS_PER_FRAME = {1: 1 + 2 + 4 + 6, 2: 1 + 2 + 2 + 6, 0: 1 + 2 + 8 + 6}
+# Kernels launched per frame: light preparation (scene update), position
+# guides and features, then per schedule the lighting kernels (1: VPL pools,
+# reuse, spatial, ray set-up, march, combine; 2: reuse, shade; 0: the 8
+# reference passes), then SVGF temporal, variance, 4 a-trous and the history.
+KERNELS_PER_FRAME = {1: 1 + 1 + 6 + 7, 2: 1 + 1 + 2 + 7, 0: 1 + 1 + 8 + 7}
 # Counted FP32 work of the march per oracle work counter (flops): BVH node
 # visit (box test), certified-box distance, field distance (transform,
 # trilinear, bounds), march step (penumbra update).

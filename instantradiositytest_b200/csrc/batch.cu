@@ -4,10 +4,11 @@
 //
 // Per frame the schedule is the single-session schedule 1 of
 // irt_frame_lighting + irt_frame_svgf, each step as one batched launch:
-//   frame upload (pinned -> device table), position guides (this frame and
-//   the previous), VPL archive slot copy + ray-counter reset, reuse, spatial
-//   + ray emission, march (views grouped by scene), combine, SVGF temporal,
-//   variance, a-trous x iterations, depth/normal history copy.
+//   frame upload (pinned -> device table), position guides and features (this
+//   frame and the previous), VPL pools (archive slot, endpoints, ray-counter
+//   reset), reuse, spatial, ray set-up and march (views grouped by scene),
+//   combine, SVGF temporal, variance, a-trous x iterations, depth/normal
+//   history copy.
 // The per-view tables hold the same pointers the single-session path passes
 // as kernel parameters, so every view's results are identical to rendering
 // it alone.  Tables depend on the frame parity (SVGF ping-pong) and on the

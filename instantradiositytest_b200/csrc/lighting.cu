@@ -1,12 +1,15 @@
 // lighting.cu — the 8 lighting entry points of lighting.wgsl as sm_100a CUDA.
 //
-// Two schedules over the same per-pixel device functions:
-//   fused (default): reuse_kernel = candidates_direct + candidates_indirect +
-//     temporal_direct + temporal_indirect (writes reservoirs [1]);
-//     shade_kernel = spatial_direct + spatial_indirect + resolve_direct +
-//     resolve_indirect (writes reservoirs [2], direct and combined radiance).
+// Three schedules over the same per-pixel device functions:
+//   ray queue (default): reuse_kernel = candidates_direct + candidates_indirect
+//     + temporal_direct + temporal_indirect (writes reservoirs [1]);
+//     spatial_prep_kernel = spatial_direct + spatial_indirect (writes
+//     reservoirs [2]) and the resolve passes' contributions and rays;
+//     combine_kernel = their outputs once the march (march.cu) is done;
+//   fused: reuse_kernel, then shade_kernel = spatial and resolve passes with
+//     the march inline;
 //   plain: one kernel per reference entry point (pass_kernel<Pass>).
-// Both write bit-identical results: the fused kernels call the same device
+// All write bit-identical results: the fused kernels call the same device
 // functions in the same order and keep intermediate reservoirs in registers
 // (f32 values identical to their stored form).
 // Threads: one per pixel, 32x8 blocks (warps span 32 consecutive pixels of a
