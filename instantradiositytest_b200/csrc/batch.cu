@@ -60,6 +60,7 @@ struct ParityTables {
     void* sviews[8] = {};          // SVGF records x n: temporal, variance, a-trous 0..3, guides, previous guides
     void* history = nullptr;       // history-copy records x n
     MarchGroup* groups = nullptr;  // device, grouped by wave
+    std::vector<MarchGroup> host_groups;
     MarchQueue* queues = nullptr;  // device
     std::vector<uint32_t> wave_groups;  // groups of wave w: [wave_groups[w], wave_groups[w + 1])
     uint32_t max_scene_bytes = 0;
@@ -324,6 +325,7 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
     }
     CK(upload(&t.groups, groups.data(), groups.size() * sizeof(MarchGroup)), "batch march groups");
     CK(upload(&t.queues, queues.data(), queues.size() * sizeof(MarchQueue)), "batch march queues");
+    t.host_groups = std::move(groups);
     t.signature = signature_of(b, scenes, frames, g, cur, prev);
     t.valid = true;
     return IRT_OK;
@@ -422,6 +424,7 @@ irt_status launch_frame(irt_batch* b, int p, cudaStream_t st, const int shape_of
         MarchBatch M{};
         M.n_groups = t.wave_groups[w + 1] - t.wave_groups[w];
         M.groups = t.groups + t.wave_groups[w];
+        M.host_groups = t.host_groups.data() + t.wave_groups[w];
         M.queues = t.queues;
         M.max_scene_bytes = t.max_scene_bytes;
         M.num_sms = b->num_sms;

@@ -288,9 +288,17 @@ struct alignas(16) MarchGroup {
     float grid_org[3], grid_inv[3], grid_size[3], grid_slack;
     uint32_t q_begin, q_end;    // the group's queues in the queue table
 };
+// Groups of one march launch, its kernel parameter (a batch of more launches again).
+constexpr uint32_t kMarchGroups = 16;
+struct MarchGroups {
+    MarchGroup g[kMarchGroups];
+    uint32_t n;
+};
+static_assert(sizeof(MarchGroups) <= 32764 - sizeof(void*), "kernel parameters of sm_70 and later");
 struct MarchBatch {
     uint32_t n_groups;
     const MarchGroup* groups;   // device
+    const MarchGroup* host_groups;
     const MarchQueue* queues;   // device
     uint32_t max_scene_bytes;
     int num_sms;

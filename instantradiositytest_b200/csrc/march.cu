@@ -64,10 +64,7 @@ namespace exact {
 // Resident warps, set-up and march at 1920x1200: the single-view march at 56
 // registers in CTAs of 192 threads, 6 per SM (36 warps, no spills), 1.89 ms;
 // 4 CTAs of 256 (64 registers, 32 warps) 1.98, 5 (48 registers, spills) 2.14,
-// 6 (40 registers) 2.47, 3 (24 warps) 2.39 before the query was slimmed.  The
-// batched march, whose lanes also keep their queue, spills at 56 registers: 8
-// CTAs of 128 (64 registers) 4.36 ms over 5.2 Mpixel of views, 9 CTAs 4.75.
-constexpr int kMarchBlocksPerSm = 8;
+// 6 (40 registers) 2.47, 3 (24 warps) 2.39 before the query was slimmed.
 constexpr int kMarchThreads = 192;
 constexpr int kMarchCtasPerSm = 6;
 // Queue entries a warp reserves per atomic (one per lane): the queue counter
@@ -494,6 +491,10 @@ __device__ __forceinline__ void lane_step(Lane& L, const DevScene& sc, const Gri
 // registers and branches of one (march 1.77 -> 1.70 ms at 1920x1200 f32); a
 // batch whose scenes differ runs the one that tests per scene.
 enum Sampler : int { kPointF32 = 0, kPointF16 = 1, kLinearF32 = 2, kAnySampler = 3 };
+// CTAs of the batched march: as the single-view kernel's, but the one for any
+// sampler, which would spill at 56 registers.
+constexpr int march_threads(int sampler) { return sampler == kAnySampler ? 128 : kMarchThreads; }
+constexpr int march_ctas(int sampler) { return sampler == kAnySampler ? 8 : kMarchCtasPerSm; }
 template <int S>
 __device__ __forceinline__ void assume_sampler(DevScene& sc) {
     if (S == kPointF32 || S == kPointF16) sc.filter.linear = 0;
@@ -656,18 +657,25 @@ __global__ void __launch_bounds__(kSetupThreads, 2) ray_setup_batched_kernel(con
 }
 
 // The march over a group's queues in order; a lane keeps its queue's index.
+// The groups are a kernel parameter: a group's constants are then read where
+// they are used, as the single-view kernel reads its own.  Copies from a record
+// in shared memory lived in registers: 64 of them, 32 warps an SM; now 56 and
+// 36 warps (8 views of 5.2 Mpixel, the whole frame 9208 -> 9162 us).
 template <int S>
-__global__ void __launch_bounds__(128, kMarchBlocksPerSm) march_batched_kernel(const MarchGroup* __restrict__ groups, uint32_t n_groups,
-                                                            const MarchQueue* __restrict__ queues) {
+__global__ void __launch_bounds__(march_threads(S), march_ctas(S)) march_batched_kernel(const __grid_constant__ MarchGroups groups,
+                                                                     const MarchQueue* __restrict__ queues) {
     extern __shared__ float4 smem[];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    for (uint32_t g = 0; g < n_groups; g++) {
-        const MarchGroup& G = stage_group(groups, g, smem);
+    for (uint32_t g = 0; g < groups.n; g++) {
+        const MarchGroup& G = groups.g[g];
+        __syncthreads();  // every warp is done with the previous group's records
+        for (uint32_t i = threadIdx.x; i < G.scene_vec4; i += blockDim.x) smem[i] = __ldg(G.march_scene + i);
+        __syncthreads();
         DevScene sc = group_scene(G);
         assume_sampler<S>(sc);
         const Grid grid = group_grid(G);
-        const SceneRefs R = scene_refs(G.f, smem + kGroupVec4);
+        const SceneRefs R = scene_refs(G.f, smem);
         uint32_t q = G.q_begin;
         bool exhausted = q >= G.q_end;
         uint32_t front = exhausted ? 0u : *(volatile const uint32_t*)&queues[q].setup.counters[0];
@@ -836,12 +844,21 @@ cudaError_t IRT_MARCH_FN(irt_launch_march_batched)(const MarchBatch& M, cudaStre
     thread_local KernelFit set_up, fits[4];
     KernelFit& march = fits[M.sampler];
     cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, kSetupThreads, smem, 2);
-    if (e == cudaSuccess) e = march.set((const void*)kernels[M.sampler], 128, smem, kMarchBlocksPerSm);
+    const int threads = march_threads(M.sampler);
+    if (e == cudaSuccess)
+        e = march.set((const void*)kernels[M.sampler], threads, M.max_scene_bytes, march_ctas(M.sampler));
     if (e != cudaSuccess) return e;
     const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < march.per_sm ? M.blocks_per_sm : march.per_sm;
     ray_setup_batched_kernel<<<M.num_sms * set_up.per_sm, kSetupThreads, smem, st>>>(M.groups, M.n_groups, M.queues);
-    kernels[M.sampler]<<<M.num_sms * bps, 128, smem, st>>>(M.groups, M.n_groups, M.queues);
-    return cudaGetLastError();
+    for (uint32_t g = 0; g < M.n_groups; g += kMarchGroups) {
+        MarchGroups part;
+        part.n = std::min(M.n_groups - g, kMarchGroups);
+        std::copy_n(M.host_groups + g, part.n, part.g);
+        kernels[M.sampler]<<<M.num_sms * bps, threads, M.max_scene_bytes, st>>>(part, M.queues);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 #if !IRT_MARCH_FAST
