@@ -13,7 +13,7 @@ struct SvgfCtx {
     G g;
     const typename G::NormalT* old_normal;
     // Per-pixel world positions of this frame and the previous one, w < 0
-    // where depth >= 1 (guide_kernel).
+    // where depth >= 1 (feature_kernel).
     const float4* guide;
     const float4* old_guide;
     // Per-pixel edge-stopping features of this frame (feature_kernel), two
@@ -121,7 +121,7 @@ struct Sv {
                 a.color = xyz(k);
                 a.m0 = n.w;
                 a.m1 = k.w;
-                a.pixel_scale = g.w;  // distance(position, camera) / height (guide_kernel)
+                a.pixel_scale = g.w;  // distance(position, camera) / height (feature_kernel)
                 return a;
             }
         }

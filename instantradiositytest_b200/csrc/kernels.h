@@ -257,8 +257,8 @@ size_t irt_lighting_args_size(int gbuffer_format);
 void irt_lighting_args_fill(const LightingLaunch& L, void* out);
 cudaError_t irt_launch_lighting_batched(const BatchLaunch& B, int stage, cudaStream_t st);
 // SVGF stages of a batch: 0 temporal, 1 variance, 2 a-trous (BatchLaunch::
-// step), 3 guides of this frame, 4 guides of the previous frame, 5 depth
-// and normal history copy, 6 guides and features of this frame.
+// step), 4 guides of the previous frame, 5 depth and normal history copy, 6
+// guides and features of this frame.
 size_t irt_svgf_view_size(int gbuffer_format);
 void irt_svgf_view_fill(const SvgfLaunch& L, void* out);
 cudaError_t irt_launch_svgf_batched(const BatchLaunch& B, int stage, cudaStream_t st);

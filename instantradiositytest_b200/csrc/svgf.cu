@@ -208,15 +208,15 @@ __global__ void __launch_bounds__(256) history_kernel(uint32_t pixels, const flo
     old_normal[i] = normal[i];
 }
 
-// Batched guides (in = depth, out = guide) and depth/normal history copy
+// Batched guides of the previous frame (in = its depth, out = guide) and depth/normal history copy
 // (in = depth, aux = normal, out = previous depth, out2 = previous normal);
 // 1-D tiles of 256 pixels.
 template <class G>
 __global__ void __launch_bounds__(256) guide_batched(const irt_frame* __restrict__ frames, const SView<G>* __restrict__ views,
-                                                     const uint32_t* __restrict__ tile_start, uint32_t n, int previous) {
+                                                     const uint32_t* __restrict__ tile_start, uint32_t n) {
     const uint32_t v = svgf_find_view(tile_start, n, blockIdx.x);
     const SView<G>& w = views[v];
-    guide_body(frames[v], (const float*)w.in, previous, (float4*)w.out,
+    guide_body(frames[v], (const float*)w.in, 1, (float4*)w.out,
                (size_t)(blockIdx.x - __ldg(tile_start + v)) * blockDim.x + threadIdx.x);
 }
 
@@ -274,8 +274,7 @@ static cudaError_t svgf_batched_typed(const BatchLaunch& B, int stage, cudaStrea
     const SView<G>* views = static_cast<const SView<G>*>(B.table);
     switch (stage) {
     case 0: svgf_temporal_batched<G, R, M><<<B.tiles, dim3(B.bx, B.by), 0, st>>>(B.frames, views, B.tile_start, B.n); break;
-    case 3:
-    case 4: guide_batched<G><<<B.tiles, 256, 0, st>>>(B.frames, views, B.tile_start, B.n, stage == 4); break;
+    case 4: guide_batched<G><<<B.tiles, 256, 0, st>>>(B.frames, views, B.tile_start, B.n); break;
     case 5: history_batched<G><<<B.tiles, 256, 0, st>>>(B.frames, views, B.tile_start, B.n); break;
     case 6: feature_batched<G><<<B.tiles, 256, 0, st>>>(B.frames, views, B.tile_start, B.n); break;
     default: return cudaErrorInvalidValue;
