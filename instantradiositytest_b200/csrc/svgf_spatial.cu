@@ -121,7 +121,8 @@ constexpr uint32_t kSpreadYoung = 64;
 template <class G, class R, class M>
 __device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* input,
                                               const typename M::T* moments, typename R::T* out, int32_t x, int32_t y) {
-    __shared__ uint32_t list[256], listed;
+    __shared__ int2 list[256];  // whole coordinates: frames may be wider than 16 bits hold
+    __shared__ uint32_t listed;
     const unsigned full = 0xffffffffu;
     const int32_t W = (int32_t)f.size[0], H = (int32_t)f.size[1];
     const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x, lane = t & 31u;
@@ -141,11 +142,11 @@ __device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<
     uint32_t base = 0;
     if (lane == 0u && in_warp) base = atomicAdd(&listed, (uint32_t)__popc(in_warp));
     base = __shfl_sync(full, base, 0);
-    if (young) list[base + (uint32_t)__popc(in_warp & ((1u << lane) - 1u))] = (uint32_t)x | (uint32_t)y << 16;
+    if (young) list[base + (uint32_t)__popc(in_warp & ((1u << lane) - 1u))] = make_int2(x, y);
     __syncthreads();
     const uint32_t n = listed;
     auto pixel = [&](uint32_t k, auto&& sums) {
-        const int32_t px = (int32_t)(list[k] & 0xffffu), py = (int32_t)(list[k] >> 16);
+        const int32_t px = list[k].x, py = list[k].y;
         const ptrdiff_t i = (ptrdiff_t)py * W + px;
         const Moments centre = M::load(moments, i);
         TapCentre a;
