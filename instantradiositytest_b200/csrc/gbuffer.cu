@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <vector>
 
 #include "dev_prims.cuh"
@@ -36,8 +37,9 @@ __device__ __forceinline__ uint32_t oct_snorm16(float x, float y, float z) {
     return ((uint32_t)(uint16_t)(int16_t)qu) | ((uint32_t)(uint16_t)(int16_t)qv << 16);
 }
 
-// Ray of the image point (u, v): d spans near to far plane, t in [0, 1).
-__device__ __forceinline__ void primary_ray(const irt_frame& f, float u, float v, float o[3], float d[3]) {
+// Ray of the image point (u, v): d spans near to far plane, t in [0, 1).  w:
+// the homogeneous coordinates of the two points.
+__device__ __forceinline__ void primary_ray(const irt_frame& f, float u, float v, float o[3], float d[3], float w[2]) {
     float nx = u * 2.f - 1.f, ny = 1.f - v * 2.f;
     float pn[4], pf[4];
     xf(f.inv_vp.m, nx, ny, 0.f, 1.f, pn);
@@ -47,17 +49,34 @@ __device__ __forceinline__ void primary_ray(const irt_frame& f, float u, float v
         o[a] = pn[a] / pn[3];
         d[a] = pf[a] / pf[3] - o[a];
     }
+    w[0] = pn[3];
+    w[1] = pf[3];
 }
 
 // Primitives a block of pixels may see, in ascending order: those whose
-// bounding sphere is not wholly beyond one of the four planes through the
-// block's corner rays, by a margin well above the f32 error of the rays (a
-// far plane's corner is good to about 1e-4 of its distance).  Every pixel of
-// the block tests the same few primitives instead of all: 1280x720, 23
-// objects 97 -> 57 us, 2560x1600, 50 objects 816 -> 300.
+// bounding sphere is not wholly beyond one of the four planes through the rays
+// of neighbouring block corners.  Every pixel of the block tests the same few
+// primitives instead of all: 1280x720, 23 objects 97 -> 57 us, 2560x1600, 50
+// objects 816 -> 300.
+//
+// The planes hold for every inv_vp, parallel projections among them: a plane
+// goes through both corners' near and far points (parallel image lines stay
+// coplanar), and its outer side follows from the sign of inv_vp's determinant
+// (`orientation`, from the host), which a block too narrow for f32 cannot get
+// wrong.  What f32 makes of the corners, and of the pixels' own rays, goes into
+// each plane's slack.  A block whose homogeneous w changes its sign is not the
+// hull of its corners and keeps all primitives, as does anything not finite.
 constexpr uint32_t kMaxListed = 2048;
+// What the lists of a frame need of its inv_vp besides the rays.
+struct ListFrame {
+    float orientation;     // sign of the determinant; 0: no planes
+    float near_sum, far_sum;  // length of the sums of |products| behind a near and a far point
+    float w_sum;           // the same of w, or 0 where every pixel has the same bits of w
+};
 struct BlockPrims {
     float corner_o[4][3], corner_d[4][3];
+    float plane[4][3];  // unit normal, outward; 0 = no plane
+    float slack[4];     // of a distance from the plane, per distance from its corner
     uint32_t count;
     uint16_t index[kMaxListed];
 };
@@ -89,37 +108,52 @@ __device__ __forceinline__ bool beyond(const BlockPrims& s, const GPrim& p) {
         }
         stretch = fmaxf(stretch, row);
     }
-    const float r = half * sqrtf(stretch);
-    float centre[3];
-    for (int a = 0; a < 3; a++)
-        centre[a] = s.corner_d[0][a] + s.corner_d[1][a] + s.corner_d[2][a] + s.corner_d[3][a];
+    const float r = 1.01f * half * sqrtf(stretch);
     for (int k = 0; k < 4; k++) {
-        const float *da = s.corner_d[k], *db = s.corner_d[(k + 1) & 3], *o = s.corner_o[k];
-        float n[3] = {da[1] * db[2] - da[2] * db[1], da[2] * db[0] - da[0] * db[2], da[0] * db[1] - da[1] * db[0]};
-        const float len = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-        float side = n[0] * centre[0] + n[1] * centre[1] + n[2] * centre[2];
-        if (side < 0.f) {
-            n[0] = -n[0];
-            n[1] = -n[1];
-            n[2] = -n[2];
-        }
+        const float *n = s.plane[k], *o = s.corner_o[k];
         const float w[3] = {c[0] - o[0], c[1] - o[1], c[2] - o[2]};
-        const float away = sqrtf(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-        // parallel corner rays (len 0) and anything not a number keep the primitive
-        if (n[0] * w[0] + n[1] * w[1] + n[2] * w[2] < -len * (1.01f * r + .02f * away + 1e-3f)) return true;
+        const float away = sqrtf(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]) + r;
+        if (n[0] * w[0] + n[1] * w[1] + n[2] * w[2] > r + s.slack[k] * away + 1e-3f) return true;
     }
     return false;
 }
-__device__ __forceinline__ void list_block_prims(const irt_frame& f, const irt::PrimTable& T, BlockPrims& s) {
-    const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x;
-    if (t < 4u) {  // the corners of the block's pixels, in a cycle
-        const float W = (float)f.size[0], H = (float)f.size[1];
-        const float x = (float)((blockIdx.x + (t == 1u || t == 2u ? 1u : 0u)) * blockDim.x);
-        const float y = (float)((blockIdx.y + (t >= 2u ? 1u : 0u)) * blockDim.y);
-        primary_ray(f, fminf(x, W) / W, fminf(y, H) / H, s.corner_o[t], s.corner_d[t]);
+// The plane through corner t of the block's pixels and the next in their
+// cycle; by lanes 0-3.
+__device__ __forceinline__ void block_plane(const irt_frame& f, const ListFrame& lf, uint32_t t, BlockPrims& s) {
+    const unsigned lanes = 0xfu;
+    const float W = (float)f.size[0], H = (float)f.size[1];
+    const float x = (float)((blockIdx.x + (t == 1u || t == 2u ? 1u : 0u)) * blockDim.x);
+    const float y = (float)((blockIdx.y + (t >= 2u ? 1u : 0u)) * blockDim.y);
+    float o[3], d[3], w[2], v[3], norm[2];
+    primary_ray(f, fminf(x, W) / W, fminf(y, H) / H, o, d, w);
+    // |a coordinate's error| <= 4 roundings of its sum, the same of w, one
+    // division: 2^-22 of them; as much again for the pixels' own rays.
+    norm[0] = fabsf(o[0]) + fabsf(o[1]) + fabsf(o[2]);
+    norm[1] = fabsf(o[0] + d[0]) + fabsf(o[1] + d[1]) + fabsf(o[2] + d[2]);
+    const float e = 0x1p-21f * (__fdividef(lf.near_sum + norm[0] * lf.w_sum, fabsf(w[0])) + norm[0] +
+                                __fdividef(lf.far_sum + norm[1] * lf.w_sum, fabsf(w[1])) + norm[1]);
+    const bool hull = __all_sync(lanes, w[0] > 0.f && w[1] > 0.f) || __all_sync(lanes, w[0] < 0.f && w[1] < 0.f);
+    const int next = (int)((t + 1u) & 3u);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        s.corner_o[t][i] = o[i];
+        s.corner_d[t][i] = d[i];
+        v[i] = __shfl_sync(lanes, o[i] + d[i], next) - o[i];
     }
-    __syncthreads();
+    const float n[3] = {d[1] * v[2] - d[2] * v[1], d[2] * v[0] - d[0] * v[2], d[0] * v[1] - d[1] * v[0]};
+    const float inv = rsqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    const float ld = fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]), lv = fabsf(v[0]) + fabsf(v[1]) + fabsf(v[2]);
+    const float error = fmaxf(e, __shfl_sync(lanes, e, next)) * (ld + lv) + 0x1p-21f * ld * lv;
+#pragma unroll
+    for (int i = 0; i < 3; i++) s.plane[t][i] = hull ? n[i] * (lf.orientation * inv) : 0.f;
+    s.slack[t] = .002f + error * inv;
+}
+__device__ __forceinline__ void list_block_prims(const irt_frame& f, const ListFrame& lf, const irt::PrimTable& T,
+                                                 BlockPrims& s) {
+    const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x;
     if (t < 32u) {
+        if (t < 4u) block_plane(f, lf, t, s);
+        __syncwarp();
         uint32_t count = 0;
         for (uint32_t first = 0; first < T.n; first += 32u) {
             const bool keep = first + t < T.n && !beyond(s, T.prims[first + t]);
@@ -132,19 +166,19 @@ __device__ __forceinline__ void list_block_prims(const irt_frame& f, const irt::
     __syncthreads();
 }
 
-__global__ void gbuffer_kernel(const __grid_constant__ irt_frame f, const irt::PrimTable T, int fmt,
-                               float* depth, void* normal, void* color, void* params, void* motion) {
+__global__ void gbuffer_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ ListFrame lf, const irt::PrimTable T,
+                               int fmt, float* depth, void* normal, void* color, void* params, void* motion) {
     __shared__ BlockPrims listed;
     const bool list = T.n <= kMaxListed;
-    if (list) list_block_prims(f, T, listed);
+    if (list) list_block_prims(f, lf, T, listed);
     uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
     uint32_t W = f.size[0], H = f.size[1];
     if (x >= W || y >= H) return;
     size_t i = (size_t)y * W + x;
     float u = ((float)x + .5f) / (float)W, v = ((float)y + .5f) / (float)H;
-    float o[3], d[3];
-    primary_ray(f, u, v, o, d);
+    float o[3], d[3], hw[2];
+    primary_ray(f, u, v, o, d, hw);
     float best;
     float nl_best[3] = {0, 0, 0};
     int hit = irtd::cast_prims(T, list ? listed.count : T.n, [&](uint32_t j) { return list ? (uint32_t)listed.index[j] : j; },
@@ -190,6 +224,29 @@ __global__ void gbuffer_kernel(const __grid_constant__ irt_frame f, const irt::P
         ((uint32_t*)params)[i] = hbits(par[0]) | ((uint32_t)hbits(par[1]) << 16);
         ((uint32_t*)motion)[i] = hbits(mot[0]) | ((uint32_t)hbits(mot[1]) << 16);
     }
+}
+
+ListFrame list_frame(const float* m) {
+    ListFrame lf{};
+    auto minor = [&](int r, int a, int b) {  // rows r and r + 1, columns a and b
+        return (double)m[4 * a + r] * m[4 * b + r + 1] - (double)m[4 * b + r] * m[4 * a + r + 1];
+    };
+    const double det = minor(0, 0, 1) * minor(2, 2, 3) - minor(0, 0, 2) * minor(2, 1, 3) + minor(0, 0, 3) * minor(2, 1, 2) +
+                       minor(0, 1, 2) * minor(2, 0, 3) - minor(0, 1, 3) * minor(2, 0, 2) + minor(0, 2, 3) * minor(2, 0, 1);
+    lf.orientation = det > 0 ? 1.f : det < 0 ? -1.f : 0.f;
+    double near2 = 0, far2 = 0;
+    for (int a = 0; a < 3; a++) {
+        const double near_a = std::fabs(m[a]) + std::fabs(m[4 + a]) + std::fabs(m[12 + a]);
+        near2 += near_a * near_a;
+        far2 += (near_a + std::fabs(m[8 + a])) * (near_a + std::fabs(m[8 + a]));
+    }
+    lf.near_sum = (float)std::sqrt(near2);
+    lf.far_sum = (float)std::sqrt(far2);
+    // x and y too small to reach the sum's last bit leave w the same everywhere
+    const double xy = std::fabs(m[3]) + std::fabs(m[7]), z = std::fabs(m[11]), one = std::fabs(m[15]);
+    const bool same = xy <= 0x1p-26 * one && (z == 0 || xy <= 0x1p-26 * z);
+    lf.w_sum = same ? 0.f : (float)(xy + z + one);
+    return lf;
 }
 
 }  // namespace
@@ -304,6 +361,6 @@ extern "C" irt_status irt_gbuffer_render(irt_context* ctx, const irt_workload* w
     dim3 block(32, 8);
     dim3 grid((f->size[0] + 31) / 32, (f->size[1] + 7) / 8);
     gbuffer_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
-        *f, T, format, depth, normal, color, params, motion);
+        *f, list_frame(f->inv_vp.m), T, format, depth, normal, color, params, motion);
     return cudaGetLastError() == cudaSuccess ? IRT_OK : IRT_E_CUDA;
 }
