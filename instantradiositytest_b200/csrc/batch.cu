@@ -6,14 +6,15 @@
 // irt_frame_lighting + irt_frame_svgf, each step as one batched launch:
 //   frame upload (pinned -> device table), position guides and features (this
 //   frame and the previous), VPL pools (archive slot, endpoints, ray-counter
-//   reset), reuse, spatial, ray set-up and march (views grouped by scene),
+//   reset), reuse, spatial, ray set-up and march (views grouped by scene and
+//   march parameters),
 //   combine, SVGF temporal, variance, a-trous x iterations, depth/normal
 //   history copy.
 // The per-view tables hold the same pointers the single-session path passes
 // as kernel parameters, so every view's results are identical to rendering
 // it alone.  Tables depend on the frame parity (SVGF ping-pong) and on the
 // caller's buffers; they are rebuilt (and graphs re-captured) when any
-// pointer or scene layout changes.
+// pointer, scene layout or march parameter changes.
 // Views run in waves: consecutive views whose pixels add up to at most the
 // wave budget share one launch per pass, and the waves run one after
 // another, so a wave's buffers are still in L2 when its next pass reads them
@@ -202,10 +203,12 @@ std::vector<uintptr_t> signature_of(const irt_batch* b, irt_scene* const* scenes
                             (uintptr_t)cur[v], (uintptr_t)prev[v], frames[v].counts[0], frames[v].counts[3],
                             (uintptr_t)sc->field_linear};
         sig.insert(sig.end(), std::begin(vals), std::end(vals));
-        uint32_t gi[7];
+        uint32_t gi[13];
         std::memcpy(gi, sc->grid_org, 12);
         std::memcpy(gi + 3, sc->grid_inv, 12);
-        std::memcpy(gi + 6, &sc->grid_slack, 4);
+        std::memcpy(gi + 6, sc->grid_size, 12);
+        std::memcpy(gi + 9, &sc->grid_slack, 4);
+        std::memcpy(gi + 10, frames[v].sdf, 12);  // the march's parameters are in its groups
         sig.insert(sig.end(), std::begin(gi), std::end(gi));
     }
     return sig;
@@ -277,23 +280,27 @@ irt_status build_tables(irt_batch* b, int p, irt_scene* const* scenes, const irt
     CK(upload(&t.largs, hl.data(), hl.size()), "batch lighting table");
     for (int k = 0; k < 8; k++) CK(upload(&t.sviews[k], hs[k].data(), hs[k].size()), "batch svgf table");
     CK(upload(&t.history, hs[8].data(), hs[8].size()), "batch history table");
-    // March: per wave, its views grouped by scene (groups in order of first
-    // appearance); a group's queues are its views' ray queues.
+    // March: per wave, its views grouped by scene and march parameters (groups
+    // in order of first appearance); a group's queues are its views' ray queues.
     std::vector<MarchGroup> groups;
     std::vector<MarchQueue> queues;
     t.max_scene_bytes = 0;
     t.wave_groups.assign(1, 0);
     for (size_t w = 0; w + 1 < b->wave_begin.size(); w++) {
         const uint32_t v0 = b->wave_begin[w], v1 = b->wave_begin[w + 1];
-        std::vector<const irt_scene*> order;
+        auto together = [&](uint32_t a, uint32_t v) {
+            return scenes[a] == scenes[v] && std::memcmp(frames[a].sdf, frames[v].sdf, sizeof(float) * 3) == 0;
+        };
+        std::vector<uint32_t> order;  // first view of each group
         for (uint32_t v = v0; v < v1; v++)
-            if (std::find(order.begin(), order.end(), scenes[v]) == order.end()) order.push_back(scenes[v]);
-        for (const irt_scene* sc : order) {
+            if (std::none_of(order.begin(), order.end(), [&](uint32_t a) { return together(a, v); })) order.push_back(v);
+        for (const uint32_t first : order) {
+            const irt_scene* sc = scenes[first];
             MarchGroup G{};
             G.q_begin = (uint32_t)queues.size();
+            G.f = frames[first];
             for (uint32_t v = v0; v < v1; v++) {
-                if (scenes[v] != sc) continue;
-                if (queues.size() == G.q_begin) G.f = frames[v];
+                if (!together(first, v)) continue;
                 irt_session* s = b->sess[v];
                 queues.push_back(MarchQueue{session_ray_setup(s, sc, cur[v], prev[v]), b->d_frames + v, s->W, s->H});
                 if (!G.error) G.error = s->error;
