@@ -46,6 +46,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "dev_sdf.cuh"
 #include "kernels.h"
@@ -741,25 +742,56 @@ static cudaError_t march_prefer_l1(const void* kernel, uint32_t smem, int blocks
 
 namespace {
 
-// Per thread and device: a kernel's dynamic shared memory attribute and its
-// resident CTAs per SM for that size.
+// A kernel's dynamic shared memory limit and its resident CTAs per SM for a
+// scene's bytes.  The limit is the function's, shared by every thread that
+// launches it on the device, so it is raised once to all a CTA can have and
+// never follows a scene.  The carveout is a hint, set when the bytes change.
 struct KernelFit {
-    int device = -1;
-    uint32_t smem = 0;
-    int per_sm = 0;
+    static constexpr int kDevices = 64, kSizes = 16;
+    struct Device {
+        bool raised;
+        uint32_t carveout_for, next;
+        uint32_t bytes[kSizes];  // 0: unused (no scene is empty)
+        int per_sm[kSizes];
+    };
+    std::mutex mu;
+    Device devices[kDevices] = {};
 
-    cudaError_t set(const void* kernel, int threads, uint32_t bytes, int prefer_blocks) {
+    cudaError_t set(const void* kernel, int threads, uint32_t bytes, int prefer_blocks, int& per_sm) {
         int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev == device && bytes == smem) return cudaSuccess;
-        device = dev;
-        smem = 0;
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e == cudaSuccess) e = march_prefer_l1(kernel, bytes, prefer_blocks);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes);
+        cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
-        if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        smem = bytes;
+        if (dev < 0 || dev >= kDevices) return cudaErrorInvalidDevice;
+        std::lock_guard<std::mutex> lock(mu);
+        Device& d = devices[dev];
+        if (!d.raised) {
+            int most = 0;
+            cudaFuncAttributes own;
+            e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&own, kernel);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         most - (int)own.sharedSizeBytes);
+            if (e != cudaSuccess) return e;
+            d.raised = true;
+        }
+        if (d.carveout_for != bytes) {
+            e = march_prefer_l1(kernel, bytes, prefer_blocks);
+            if (e != cudaSuccess) return e;
+            d.carveout_for = bytes;
+        }
+        for (int k = 0; k < kSizes; k++)
+            if (d.bytes[k] == bytes) {
+                per_sm = d.per_sm[k];
+                return cudaSuccess;
+            }
+        int fits = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, kernel, threads, bytes);
+        if (e != cudaSuccess) return e;
+        if (fits < 1) return cudaErrorInvalidConfiguration;
+        const uint32_t k = d.next++ % kSizes;
+        d.bytes[k] = bytes;
+        d.per_sm[k] = per_sm = fits;
         return cudaSuccess;
     }
 };
@@ -793,8 +825,9 @@ IRT_MARCH_NS::Grid launch_grid(const MarchLaunch& M) {
 cudaError_t IRT_MARCH_FN(irt_launch_ray_pools)(const MarchLaunch& M, cudaStream_t st) {
     using namespace IRT_MARCH_NS;
     const uint32_t smem = irt_march_scene_bytes(M.frame->counts[3]);
-    thread_local KernelFit fit;
-    cudaError_t e = fit.set((const void*)ray_pools_kernel, kMarchThreads, smem, 1);
+    static KernelFit fit;
+    int per_sm;
+    cudaError_t e = fit.set((const void*)ray_pools_kernel, kMarchThreads, smem, 1, per_sm);
     if (e != cudaSuccess) return e;
     const uint32_t entries = (M.setup.slots + 2u) * M.setup.vpl_count;
     const uint32_t blocks = std::min((uint32_t)M.num_sms, (entries + kMarchThreads - 1) / kMarchThreads);
@@ -808,17 +841,18 @@ cudaError_t IRT_MARCH_FN(irt_launch_march)(const MarchLaunch& M, cudaStream_t st
     typedef decltype(&march_kernel<kPointF32>) Kernel;
     static const Kernel kernels[] = {march_kernel<kPointF32>, march_kernel<kPointF16>, march_kernel<kLinearF32>};
     const int sampler = march_sampler(M.field_filter, M.sdf_f16);
-    thread_local KernelFit set_up, fits[3];
-    KernelFit& march = fits[sampler];
-    cudaError_t e = set_up.set((const void*)ray_setup_kernel, kSetupThreads, smem, 2);
-    if (e == cudaSuccess) e = march.set((const void*)kernels[sampler], kMarchThreads, smem, kMarchCtasPerSm);
+    static KernelFit set_up, march[3];
+    int set_up_per_sm, march_per_sm;
+    cudaError_t e = set_up.set((const void*)ray_setup_kernel, kSetupThreads, smem, 2, set_up_per_sm);
+    if (e == cudaSuccess)
+        e = march[sampler].set((const void*)kernels[sampler], kMarchThreads, smem, kMarchCtasPerSm, march_per_sm);
     if (e != cudaSuccess) return e;
     const irtd::DevScene sc = launch_scene(M);
     const Grid g = launch_grid(M);
-    e = launch_behind(ray_setup_kernel, dim3(M.num_sms * set_up.per_sm), dim3(kSetupThreads), smem, st, *M.frame, sc,
+    e = launch_behind(ray_setup_kernel, dim3(M.num_sms * set_up_per_sm), dim3(kSetupThreads), smem, st, *M.frame, sc,
                       M.march_scene, smem / 16, g, M.setup);
     if (e != cudaSuccess) return e;
-    return launch_behind(kernels[sampler], dim3(M.num_sms * march.per_sm), dim3(kMarchThreads), smem, st, *M.frame, sc,
+    return launch_behind(kernels[sampler], dim3(M.num_sms * march_per_sm), dim3(kMarchThreads), smem, st, *M.frame, sc,
                          M.march_scene, smem / 16, g, M.setup);
 }
 
@@ -826,10 +860,11 @@ cudaError_t IRT_MARCH_FN(irt_launch_ray_pools_batched)(const MarchBatch& M, cuda
     using namespace IRT_MARCH_NS;
     if (M.n_groups == 0) return cudaSuccess;
     const uint32_t smem = kGroupVec4 * 16 + M.max_scene_bytes;
-    thread_local KernelFit fit;
-    cudaError_t e = fit.set((const void*)ray_pools_batched_kernel, 128, smem, 1);
+    static KernelFit fit;
+    int per_sm;
+    cudaError_t e = fit.set((const void*)ray_pools_batched_kernel, 128, smem, 1, per_sm);
     if (e != cudaSuccess) return e;
-    ray_pools_batched_kernel<<<M.num_sms * std::min(fit.per_sm, 2), 128, smem, st>>>(M.groups, M.n_groups, M.queues);
+    ray_pools_batched_kernel<<<M.num_sms * std::min(per_sm, 2), 128, smem, st>>>(M.groups, M.n_groups, M.queues);
     return cudaGetLastError();
 }
 
@@ -841,15 +876,16 @@ cudaError_t IRT_MARCH_FN(irt_launch_march_batched)(const MarchBatch& M, cudaStre
     static const Kernel kernels[] = {march_batched_kernel<kPointF32>, march_batched_kernel<kPointF16>,
                                      march_batched_kernel<kLinearF32>, march_batched_kernel<kAnySampler>};
     if (M.sampler < 0 || M.sampler > kAnySampler) return cudaErrorInvalidValue;
-    thread_local KernelFit set_up, fits[4];
-    KernelFit& march = fits[M.sampler];
-    cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, kSetupThreads, smem, 2);
+    static KernelFit set_up, march[4];
+    int set_up_per_sm, march_per_sm;
+    cudaError_t e = set_up.set((const void*)ray_setup_batched_kernel, kSetupThreads, smem, 2, set_up_per_sm);
     const int threads = march_threads(M.sampler);
     if (e == cudaSuccess)
-        e = march.set((const void*)kernels[M.sampler], threads, M.max_scene_bytes, march_ctas(M.sampler));
+        e = march[M.sampler].set((const void*)kernels[M.sampler], threads, M.max_scene_bytes, march_ctas(M.sampler),
+                                 march_per_sm);
     if (e != cudaSuccess) return e;
-    const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < march.per_sm ? M.blocks_per_sm : march.per_sm;
-    ray_setup_batched_kernel<<<M.num_sms * set_up.per_sm, kSetupThreads, smem, st>>>(M.groups, M.n_groups, M.queues);
+    const int bps = M.blocks_per_sm > 0 && M.blocks_per_sm < march_per_sm ? M.blocks_per_sm : march_per_sm;
+    ray_setup_batched_kernel<<<M.num_sms * set_up_per_sm, kSetupThreads, smem, st>>>(M.groups, M.n_groups, M.queues);
     for (uint32_t g = 0; g < M.n_groups; g += kMarchGroups) {
         MarchGroups part;
         part.n = std::min(M.n_groups - g, kMarchGroups);
