@@ -89,45 +89,46 @@ struct SceneLayout {
 };
 
 // Replaces the scene's block and staging by ones of this capacity; nothing of
-// the old ones is kept, so the leaf-order cache is to be built again.
+// the old ones is kept, so the leaf-order cache is to be built again, and until
+// the update that grows has completed the scene has no objects to render.  A
+// growth that fails leaves the scene as it was.
 static irt_status scene_grow(irt_scene* sc, uint32_t object_cap, uint32_t light_cap) {
     irt_context* ctx = sc->ctx;
-    for (cudaEvent_t& e : sc->pinned_free) {
-        if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "staging");
-        CK(cudaEventSynchronize(e), "staging");
+    const SceneLayout at(object_cap, light_cap);
+    char* block = nullptr;
+    uint64_t added = 0;
+    irt_status st = dev_alloc(ctx, &block, at.total, added);
+    if (st) return st;
+    unsigned char* pinned = nullptr;
+    cudaError_t e = cudaMallocHost(&pinned, 2 * at.copied);
+    for (cudaEvent_t& ev : sc->pinned_free) {
+        if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventSynchronize(ev);
     }
+    if (e != cudaSuccess) {
+        if (pinned) cudaFreeHost(pinned);
+        cudaFree(block);
+        return cuda_fail(ctx, e, "staging");
+    }
+    std::memset(pinned, 0, 2 * at.copied);
     if (sc->pinned) cudaFreeHost(sc->pinned);
     if (sc->block) cudaFree(sc->block);  // waits for the work that reads it
-    sc->pinned = nullptr;
-    sc->block = nullptr;
-    sc->objects = nullptr;
-    sc->nodes = nullptr;
-    sc->lights = sc->lights_prep = nullptr;
-    sc->march_scene = nullptr;
-    sc->cells = nullptr;
-    sc->cached_nodes.clear();
-    sc->cached_objects.clear();
-    sc->bytes -= sc->block_bytes;
-    ctx->in_use -= sc->block_bytes;
-    sc->block_bytes = 0;
-    sc->object_cap = sc->light_cap = 0;
-    const SceneLayout at(object_cap, light_cap);
-    CK(cudaMallocHost(&sc->pinned, 2 * at.copied), "staging");
-    std::memset(sc->pinned, 0, 2 * at.copied);
-    uint64_t added = 0;
-    irt_status st = dev_alloc(ctx, &sc->block, at.total, added);
-    if (st) return st;
+    sc->bytes += added - sc->block_bytes;
+    ctx->in_use += added - sc->block_bytes;
     sc->block_bytes = added;
-    sc->bytes += added;
-    ctx->in_use += added;
-    sc->objects = reinterpret_cast<irt_object*>(sc->block + at.objects);
-    sc->nodes = reinterpret_cast<irt_node*>(sc->block + at.nodes);
-    sc->lights = reinterpret_cast<irt_light*>(sc->block + at.lights);
-    sc->lights_prep = reinterpret_cast<irt_light*>(sc->block + at.lights_prep);
-    sc->march_scene = reinterpret_cast<float4*>(sc->block + at.march);
-    sc->cells = reinterpret_cast<uint4*>(sc->block + at.cells);
+    sc->pinned = pinned;
+    sc->block = block;
+    sc->objects = reinterpret_cast<irt_object*>(block + at.objects);
+    sc->nodes = reinterpret_cast<irt_node*>(block + at.nodes);
+    sc->lights = reinterpret_cast<irt_light*>(block + at.lights);
+    sc->lights_prep = reinterpret_cast<irt_light*>(block + at.lights_prep);
+    sc->march_scene = reinterpret_cast<float4*>(block + at.march);
+    sc->cells = reinterpret_cast<uint4*>(block + at.cells);
     sc->object_cap = object_cap;
     sc->light_cap = light_cap;
+    sc->object_count = sc->light_count = 0;
+    sc->cached_nodes.clear();
+    sc->cached_objects.clear();
     return IRT_OK;
 }
 

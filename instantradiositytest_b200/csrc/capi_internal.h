@@ -174,7 +174,10 @@ uint32_t normal_bytes_of(int fmt) {
     return fmt == IRT_GBUFFER_F32 ? 16u : (fmt == IRT_GBUFFER_F16 ? 8u : 4u);
 }
 
+// The error is reported here; left as the thread's last error, the next launch
+// that asks for its own would report it again.
 irt_status cuda_fail(irt_context* ctx, cudaError_t e, const char* what) {
+    cudaGetLastError();
     if (ctx) ctx->set_error(std::string(what) + ": " + cudaGetErrorString(e));
     return IRT_E_CUDA;
 }
