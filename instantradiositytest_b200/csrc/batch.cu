@@ -659,6 +659,10 @@ irt_status irt_batch_render(irt_batch* b, irt_scene* const* scenes, const irt_fr
             ctx->set_error("batched frame counts differ from the batch/scene");
             return IRT_E_INVALID;
         }
+        if (sc->object_count == 0) {  // nothing uploaded yet: no tables to launch on
+            ctx->set_error("the scene has had no update");
+            return IRT_E_INVALID;
+        }
         if (f.restir[0] == 0 || f.restir[0] > 256 || f.restir[1] == 0 || f.restir[1] > 256 || f.restir[2] > 32 ||
             f.restir[3] > 256 || !(f.sdf[0] >= 1.f && f.sdf[0] <= 1024.f) || !(f.sdf[1] > 0.f)) {
             ctx->set_error("frame ReSTIR/SDF parameters out of range");

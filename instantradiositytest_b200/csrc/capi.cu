@@ -644,6 +644,10 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
         ctx->set_error("frame counts differ from the session/scene");
         return IRT_E_INVALID;
     }
+    if (sc->object_count == 0) {  // nothing uploaded yet: no tables to launch on
+        ctx->set_error("the scene has had no update");
+        return IRT_E_INVALID;
+    }
     // Loop bounds the kernels take from the frame stay within the ranges
     // Settings::validate admits (src/settings.rs:63-94).
     if (f->restir[0] == 0 || f->restir[0] > 256 || f->restir[1] == 0 || f->restir[1] > 256 || f->restir[2] > 32 ||
