@@ -781,8 +781,10 @@ irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer*
         mark(s, 8, st);
     } else {
         // Positions for this frame (already there when the lighting ran).
-        if (s->guide_frame != f->size[2]) CK(compute_guides(s, f, g, st), "position guides");
+        const bool fresh = s->guide_frame != f->size[2];
+        if (fresh) CK(compute_guides(s, f, g, st), "position guides");
         SvgfLaunch L{};
+        L.after_guides = fresh;
         L.frame = f;
         L.gbuffer = *g;
         L.old_depth = s->prev_depth;
@@ -798,6 +800,7 @@ irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer*
         L.out = s->temporal;
         L.moments_out = s->moments[cur];
         CK(irt_launch_svgf(L, 0, st), "svgf temporal");
+        L.after_guides = 0;
         mark(s, 6, st);
         L.in = s->temporal;
         L.moments_in = s->moments[cur];

@@ -182,6 +182,24 @@ __device__ __forceinline__ V3 brdf(const Surface& s, V3 wi) {
     return out;
 }
 
+// A load of what the kernel before this one in the frame may have written
+// (launch_behind, kernels.h).
+template <class T>
+__device__ __forceinline__ T load_written(const T* p) {
+    __builtin_assume(__isGlobal(p));
+    return *p;
+}
+// How a function that serves several kernels loads: what nothing writes while
+// its kernel is resident, or what the kernel before it may have written.
+struct Settled {
+    template <class T>
+    __device__ __forceinline__ static T load(const T* p) { return __ldg(p); }
+};
+struct Written {
+    template <class T>
+    __device__ __forceinline__ static T load(const T* p) { return load_written(p); }
+};
+
 // Light and VPL records as three 16-byte vectors (read-only cache loads).
 // Lights are read from the per-frame prepared copy (prepare_lights_kernel):
 // da holds the normalised spot direction and cos(angle / 2) instead of the
@@ -244,7 +262,7 @@ struct Res {
 };
 __device__ __forceinline__ Res res_load(const irt_reservoir* base, size_t i) {
     const uint4* p = reinterpret_cast<const uint4*>(base + i);
-    uint4 a = __ldg(p), b = __ldg(p + 1);
+    uint4 a = load_written(p), b = load_written(p + 1);
     return Res{a.x, a.y, a.z, a.w, __uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), b.w};
 }
 // A reservoir is one 32-byte sector, moved as two 128-bit accesses.
@@ -295,9 +313,12 @@ struct GbF32 {
     const float2* motion;
     typedef float4 NormalT;
     __device__ __forceinline__ float d(size_t i) const { return __ldg(depth + i); }
-    __device__ __forceinline__ V3 n(size_t i) const { return xyz(__ldg(normal + i)); }
-    __device__ __forceinline__ V3 c(size_t i) const { return xyz(__ldg(color + i)); }
-    __device__ __forceinline__ float2 pm(size_t i) const { return __ldg(params + i); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ V3 n(size_t i) const { return xyz(Ld::load(normal + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ V3 c(size_t i) const { return xyz(Ld::load(color + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ float2 pm(size_t i) const { return Ld::load(params + i); }
     __device__ __forceinline__ float2 mv(size_t i) const { return __ldg(motion + i); }
     __device__ __forceinline__ static V3 decode_normal(NormalT v) { return xyz(v); }
 };
@@ -321,9 +342,12 @@ struct GbF16 {
     const uint32_t* motion;
     typedef uint2 NormalT;
     __device__ __forceinline__ float d(size_t i) const { return __ldg(depth + i); }
-    __device__ __forceinline__ V3 n(size_t i) const { return half4_xyz(__ldg(normal + i)); }
-    __device__ __forceinline__ V3 c(size_t i) const { return half4_xyz(__ldg(color + i)); }
-    __device__ __forceinline__ float2 pm(size_t i) const { return half2_f2(__ldg(params + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ V3 n(size_t i) const { return half4_xyz(Ld::load(normal + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ V3 c(size_t i) const { return half4_xyz(Ld::load(color + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ float2 pm(size_t i) const { return half2_f2(Ld::load(params + i)); }
     __device__ __forceinline__ float2 mv(size_t i) const { return half2_f2(__ldg(motion + i)); }
     __device__ __forceinline__ static V3 decode_normal(NormalT v) { return half4_xyz(v); }
 };
@@ -347,12 +371,15 @@ struct GbPacked {
     const uint32_t* motion;
     typedef uint32_t NormalT;
     __device__ __forceinline__ float d(size_t i) const { return __ldg(depth + i); }
-    __device__ __forceinline__ V3 n(size_t i) const { return oct_decode(__ldg(normal + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ V3 n(size_t i) const { return oct_decode(Ld::load(normal + i)); }
+    template <class Ld = Settled>
     __device__ __forceinline__ V3 c(size_t i) const {
-        uint32_t v = __ldg(color + i);
+        uint32_t v = Ld::load(color + i);
         return V3{(float)(v & 255u) / 255.f, (float)((v >> 8) & 255u) / 255.f, (float)((v >> 16) & 255u) / 255.f};
     }
-    __device__ __forceinline__ float2 pm(size_t i) const { return half2_f2(__ldg(params + i)); }
+    template <class Ld = Settled>
+    __device__ __forceinline__ float2 pm(size_t i) const { return half2_f2(Ld::load(params + i)); }
     __device__ __forceinline__ float2 mv(size_t i) const { return half2_f2(__ldg(motion + i)); }
     __device__ __forceinline__ static V3 decode_normal(NormalT v) { return oct_decode(v); }
 };

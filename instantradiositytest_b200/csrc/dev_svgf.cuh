@@ -75,7 +75,7 @@ struct MomF16 {
     }
 };
 
-template <class G>
+template <class G, class Ld>
 struct Sv {
     // Feature records are read by the temporal and variance passes for G-buffer
     // formats that decode per tap (on f32 planes they move 0.013 ms from one to
@@ -93,7 +93,7 @@ struct Sv {
     __device__ __forceinline__ float uvy(int32_t y) const { return ((float)(uint32_t)y + .5f) / (float)H; }
     // svgf.wgsl:19
     __device__ __forceinline__ V3 position(int32_t x, int32_t y) const {
-        return xyz(__ldg(c.guide + idx(x, y)));
+        return xyz(Ld::load(c.guide + idx(x, y)));
     }
     // svgf.wgsl:20-26
     // `a`, `n`: the pixel's position and (decoded) normal, `reach` =
@@ -101,7 +101,7 @@ struct Sv {
     __device__ __forceinline__ bool history_ok(V3 a, V3 n, float reach, int32_t qx, int32_t qy) const {
         if (f.flags[0] == 0u || f.flags[1] != f.size[3] || !inside(qx, qy)) return false;
         size_t q = idx(qx, qy);
-        const float4 guide = __ldg(c.old_guide + q);
+        const float4 guide = Ld::load(c.old_guide + q);
         if (guide.w < 0.f) return false;  // depth >= 1
         V3 b = xyz(guide);
         return distance(a, b) < reach && dot(n, G::decode_normal(__ldg(c.old_normal + q))) > f.temporal[2];
@@ -115,7 +115,7 @@ struct Sv {
         size_t i = idx(x, y);
         if constexpr (kFeatures) {
             if (c.feat) {
-                const float4 g = __ldg(c.guide + i), n = __ldg(c.feat + 2 * i), k = __ldg(c.feat + 2 * i + 1);
+                const float4 g = Ld::load(c.guide + i), n = Ld::load(c.feat + 2 * i), k = Ld::load(c.feat + 2 * i + 1);
                 a.position = xyz(g);
                 a.normal = xyz(n);
                 a.color = xyz(k);
@@ -140,9 +140,9 @@ struct Sv {
         size_t q = idx(qx, qy);
         if constexpr (kFeatures) {
             if (c.feat) {
-                const float4 g = __ldg(c.guide + q);
+                const float4 g = Ld::load(c.guide + q);
                 if (g.w < 0.f) return 0.f;  // depth >= 1
-                const float4 n = __ldg(c.feat + 2 * q), k = __ldg(c.feat + 2 * q + 1);
+                const float4 n = Ld::load(c.feat + 2 * q), k = Ld::load(c.feat + 2 * q + 1);
                 float wn = pow64(wmax(dot(a.normal, xyz(n)), 0.f));
                 float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
                 float wz = expf(-fabsf(dot(xyz(g) - a.position, a.normal)) / tolerance);
@@ -152,7 +152,7 @@ struct Sv {
                 return wn * wz * wc;
             }
         }
-        const float4 guide = __ldg(c.guide + q);
+        const float4 guide = Ld::load(c.guide + q);
         if (guide.w < 0.f) return 0.f;  // depth >= 1
         V3 nq = c.g.n(q);
         float wn = pow64(wmax(dot(a.normal, nq), 0.f));

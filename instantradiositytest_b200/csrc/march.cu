@@ -309,9 +309,9 @@ __device__ __forceinline__ void ray_setup_block(const RaySetup& s, const DevScen
     uint32_t light = kNoRay, vpl = kNoRay, hint = kNone, bin_d = 0, bin_v = 0, rank_d = 0, rank_v = 0;
     MarchState d, v;
     if (x < W && y < H) {
-        const float4 prep = __ldg(s.prep + i);
+        const float4 prep = load_written(s.prep + i);
         light = __float_as_uint(prep.w);
-        vpl = __ldg(s.prep_vpl + i);
+        vpl = load_written(s.prep_vpl + i);
         if (light != kNoRay || vpl != kNoRay) {
             const V3 p = xyz(__ldg(s.guide + i));
             hint = query_closest(sc, g, R.objs, R.n_obj, p);
@@ -448,8 +448,8 @@ __device__ __forceinline__ void lane_reset(Lane& L) {
 // The ray of record `at`, as ray_setup_tile left it, and its first query.
 __device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t at, const SceneRefs& R) {
     const float4* r = reinterpret_cast<const float4*>(s.rays + at);
-    const float4 a = __ldg(r), b = __ldg(r + 1);
-    const uint32_t hint = __ldg(s.hints + at);
+    const float4 a = load_written(r), b = load_written(r + 1);
+    const uint32_t hint = load_written(s.hints + at);
     L.m.origin = V3{a.x, a.y, a.z};
     L.m.dir = V3{b.x, b.y, b.z};
     L.m.limit = b.w;

@@ -18,12 +18,13 @@ namespace irtd {
 // variance of the bilinear taps about their mean, then
 // (1-b)*var_h + b*(1-b)*(l - mean_h)^2), which equals the reference's
 // E[l^2] - E[l]^2 without its cancellation.
-template <class G, class R, class M>
+// Ld: the guides and features are settled, or the kernel before wrote them.
+template <class G, class R, class M, class Ld>
 __device__ __forceinline__ void temporal_body(const irt_frame& f, const SvgfCtx<G>& c, const typename R::T* noisy,
                                               const typename R::T* old_radiance, const typename M::T* old_moments,
                                               typename R::T* radiance_out, typename M::T* moments_out, int32_t x,
                                               int32_t y) {
-    Sv<G> sv(f, c);
+    Sv<G, Ld> sv(f, c);
     if (x >= sv.W || y >= sv.H) return;
     size_t i = sv.idx(x, y);
     float4 c4 = R::load(noisy, i);
@@ -32,7 +33,7 @@ __device__ __forceinline__ void temporal_body(const irt_frame& f, const SvgfCtx<
     V3 history = V3{0.f, 0.f, 0.f};
     float hm0 = 0.f, hm1 = 0.f, length_history = 0.f, total = 0.f;
     float tap_w[4] = {0.f, 0.f, 0.f, 0.f}, tap_mean[4], tap_dev[4];  // MomF16 only
-    if (!(__ldg(&c.guide[i].w) < 0.f)) {  // depth < 1
+    if (!(Ld::load(&c.guide[i].w) < 0.f)) {  // depth < 1
         float2 mv = c.g.mv(i);
         float px = (sv.uvx(x) - mv.x) * (float)sv.W - .5f;
         float py = (sv.uvy(y) - mv.y) * (float)sv.H - .5f;
@@ -127,13 +128,13 @@ __device__ __forceinline__ void temporal_body(const irt_frame& f, const SvgfCtx<
 // storage: 3 blocks by registers (the f16-moments forms take 80) 0.302 /
 // 0.394 ms, 4 blocks 0.299 / 0.334, 5 blocks 0.266 / 0.308, 6 blocks 0.266 /
 // 0.290, 8 blocks 0.254 / 0.296 ms.
-template <class G, class R, class M>
+template <class G, class R, class M, class Ld>
 __global__ void __launch_bounds__(256, 8) svgf_temporal_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
                                                             const typename R::T* noisy, const typename R::T* old_radiance,
                                                             const typename M::T* old_moments, typename R::T* radiance_out,
                                                             typename M::T* moments_out) {
     frame_kernel_begin();
-    temporal_body<G, R, M>(f, c, noisy, old_radiance, old_moments, radiance_out, moments_out,
+    temporal_body<G, R, M, Ld>(f, c, noisy, old_radiance, old_moments, radiance_out, moments_out,
                            blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
 
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(256, 8) svgf_temporal_batched(const irt_frame*
     int32_t x, y;
     svgf_tile_xy(f.size[0], blockIdx.x - __ldg(tile_start + v), x, y);
     typedef typename R::T T;
-    temporal_body<G, R, M>(f, w.c, (const T*)w.in, (const T*)w.aux, (const typename M::T*)w.moments_in, (T*)w.out,
+    temporal_body<G, R, M, Settled>(f, w.c, (const T*)w.in, (const T*)w.aux, (const typename M::T*)w.moments_in, (T*)w.out,
                            (typename M::T*)w.moments_out, x, y);
 }
 
@@ -165,7 +166,7 @@ __device__ __forceinline__ void guide_body(const irt_frame& f, const float* dept
     const uint32_t W = f.size[0];
     if (i >= (size_t)W * f.size[1]) return;
     uint32_t x = (uint32_t)(i % W), y = (uint32_t)(i / W);
-    float d = __ldg(depth + i);
+    float d = load_written(depth + i);  // by the program or the last frame
     V3 p = world(((float)x + .5f) / (float)W, ((float)y + .5f) / (float)f.size[1], d,
                  previous ? f.previous_inv_vp : f.inv_vp);
     float s = d < 1.f ? distance(p, V3{f.camera[0], f.camera[1], f.camera[2]}) / (float)f.size[1] : -1.f;
@@ -178,8 +179,8 @@ template <class G>
 __device__ __forceinline__ void feature_body(const irt_frame& f, const G& g, float4* guide, float4* feat, size_t i) {
     guide_body(f, g.depth, 0, guide, i);
     if (i >= (size_t)f.size[0] * f.size[1]) return;
-    V3 n = g.n(i), c = g.c(i);
-    float2 pm = g.pm(i);
+    V3 n = g.template n<Written>(i), c = g.template c<Written>(i);
+    float2 pm = g.template pm<Written>(i);
     feat[2 * i] = make_float4(n.x, n.y, n.z, pm.x);
     feat[2 * i + 1] = make_float4(c.x, c.y, c.z, pm.y);
 }
@@ -252,8 +253,9 @@ static cudaError_t svgf_typed(const SvgfLaunch& L, int stage, cudaStream_t st) {
     dim3 grid((f.size[0] + 31) / 32, (f.size[1] + 7) / 8);
     switch (stage) {
     case 0:
-        return launch_behind(svgf_temporal_kernel<G, R, M>, grid, block, 0, st, f, c, (const T*)L.in, (const T*)L.aux,
-                             (const typename M::T*)L.moments_in, (T*)L.out, (typename M::T*)L.moments_out);
+        return launch_behind(L.after_guides ? svgf_temporal_kernel<G, R, M, Written> : svgf_temporal_kernel<G, R, M, Settled>, grid,
+                             block, 0, st, f, c, (const T*)L.in, (const T*)L.aux, (const typename M::T*)L.moments_in,
+                             (T*)L.out, (typename M::T*)L.moments_out);
     case 6: {
         size_t P = (size_t)f.size[0] * f.size[1];
         return launch_behind(feature_kernel<G>, dim3((unsigned)((P + 255) / 256)), dim3(256), 0, st, f, c.g,

@@ -17,15 +17,24 @@ struct TapGeometry {
     float4 position, normal, color;
 };
 // The planes of a row of pixels, from which a tap at a constant distance is
-// an immediate offset.
-template <class G>
+// an immediate offset.  Ld: settled, or written by the kernel before this one
+// (the variance pass of a filter that has no temporal one before it).
+template <class G, class Ld>
 struct TapRow {
     const float4* guide;
     const float4* feat;
     __device__ __forceinline__ TapRow(const SvgfCtx<G>& c, ptrdiff_t i) : guide(c.guide + i), feat(c.feat + 2 * i) {}
     __device__ __forceinline__ TapGeometry at(int32_t dx) const {
         TapGeometry t;
-        t.position = __ldg(guide + dx);
+        t.position = Ld::load(guide + dx);
+        if constexpr (std::is_same<Ld, Written>::value) {
+            asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=f"(t.normal.x), "=f"(t.normal.y), "=f"(t.normal.z), "=f"(t.normal.w), "=f"(t.color.x),
+                           "=f"(t.color.y), "=f"(t.color.z), "=f"(t.color.w)
+                         : "l"(feat + 2 * dx)
+                         : "memory");
+            return t;
+        }
         asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
             : "=f"(t.normal.x), "=f"(t.normal.y), "=f"(t.normal.z), "=f"(t.normal.w), "=f"(t.color.x),
               "=f"(t.color.y), "=f"(t.color.z), "=f"(t.color.w)
@@ -80,7 +89,7 @@ struct VarianceSums {
         for (int32_t xx = -3; xx <= 3; xx++) {
             const int32_t qx = px + xx;
             const ptrdiff_t q = at + min(max(qx, 0), W - 1);
-            const TapGeometry g = TapRow<G>(c, q).at(0);
+            const TapGeometry g = TapRow<G, Written>(c, q).at(0);
             const Moments m = M::load(moments, q);
             float wn, geom;
             const bool counts = a.weigh(g, wn, geom) && row_in && qx >= 0 && qx < W;
@@ -131,7 +140,7 @@ __device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<
     bool young = false;
     if (x < W && y < H) {
         const ptrdiff_t i = (ptrdiff_t)y * W + x;
-        young = M::load(moments, i).age < 4.f && !(__ldg(&c.guide[i].w) < 0.f);  // depth < 1
+        young = M::load(moments, i).age < 4.f && !(load_written(&c.guide[i].w) < 0.f);  // depth < 1
         if (!young) {
             float4 in = R::load(input, i);
             in.w = wmin(in.w, 65000.f);
@@ -150,7 +159,7 @@ __device__ __forceinline__ void variance_body(const irt_frame& f, const SvgfCtx<
         const ptrdiff_t i = (ptrdiff_t)py * W + px;
         const Moments centre = M::load(moments, i);
         TapCentre a;
-        a.set(TapRow<G>(c, i).at(0), 1.f);
+        a.set(TapRow<G, Written>(c, i).at(0), 1.f);
         VarianceSums<M> v;
         if (!sums(v, a, M::central ? centre.mean : 0.f, px, py)) return;
         const float4 in = R::load(input, i);
@@ -248,7 +257,7 @@ __device__ __forceinline__ bool atrous_begin(Atrous& a, const SvgfCtx<G>& c, con
                                              int32_t x, int32_t y, float step) {
     const ptrdiff_t i = (ptrdiff_t)y * W + x;
     const float4 c4 = R::load(input, i);
-    const TapGeometry own = TapRow<G>(c, i).at(0);
+    const TapGeometry own = TapRow<G, Settled>(c, i).at(0);
     if (own.position.w < 0.f) {  // depth >= 1
         R::store(out, i, c4);
         if (out2) R::store(out2, i, c4);
@@ -293,7 +302,7 @@ __device__ __forceinline__ void atrous_body(const irt_frame& f, const SvgfCtx<G>
     if (x >= 2 * Step && y >= 2 * Step && x < W - 2 * Step && y < H - 2 * Step) {
 #pragma unroll
         for (int32_t yy = -2; yy <= 2; yy++) {
-            const TapRow<G> row(c, i + (ptrdiff_t)(yy * Step) * W);
+            const TapRow<G, Settled> row(c, i + (ptrdiff_t)(yy * Step) * W);
             const typename R::T* in = input + i + (ptrdiff_t)(yy * Step) * W;
 #pragma unroll
             for (int32_t xx = -2; xx <= 2; xx++)
@@ -305,7 +314,7 @@ __device__ __forceinline__ void atrous_body(const irt_frame& f, const SvgfCtx<G>
             const int32_t xx = k % 5 - 2, yy = k / 5 - 2, qx = x + xx * Step, qy = y + yy * Step;
             if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
             const ptrdiff_t q = (ptrdiff_t)qy * W + qx;
-            a.tap(TapRow<G>(c, q).at(0), R::load(input, q), wavelet_kernel(xx) * wavelet_kernel(yy));
+            a.tap(TapRow<G, Settled>(c, q).at(0), R::load(input, q), wavelet_kernel(xx) * wavelet_kernel(yy));
         }
     }
     atrous_end<R>(a, out, out2, i);
@@ -313,8 +322,7 @@ __device__ __forceinline__ void atrous_body(const irt_frame& f, const SvgfCtx<G>
 
 template <class G, class R, int32_t Step>
 __global__ void __launch_bounds__(256, 4) svgf_atrous_kernel(const __grid_constant__ irt_frame f, const __grid_constant__ SvgfCtx<G> c,
-                                                          const typename R::T* __restrict__ input, typename R::T* __restrict__ out,
-                                                          typename R::T* __restrict__ out2) {
+                                                          const typename R::T* input, typename R::T* __restrict__ out, typename R::T* __restrict__ out2) {
     frame_kernel_begin();
     atrous_body<G, R, Step>(f, c, input, out, out2, blockIdx.x * blockDim.x + threadIdx.x,
                             blockIdx.y * blockDim.y + threadIdx.y);
