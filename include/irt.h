@@ -278,7 +278,8 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* scene, const irt_
                               const irt_gbuffer* gbuffer, const irt_vpl* current_vpls,
                               const irt_vpl* previous_vpls, void* stream);
 /* Svgf::encode (src/svgf.rs:140-261) followed by the depth/normal history
- * copy (src/renderer.rs:1951-1960). */
+ * copy (src/renderer.rs:1951-1960), over the planes given here (the lighting
+ * may have been given others). */
 irt_status irt_frame_svgf(irt_session* s, const irt_frame* frame, const irt_gbuffer* gbuffer,
                           void* stream);
 /* Both of the above. */

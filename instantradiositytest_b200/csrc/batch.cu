@@ -791,7 +791,6 @@ irt_status irt_batch_render(irt_batch* b, irt_scene* const* scenes, const irt_fr
         irt_session* s = b->sess[v];
         s->last_frame = index;
         s->have_frame = true;
-        s->guide_frame = index;
     }
     return IRT_OK;
 }

@@ -624,9 +624,7 @@ static cudaError_t compute_guides(irt_session* s, const irt_frame* f, const irt_
     G.radiance_f16 = s->desc.radiance_format == IRT_RADIANCE_F16;
     // positions and edge-stopping features, and the previous pixels' positions
     G.old_guide_out = s->guide[1];
-    cudaError_t e = irt_launch_svgf(G, 6, st);
-    if (e == cudaSuccess) s->guide_frame = f->size[2];
-    return e;
+    return irt_launch_svgf(G, 6, st);
 }
 
 static void mark(irt_session* s, int k, cudaStream_t st) {
@@ -765,11 +763,9 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
     return IRT_OK;
 }
 
-irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer* g, void* stream) {
-    if (!s) return IRT_E_INVALID;
+// `guides_done`: this frame's guides and features are of this G-buffer already.
+static irt_status frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer* g, void* stream, bool guides_done) {
     irt_context* ctx = s->ctx;
-    irt_status chk = check_frame(s, f, g);
-    if (chk) return chk;
     DeviceGuard dg(ctx->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int cur = (int)(f->size[2] % 2u), old = 1 - cur;
@@ -780,11 +776,9 @@ irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer*
         mark(s, 7, st);
         mark(s, 8, st);
     } else {
-        // Positions for this frame (already there when the lighting ran).
-        const bool fresh = s->guide_frame != f->size[2];
-        if (fresh) CK(compute_guides(s, f, g, st), "position guides");
+        if (!guides_done) CK(compute_guides(s, f, g, st), "position guides");
         SvgfLaunch L{};
-        L.after_guides = fresh;
+        L.after_guides = !guides_done;
         L.frame = f;
         L.gbuffer = *g;
         L.old_depth = s->prev_depth;
@@ -840,11 +834,20 @@ irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer*
     return IRT_OK;
 }
 
+// By itself the denoiser takes everything from the planes it is given: a frame
+// index does not tell whether the lighting saw the same ones (42 us at 1920x1200).
+irt_status irt_frame_svgf(irt_session* s, const irt_frame* f, const irt_gbuffer* g, void* stream) {
+    if (!s) return IRT_E_INVALID;
+    irt_status chk = check_frame(s, f, g);
+    if (chk) return chk;
+    return frame_svgf(s, f, g, stream, false);
+}
+
 irt_status irt_render_frame(irt_session* s, const irt_scene* sc, const irt_frame* f, const irt_gbuffer* g,
                             const irt_vpl* cur, const irt_vpl* prev, void* stream) {
     irt_status r = irt_frame_lighting(s, sc, f, g, cur, prev, stream);
     if (r) return r;
-    return irt_frame_svgf(s, f, g, stream);
+    return frame_svgf(s, f, g, stream, true);
 }
 
 // ------------------------------------------------------------------ host inputs

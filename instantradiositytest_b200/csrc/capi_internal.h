@@ -121,7 +121,6 @@ struct irt_session {
     // pixels from the previous depth and previous_inv_vp
     float4* guide[2] = {nullptr, nullptr};
     float4* feat = nullptr;  // this frame's SVGF edge-stopping features, 2 float4 per pixel
-    uint32_t guide_frame = 0xffffffffu;
     int num_sms = 0;
     // Host-input pipeline (irt_render_frame_host), created on first use:
     // a copy stream, double-buffered device G-buffers, three VPL pools plus
