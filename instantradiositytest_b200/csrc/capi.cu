@@ -389,8 +389,8 @@ irt_status irt_scene_update(irt_scene* sc, const irt_object* objects, uint32_t o
             sc->grid_size[a] = LC.grid_size[a] = (float)((hi - lo) / kGridRes);
             sc->grid_inv[a] = (float)(kGridRes / (hi - lo));
         }
-        // The f32 error of a distance and of a point's place in its cell; for
-        // the filtered sampler also what its weights may miss by.
+        // The f32 error of a distance and of a point's place in its cell, and
+        // what the scene's sampler may miss the field by.
         double d2 = 0, far = 0, voxel = 0;
         for (int a = 0; a < 3; a++) {
             d2 += (double)sc->grid_size[a] * sc->grid_size[a];

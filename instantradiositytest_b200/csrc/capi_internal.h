@@ -75,7 +75,7 @@ inline irtd::FieldFilter scene_field_filter(const irt_scene* sc) {
     irtd::FieldFilter f{};
     f.linear = sc->field_linear ? sc->atlas_linear : 0;
     for (int a = 0; a < 3; a++) f.dims[a] = (float)sc->atlas_dims[a];
-    f.bound_slack = sc->field_linear ? 1.f / 32.f : 0.f;
+    f.bound_slack = sc->field_linear ? 1.f / 32.f : sc->sdf_f16 ? 1.f / 1024.f : 0.f;
     return f;
 }
 

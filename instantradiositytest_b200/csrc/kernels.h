@@ -15,8 +15,11 @@ namespace irtd {
 struct FieldFilter {
     cudaTextureObject_t linear;  // the atlas: texel coordinates, linear filter, clamp
     float dims[3];               // atlas extent in texels
-    // Voxels by which a sampled distance may miss the trilinear value (three
-    // axes of 8-bit weights), for the leaf-order cache's bounds; 0 unfiltered.
+    // Voxels by which a sampled distance may miss the trilinear value of the
+    // exact field, for the leaf-order cache's bounds: three axes of 8-bit weights
+    // for the filtered sampler; an f16 texel's 2^-10 of its value, which exceeds
+    // the distance by half a voxel and within a cell by up to one (the part that
+    // grows with the distance is in the cache's slope); 0 for f32 points.
     float bound_slack;
 };
 }  // namespace irtd

@@ -12,8 +12,8 @@
 //   * the box bound: distance from c to the object's BVH leaf box, x 0.9998;
 //   * the object's own distance at c, where positive;
 // less a margin for the f32 evaluation of either side, of f16 texels (rounded
-// down by up to 2^-10 of a distance) and of the filtered sampler's 8-bit
-// weights.  The march visits a cell's objects in this order and stops at the
+// down by up to 2^-10 of their value: the distance and up to a voxel) and of the
+// filtered sampler's 8-bit weights.  The march visits a cell's objects in this order and stops at the
 // first bound above its best distance + |p - c|; every object it skips has a
 // distance above that best, so the minimum, the closest object and its voxel
 // are those of the reference walk.  Distances use the march's own device code.
