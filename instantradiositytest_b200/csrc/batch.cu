@@ -158,7 +158,6 @@ LightingLaunch lighting_launch(irt_session* s, const irt_scene* sc, const irt_fr
     L.cur_vpls = cur;
     L.prev_vpls = prev;
     L.archive = s->archive;
-    L.prev_depth = s->prev_depth;
     L.prev_normal = s->prev_normal;
     for (int k = 0; k < 3; k++) {
         L.dres[k] = s->dres[k];

@@ -196,7 +196,6 @@ irt_status irt_scene_create(irt_context* ctx, const irt_mesh* meshes, uint32_t m
     sc->ctx = ctx;
     sc->mesh_count = mesh_count;
     sc->sdf_f16 = sdf_format == IRT_SDF_F16;
-    for (int a = 0; a < 3; a++) sc->atlas_dims[a] = atlas_dims[a];
     sc->host_meshes.assign(meshes, meshes + mesh_count);
     auto fail = [&](irt_status s) {
         irt_scene_destroy(sc);
@@ -713,7 +712,6 @@ irt_status irt_frame_lighting(irt_session* s, const irt_scene* sc, const irt_fra
     L.cur_vpls = cur;
     L.prev_vpls = prev;
     L.archive = s->archive;
-    L.prev_depth = s->prev_depth;
     L.prev_normal = s->prev_normal;
     for (int k = 0; k < 3; k++) {
         L.dres[k] = s->dres[k];

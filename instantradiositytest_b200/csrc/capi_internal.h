@@ -38,7 +38,6 @@ struct irt_scene {
     int field_linear = 0;            // in use since the last irt_scene_update
     int field_linear_requested = 0;  // irt_scene_set_field_filter, applied by the next update
     int sdf_f16 = 0;
-    uint32_t atlas_dims[3] = {0, 0, 0};
     // Corner cells: per field mesh, the 8 corner texels of each of its
     // (res-1)^3 cells in one record (f32: 32 B, f16: 16 B); a mesh's first
     // cell index is in hi[3] of its rows (host_meshes and the device copy).
@@ -74,7 +73,6 @@ struct irt_scene {
 inline irtd::FieldFilter scene_field_filter(const irt_scene* sc) {
     irtd::FieldFilter f{};
     f.linear = sc->field_linear ? sc->atlas_linear : 0;
-    for (int a = 0; a < 3; a++) f.dims[a] = (float)sc->atlas_dims[a];
     f.bound_slack = sc->field_linear ? 1.f / 32.f : sc->sdf_f16 ? 1.f / 1024.f : 0.f;
     return f;
 }

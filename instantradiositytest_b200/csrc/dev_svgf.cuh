@@ -19,8 +19,8 @@ struct SvgfCtx {
     // Per-pixel edge-stopping features of this frame (feature_kernel), two
     // float4 per pixel: (normal, roughness), (colour, metal) — the decoded
     // G-buffer values a tap reads, in one 256-bit load instead of 3 or 4 plane
-    // reads and decodes.  The a-trous pass needs them and `guide`; temporal and
-    // variance read them where a plane would be decoded.
+    // reads and decodes.  Temporal reads f32 planes as they are, the other
+    // passes only these and `guide`.
     const float4* feat;
 };
 
@@ -77,9 +77,8 @@ struct MomF16 {
 
 template <class G, class Ld>
 struct Sv {
-    // Feature records are read by the temporal and variance passes for G-buffer
-    // formats that decode per tap (on f32 planes they move 0.013 ms from one to
-    // 0.007 ms in the other).
+    // The temporal pass reads feature records for G-buffer formats that decode
+    // per tap, f32 planes as they are.
     static constexpr bool kFeatures = !std::is_same<G, GbF32>::value;
     const irt_frame& f;
     const SvgfCtx<G>& c;
@@ -114,24 +113,22 @@ struct Sv {
         Guide a;
         size_t i = idx(x, y);
         if constexpr (kFeatures) {
-            if (c.feat) {
-                const float4 g = Ld::load(c.guide + i), n = Ld::load(c.feat + 2 * i), k = Ld::load(c.feat + 2 * i + 1);
-                a.position = xyz(g);
-                a.normal = xyz(n);
-                a.color = xyz(k);
-                a.m0 = n.w;
-                a.m1 = k.w;
-                a.pixel_scale = g.w;  // distance(position, camera) / height (feature_kernel)
-                return a;
-            }
+            const float4 g = Ld::load(c.guide + i), n = Ld::load(c.feat + 2 * i), k = Ld::load(c.feat + 2 * i + 1);
+            a.position = xyz(g);
+            a.normal = xyz(n);
+            a.color = xyz(k);
+            a.m0 = n.w;
+            a.m1 = k.w;
+            a.pixel_scale = g.w;  // distance(position, camera) / height (feature_kernel)
+        } else {
+            a.position = position(x, y);
+            a.normal = c.g.n(i);
+            a.color = c.g.c(i);
+            float2 pm = c.g.pm(i);
+            a.m0 = pm.x;
+            a.m1 = pm.y;
+            a.pixel_scale = distance(a.position, camera()) / (float)f.size[1];
         }
-        a.position = position(x, y);
-        a.normal = c.g.n(i);
-        a.color = c.g.c(i);
-        float2 pm = c.g.pm(i);
-        a.m0 = pm.x;
-        a.m1 = pm.y;
-        a.pixel_scale = distance(a.position, camera()) / (float)f.size[1];
         return a;
     }
     // svgf.wgsl:32-44
@@ -139,31 +136,30 @@ struct Sv {
         if (!inside(qx, qy)) return 0.f;
         size_t q = idx(qx, qy);
         if constexpr (kFeatures) {
-            if (c.feat) {
-                const float4 g = Ld::load(c.guide + q);
-                if (g.w < 0.f) return 0.f;  // depth >= 1
-                const float4 n = Ld::load(c.feat + 2 * q), k = Ld::load(c.feat + 2 * q + 1);
-                float wn = pow64(wmax(dot(a.normal, xyz(n)), 0.f));
-                float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
-                float wz = expf(-fabsf(dot(xyz(g) - a.position, a.normal)) / tolerance);
-                V3 dc = a.color - xyz(k);
-                float d0 = a.m0 - n.w, d1 = a.m1 - k.w;
-                float wc = expf(-length(dc) * 8.f - sqrtf(d0 * d0 + d1 * d1) * 8.f);
-                return wn * wz * wc;
-            }
+            const float4 g = Ld::load(c.guide + q);
+            if (g.w < 0.f) return 0.f;  // depth >= 1
+            const float4 n = Ld::load(c.feat + 2 * q), k = Ld::load(c.feat + 2 * q + 1);
+            float wn = pow64(wmax(dot(a.normal, xyz(n)), 0.f));
+            float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
+            float wz = expf(-fabsf(dot(xyz(g) - a.position, a.normal)) / tolerance);
+            V3 dc = a.color - xyz(k);
+            float d0 = a.m0 - n.w, d1 = a.m1 - k.w;
+            float wc = expf(-length(dc) * 8.f - sqrtf(d0 * d0 + d1 * d1) * 8.f);
+            return wn * wz * wc;
+        } else {
+            const float4 guide = Ld::load(c.guide + q);
+            if (guide.w < 0.f) return 0.f;  // depth >= 1
+            V3 nq = c.g.n(q);
+            float wn = pow64(wmax(dot(a.normal, nq), 0.f));
+            V3 wq = xyz(guide);
+            float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
+            float wz = expf(-fabsf(dot(wq - a.position, a.normal)) / tolerance);
+            V3 dc = a.color - c.g.c(q);
+            float2 pm = c.g.pm(q);
+            float d0 = a.m0 - pm.x, d1 = a.m1 - pm.y;
+            float wc = expf(-length(dc) * 8.f - sqrtf(d0 * d0 + d1 * d1) * 8.f);
+            return wn * wz * wc;
         }
-        const float4 guide = Ld::load(c.guide + q);
-        if (guide.w < 0.f) return 0.f;  // depth >= 1
-        V3 nq = c.g.n(q);
-        float wn = pow64(wmax(dot(a.normal, nq), 0.f));
-        V3 wq = xyz(guide);
-        float tolerance = wmax(.0001f, a.pixel_scale * stride * .5f);
-        float wz = expf(-fabsf(dot(wq - a.position, a.normal)) / tolerance);
-        V3 dc = a.color - c.g.c(q);
-        float2 pm = c.g.pm(q);
-        float d0 = a.m0 - pm.x, d1 = a.m1 - pm.y;
-        float wc = expf(-length(dc) * 8.f - sqrtf(d0 * d0 + d1 * d1) * 8.f);
-        return wn * wz * wc;
     }
 };
 
@@ -233,7 +229,7 @@ __host__ inline SvgfCtx<G> make_ctx(const SvgfLaunch& L) {
     c.old_normal = reinterpret_cast<const typename G::NormalT*>(L.old_normal);
     c.guide = L.guide;
     c.old_guide = L.old_guide;
-    c.feat = L.guide ? L.feat : nullptr;
+    c.feat = L.feat;
     return c;
 }
 

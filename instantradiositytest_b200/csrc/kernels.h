@@ -14,7 +14,6 @@ namespace irtd {
 // point-sampled trilinear of common.wgsl:31-38.
 struct FieldFilter {
     cudaTextureObject_t linear;  // the atlas: texel coordinates, linear filter, clamp
-    float dims[3];               // atlas extent in texels
     // Voxels by which a sampled distance may miss the trilinear value of the
     // exact field, for the leaf-order cache's bounds: three axes of 8-bit weights
     // for the filtered sampler; an f16 texel's 2^-10 of its value, which exceeds
@@ -124,7 +123,6 @@ struct LightingLaunch {
     const irt_vpl* cur_vpls;
     const irt_vpl* prev_vpls;
     const irt_vpl* archive;
-    const float* prev_depth;
     const void* prev_normal;
     irt_reservoir* dres[3];
     irt_reservoir* ires[3];

@@ -30,7 +30,6 @@ struct LightArgs {
     const irt_vpl* cur;
     const irt_vpl* prev;
     const irt_vpl* arch;
-    const float* prev_depth;
     const typename G::NormalT* prev_normal;
     irt_reservoir* dres[3];
     irt_reservoir* ires[3];
@@ -593,7 +592,6 @@ static LightArgs<G> make_args(const LightingLaunch& L) {
     a.cur = L.cur_vpls;
     a.prev = L.prev_vpls;
     a.arch = L.archive;
-    a.prev_depth = L.prev_depth;
     a.prev_normal = reinterpret_cast<const typename G::NormalT*>(L.prev_normal);
     for (int k = 0; k < 3; k++) {
         a.dres[k] = L.dres[k];

@@ -445,7 +445,7 @@ __device__ __forceinline__ void lane_reset(Lane& L) {
     L.qy.oid = kNone;
     L.active = false;
 }
-// The ray of record `at`, as ray_setup_tile left it, and its first query.
+// The ray of record `at`, as ray_setup_block left it, and its first query.
 __device__ __forceinline__ void lane_take(Lane& L, const RaySetup& s, uint32_t at, const SceneRefs& R) {
     const float4* r = reinterpret_cast<const float4*>(s.rays + at);
     const float4 a = load_written(r), b = load_written(r + 1);

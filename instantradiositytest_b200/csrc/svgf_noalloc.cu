@@ -31,8 +31,7 @@ constexpr int kMaxDevices = 64;
 
 // Per pixel: [0] ping and [1] pong a-trous images (f32x4; f16x4 images use
 // the first half of each), [2] world position + SVGF pixel scale, [3..4]
-// edge-stopping feature records (two f32x4 per pixel, decoded G-buffer
-// formats only).
+// edge-stopping feature records (two f32x4 per pixel).
 static __device__ __align__(256) float4 g_svgf_scratch[5][kNoAllocMaxPixels];
 
 // Device address of g_svgf_scratch per device ordinal, looked up on the first
@@ -112,8 +111,9 @@ extern "C" irt_status irt_svgf_spatial_noalloc(const irt_frame* frame, const irt
     L.gbuffer = *gbuffer;
     L.radiance_f16 = radiance_format == IRT_RADIANCE_F16;
     L.moments_f16 = moments_format == IRT_MOMENTS_F16;
-    // The frame's per-pixel positions and edge-stopping features, written by the same kernels a session
-    // runs before its SVGF passes, so the results equal a session's.
+    // The frame's per-pixel positions and edge-stopping features, written by
+    // the same kernel a session runs before its SVGF passes, so the results
+    // equal a session's.
     L.out = guide;
     L.out2 = feat;
     cudaError_t e = irt_launch_svgf(L, 6, st);
