@@ -51,7 +51,9 @@ inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, si
     a.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &a;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // returned here, not to the next launch's check
+    return e;
 }
 #ifdef __CUDACC__
 namespace irtd {
