@@ -67,7 +67,7 @@ __device__ __forceinline__ V3 normalize(V3 a) {
     return a / s;
 #else
     const float r = __frcp_rn(s);
-    const bool mid = s > 1e-15f && s < 1e15f;
+    const bool mid = s > 0.f && s < INFINITY;
     return {mid ? div_by(a.x, s, r) : a.x * r, mid ? div_by(a.y, s, r) : a.y * r, mid ? div_by(a.z, s, r) : a.z * r};
 #endif
 }
