@@ -57,7 +57,7 @@ __device__ __forceinline__ void primary_ray(const irt_frame& f, float u, float v
 // bounding sphere is not wholly beyond one of the four planes through the rays
 // of neighbouring block corners.  Every pixel of the block tests the same few
 // primitives instead of all: 1280x720, 23 objects 97 -> 57 us, 2560x1600, 50
-// objects 816 -> 300.
+// objects 816 -> 303.
 //
 // The planes hold for every inv_vp, parallel projections among them: a plane
 // goes through both corners' near and far points (parallel image lines stay
